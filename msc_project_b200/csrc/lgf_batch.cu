@@ -108,7 +108,7 @@ int run_wave(lgf_ctx* ctx, int prec, std::vector<JobRun*>& runs, GroupBase* grp,
             if (e != LGF_OK) return e;
             last_measured = which;
         }
-        *launches += 3;
+        *launches += grp->launches_per_measure();
         return grp->replay_measure();
     };
     // t0 measurements

@@ -13,6 +13,8 @@
 //   - the stage and measurement tile lists cover every tile exactly once for
 //     row-block and column orders and a range of budgets and block sizes, and
 //     the measurement's strips or patches cover every site of a slice once;
+//   - the units of the measurement's plane kernel cover every site of every
+//     plane once as an output, with the three rows before it in the unit;
 //   - the launch segments of a group (member_runs) split a list of members
 //     into at most `slots` back-to-back runs of whole members covering it.
 // Prints one line and exits 0 when everything holds.
@@ -25,6 +27,7 @@
 #ifndef LGF_MEAS_PATCH
 #define LGF_MEAS_PATCH 1
 #endif
+#include "lgf_measure.cuh"
 #include "lgf_tiles.h"
 
 using namespace lgf;
@@ -187,6 +190,45 @@ static void check_tiles(const Geom& g) {
     }
 }
 
+// every site is an output of exactly one unit per plane, and the sites one to
+// three steps back along mu are where the kernel looks for them in the unit
+template <int ROUND> static void check_plane_units(const Geom& g) {
+    for (int T : {96, 192, 384}) {
+        const int n = plane_units(g, ROUND, T);
+        for (int j = 0; j < 3; ++j) {
+            std::vector<char> hit(g.V, 0);
+            const int mu = round_mu<ROUND>(j);
+            const ColumnTiling ct = column_tiling(g, mu, T);
+            CHECK(ct.C >= 1 && ct.rows * ct.C <= T);
+            for (int u = 0; u < n; ++u) {
+                const PlaneUnit pu = plane_unit<ROUND>(g, T, u);
+                CHECK(pu.j >= 0 && pu.j < 3 && pu.block >= 0 && pu.block < ct.blocks + (pu.j != j) * g.V && pu.tile >= 0);
+                if (pu.j != j) continue;
+                CHECK(pu.tile < ct.tiles);
+                std::vector<int> site(T, -1);
+                UnitSite us;
+                for (int t = 0; t < T; ++t)
+                    if (unit_site(g, mu, ct, pu, t % ct.C, t / ct.C, &us)) {
+                        CHECK(us.s >= 0 && us.s < g.V);
+                        CHECK(site_coord(g, us.s).x[mu] == us.xmu);
+                        site[t] = us.s;
+                    }
+                for (int t = 0; t < T; ++t) {
+                    if (!unit_site(g, mu, ct, pu, t % ct.C, t / ct.C, &us) || !us.out) continue;
+                    CHECK(!hit[us.s]++);
+                    int b = t, s = us.s;
+                    for (int k = 1; k <= 3; ++k) {
+                        b = b - ct.C < 0 ? b - ct.C + ct.rows * ct.C : b - ct.C;
+                        s = bwd(g, s, mu, site_coord(g, s).x[mu]);
+                        CHECK(b >= 0 && b < T && site[b] == s);
+                    }
+                }
+            }
+            for (int s = 0; s < g.V; ++s) CHECK(hit[s] == 1);
+        }
+    }
+}
+
 static void check_member_runs() {
     const std::vector<std::vector<int>> lists = {
         {}, {0}, {5}, {20736}, {43, 43, 43}, {683, 20736, 683, 683, 2048, 165888, 1},
@@ -223,7 +265,16 @@ int main() {
         check_layout<double>(g);
         check_layout<float>(g);
         check_tiles(g);
+        check_plane_units<0>(g);
+        check_plane_units<1>(g);
         ++n;
+    }
+    // extents above a unit's sites: row tiles with three rows of halo
+    const int tall[][4] = {{100, 4, 4, 4}, {4, 392, 4, 6}, {4, 6, 200, 4}, {194, 4, 4, 4}};
+    for (const auto& sh : tall) {
+        const Geom g = make_geom(sh);
+        check_plane_units<0>(g);
+        check_plane_units<1>(g);
     }
     if (g_fail) {
         std::printf("index check FAILED: %d failures\n", g_fail);

@@ -217,7 +217,7 @@ int count_measurements(const lgf_flow_opts& o) {
 // Outputs: mtiles (the selected segments back to back), rtiles (member, t)
 // for t < N0, jobs[k] = member, counts = {tiles, slices, nsel}.  Grid
 // (max(nsel, 1), any): block (k, y) copies a share of segment k.
-constexpr int SEL_HEADER = 4, SEL_FIELDS = 6;
+constexpr int SEL_HEADER = 4, SEL_SEGS = 2, SEL_FIELDS = 6;  // ints; int2 segments before the launch segments; ints
 __global__ void __launch_bounds__(256) k_select_measure(const int* __restrict__ sel, int fields,
                                                         const int4* __restrict__ all, int4* __restrict__ mtiles,
                                                         int2* __restrict__ rtiles, int* __restrict__ jobs,
@@ -250,7 +250,7 @@ public:
           int slots)
         : ctx_(ctx), shape_(shape), threads_(shape.threads), max_members_(max_members), max_tiles_(max_tiles),
           dynamic_(dynamic), per_volume_(per_volume), slots_(std::max(1, std::min(slots, max_members))),
-          step_execs_(slots_ + 1, nullptr), meas_execs_(slots_ + 1, nullptr) {}
+          step_execs_(slots_ + 1, nullptr), meas_execs_(2 * (slots_ + 1), nullptr) {}
     ~Group() override {
         cudaStreamSynchronize(ctx_->stream);  // the lists are in use until then
         drop_graphs();
@@ -277,16 +277,22 @@ public:
         int nb = 0;
         LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_stage<R, 1>, threads_, 0));
         stage_grid_max_ = std::max(1, nb) * ctx_->sm_count;
-        if (shape_.meas_split == 2) {
-            LGF_CUDA_TRY(ctx_, (prepare_measure_kernel<R, false, 2>()));
-            LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_measure<R, false, 2>,
-                                                                             MEAS_SITES * 12, measure_smem_bytes<R>()));
-        } else {
-            LGF_CUDA_TRY(ctx_, (prepare_measure_kernel<R, false, 1>()));
-            LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_measure<R, false, 1>,
-                                                                             MEAS_SITES * 6, measure_smem_bytes<R>()));
-        }
-        meas_grid_max_ = std::max(1, nb) * ctx_->sm_count;
+        // Measurement blocks: 4 tiles (loops) and 384 sites (planes) per block,
+        // halved for one-warp-per-plane shapes, and smaller for lattices that
+        // would not give every SM a block.
+        const long long cap_sites = max_tiles_ * (threads_ / 4);
+        meas_groups_ = shape_.meas_split == 2 ? LOOP_MAX_GROUPS : LOOP_MAX_GROUPS / 2;
+        while (meas_groups_ > 1 && cap_sites < (long long)MEAS_SITES * meas_groups_ * ctx_->sm_count) meas_groups_ /= 2;
+        unit_sites_ = shape_.meas_split == 2 ? PLANE_MAX_SITES : PLANE_MAX_SITES / 2;
+        while (unit_sites_ > 96 && 3 * cap_sites < (long long)unit_sites_ * ctx_->sm_count) unit_sites_ /= 2;
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_measure<R, true>, MEAS_SITES * MEAS_WARPS, measure_smem_bytes<R>(), &nb)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_measure<R, false>, MEAS_SITES * MEAS_WARPS, measure_smem_bytes<R>(), &small_grid_max_)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_loops<R, 0>, 96 * meas_groups_, loops_smem_bytes(meas_groups_), &loops_grid_max_)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_loops<R, 1>, 96 * meas_groups_, loops_smem_bytes(meas_groups_), &nb)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 0, false>, unit_sites_, planes_smem_bytes<R>(unit_sites_), &planes_grid_max_)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 1, false>, unit_sites_, planes_smem_bytes<R>(unit_sites_), &nb)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 0, true>, unit_sites_, planes_smem_bytes<R>(unit_sites_), &nb)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 1, true>, unit_sites_, planes_smem_bytes<R>(unit_sites_), &nb)));
         if (dynamic_) {
             // members change after capture: size the measurement lists for the
             // largest resident set the tile capacity allows (x0 extents <= 256)
@@ -407,14 +413,21 @@ public:
 
     // The selection table goes through a page-locked area and the lists are
     // assembled on the device (k_select_measure): no host wait.
-    int set_measured(const std::vector<int>& which) override {
-        if ((int)which.size() > max_members_) return set_error(ctx_, LGF_EINVAL, "measurement list exceeds capacity");
+    int set_measured(const std::vector<int>& measured) override {
+        if ((int)measured.size() > max_members_) return set_error(ctx_, LGF_EINVAL, "measurement list exceeds capacity");
+        for (int i : measured)
+            if (i < 0 || i >= (int)members_.size()) return set_error(ctx_, LGF_EINVAL, "no member %d to measure", i);
+        // small lattices (one launch) first, then the others
+        std::vector<int> which(measured);
+        const size_t nsmall = std::stable_partition(which.begin(), which.end(), [&](int i) { return small_measure(members_[i]->g); }) -
+                              which.begin();
         std::vector<int> sel(sel_ints((int)which.size()), 0);
         std::vector<int> lens(which.size());
-        long long tm = 0, tr = 0;
+        PlaneMember* units[2] = {reinterpret_cast<PlaneMember*>(&sel[sel_members(0)]),
+                                 reinterpret_cast<PlaneMember*>(&sel[sel_members(1)])};
+        long long tm = 0, ts = 0, tr = 0, tu[2] = {0, 0};
         for (size_t k = 0; k < which.size(); ++k) {
             const int i = which[k];
-            if (i < 0 || i >= (int)members_.size()) return set_error(ctx_, LGF_EINVAL, "no member %d to measure", i);
             lens[k] = seg_len_[i];
             int* f = &sel[sel_fields() + SEL_FIELDS * k];
             f[0] = i;
@@ -425,19 +438,38 @@ public:
             f[5] = (int)tr;
             tm += seg_len_[i];
             tr += members_[i]->g.n[0];
+            if (k < nsmall) ts = tm;
+            for (int round = 0; round < 2; ++round) {
+                units[round][k] = {i, (int)tu[round]};
+                tu[round] += plane_units(members_[i]->g, round, unit_sites_);
+            }
         }
-        if (tm > mtiles_cap_ || tr > rtiles_cap_ || (long long)which.size() > jobs_cap_)
+        if (tm > mtiles_cap_ || tr > rtiles_cap_ || (long long)which.size() > jobs_cap_ ||
+            std::max(tu[0], tu[1]) > (1LL << 31) - 1024)
             return set_error(ctx_, LGF_EINVAL, "measurement list exceeds capacity");
         sel[0] = (int)which.size();
         sel[1] = (int)tm;
         sel[2] = (int)tr;
-        // the measurement kernel's launch segments, over the selected members in list order
-        const std::vector<int2> segs = member_runs(lens, slots_, 8LL * meas_grid_max_);
+        int2* seg = reinterpret_cast<int2*>(&sel[SEL_HEADER]);
+        seg[0] = make_int2(0, (int)ts);               // the small lattices' tiles
+        seg[1] = make_int2((int)ts, (int)(tm - ts));  // the others'
+        // the others' launch segments, in list order: runs of whole members by
+        // their tiles, and the same members' plane units
+        const std::vector<int2> segs = member_runs(std::vector<int>(lens.begin() + nsmall, lens.end()), slots_, 8LL * loops_grid_max_);
+        size_t m = nsmall;
+        long long pos = 0;
         for (size_t k = 0; k < segs.size(); ++k) {
-            sel[SEL_HEADER + 2 * k] = segs[k].x;
-            sel[SEL_HEADER + 2 * k + 1] = segs[k].y;
+            seg[SEL_SEGS + k] = make_int2((int)ts + segs[k].x, segs[k].y);
+            const size_t m0 = m;
+            while (m < which.size() && pos < (long long)segs[k].x + segs[k].y) pos += lens[m++];
+            for (int round = 0; round < 2; ++round) {
+                const int u0 = m0 < which.size() ? units[round][m0].start : (int)tu[round];
+                const int u1 = m < which.size() ? units[round][m].start : (int)tu[round];
+                seg[SEL_SEGS + (round + 1) * slots_ + k] = make_int2(u0, u1 - u0);
+            }
         }
-        meas_nseg_ = (int)segs.size();
+        meas_small_ = nsmall > 0;
+        meas_nseg_ = nsmall < which.size() ? (int)segs.size() : 0;
         {
             std::lock_guard<std::mutex> lk(ctx_->list_mu);
             char* h = nullptr;
@@ -460,20 +492,27 @@ public:
         if (k < 3) {
             for (int j = 0; j < stage_nseg_; ++j) launch_stage(k + 1, j);
         } else {
-            launch_measure_kernel(meas_nseg_);
+            launch_measure_kernels<false>(meas_nseg_, meas_small_, MeasSites{});
         }
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
     }
 
-    int launch_measure() override { return launch_measurement(meas_nseg_); }
+    int launch_measure() override { return launch_measurement(meas_nseg_, meas_small_); }
+
+    // one pass over the measured members that also writes per-site outputs (single-lattice groups)
+    int launch_sites(const MeasSites& out) override {
+        launch_measure_kernels<true>(meas_nseg_, meas_small_, out);
+        LGF_CUDA_TRY(ctx_, cudaGetLastError());
+        return LGF_OK;
+    }
 
     // drop the graphs and capture those of the current segment counts
     int capture() override {
         drop_graphs();
         int rc = capture_one(true, stage_nseg_, &step_execs_[stage_nseg_]);
         if (rc != LGF_OK) return rc;
-        return capture_one(false, meas_nseg_, &meas_execs_[meas_nseg_]);
+        return capture_one(false, meas_nseg_, &meas_execs_[meas_graph()]);
     }
     // graph launch; a graph per count of launch segments, captured on first use
     int replay_step() override {
@@ -488,7 +527,7 @@ public:
     }
     int replay_measure() override {
         NvtxRange r("lgf.measure");
-        cudaGraphExec_t& g = meas_execs_[meas_nseg_];
+        cudaGraphExec_t& g = meas_execs_[meas_graph()];
         if (!g) {
             int rc = capture_one(false, meas_nseg_, &g);
             if (rc != LGF_OK) return rc;
@@ -497,17 +536,31 @@ public:
         return LGF_OK;
     }
     int launches_per_step() const override { return 3; }
+    int launches_per_measure() const override { return (meas_small_ ? 1 : 0) + (meas_nseg_ ? 5 : 0) + 2; }
     int threads() const override { return threads_; }
     const TileShape& shape() const override { return shape_; }
 
 private:
     int stage_grid() const { return dynamic_ ? stage_grid_max_ : std::max(1, std::min(ntiles_, stage_grid_max_)); }
-    int meas_grid() const {
-        return dynamic_ ? meas_grid_max_ : std::max(1, std::min((int)std::max<long long>(mtiles_cap_, 1), meas_grid_max_));
+    // a measurement kernel's grid: its persistent grid, or fewer blocks when its lists are shorter
+    int meas_grid(long long work, int grid_max) const {
+        return dynamic_ ? grid_max : (int)std::max(1LL, std::min(work, (long long)grid_max));
     }
-    // ints of a selection table for n members: header, launch segments, member fields
-    int sel_fields() const { return SEL_HEADER + 2 * slots_; }
+    // raise the kernel's shared-memory limit and find its persistent grid
+    template <typename K> cudaError_t meas_occupancy(K kernel, int threads, size_t smem, int* grid) const {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int nb = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem);
+        *grid = std::max(1, nb) * ctx_->sm_count;
+        return e;
+    }
+    // ints of a selection table for n members: header, the tiles of the small
+    // and of the other lattices, the others' launch segments (loop tiles,
+    // round 0 units, round 1 units), unit tables of the two rounds, member fields
+    int sel_members(int round) const { return SEL_HEADER + 2 * SEL_SEGS + 6 * slots_ + 2 * max_members_ * round; }
+    int sel_fields() const { return SEL_HEADER + 2 * SEL_SEGS + 6 * slots_ + 4 * max_members_; }
     size_t sel_ints(int n) const { return (size_t)sel_fields() + (size_t)SEL_FIELDS * std::max(n, 1); }
+    int meas_graph() const { return 2 * meas_nseg_ + (meas_small_ ? 1 : 0); }
     bool captured() const {
         for (auto g : step_execs_) if (g) return true;
         for (auto g : meas_execs_) if (g) return true;
@@ -536,34 +589,46 @@ private:
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
     }
-    int launch_measurement(int nseg) {
+    int launch_measurement(int nseg, bool small) {
         NvtxRange r("lgf.measure_launch");
         const int rg = dynamic_ ? ctx_->sm_count : std::max(1, (int)std::min<long long>(rtiles_cap_, 4 * ctx_->sm_count));
         const int jg = dynamic_ ? std::min(jobs_cap_, 4 * ctx_->sm_count) : std::max(1, (int)std::min<long long>(jobs_cap_, 4 * ctx_->sm_count));
-        launch_measure_kernel(nseg);
+        launch_measure_kernels<false>(nseg, small, MeasSites{});
         k_reduce_slices<R><<<rg, RED_THREADS, 0, ctx_->stream>>>(d_desc_, d_rtiles_, d_counts_ + 2);
         k_reduce_total<R><<<std::max(1, jg), RED_THREADS, 0, ctx_->stream>>>(d_desc_, d_jobs_, d_counts_ + 3);
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
     }
-    // the measurement kernel over launch segments 0..nseg-1 (read from the selection table)
-    void launch_measure_kernel(int nseg) {
-        const int grid = meas_grid();
+    // the measurement kernels over the selection table's segments
+    template <bool OUT> void launch_measure_kernels(int nseg, bool small, const MeasSites& out) {
         const int2* segs = reinterpret_cast<const int2*>(d_sel_ + SEL_HEADER);
+        if (small)
+            k_measure<R, OUT><<<meas_grid(mtiles_cap_, small_grid_max_), dim3(MEAS_SITES, MEAS_WARPS), measure_smem_bytes<R>(), ctx_->stream>>>(
+                d_desc_, d_mtiles_, segs, out);
+        if (nseg == 0) return;
+        const int2* runs = segs + SEL_SEGS;
+        launch_round<0, OUT>(runs, runs + slots_, nseg, out);
+        launch_round<1, OUT>(runs, runs + 2 * slots_, nseg, out);
+        const int warps = SITES_THREADS / 32;
+        k_meas_sites<R, OUT><<<meas_grid((mtiles_cap_ + warps - 1) / warps, 8 * ctx_->sm_count), SITES_THREADS, 0, ctx_->stream>>>(
+            d_desc_, d_mtiles_, segs + 1, out);
+    }
+    template <int ROUND, bool OUT> void launch_round(const int2* tiles, const int2* units, int nseg, const MeasSites& out) {
+        const PlaneMember* members = reinterpret_cast<const PlaneMember*>(d_sel_ + sel_members(ROUND));
+        const int lg = meas_grid((mtiles_cap_ + meas_groups_ - 1) / meas_groups_, loops_grid_max_);
+        const int pg = meas_grid(dynamic_ || members_.empty() ? 1 : plane_units(members_[0]->g, ROUND, unit_sites_), planes_grid_max_);
         for (int j = 0; j < nseg; ++j) {
-            if (shape_.meas_split == 2)
-                k_measure<R, false, 2><<<grid, dim3(MEAS_SITES, 12), measure_smem_bytes<R>(), ctx_->stream>>>(
-                    d_desc_, d_mtiles_, segs + j, MeasOut{});
-            else
-                k_measure<R, false, 1><<<grid, dim3(MEAS_SITES, 6), measure_smem_bytes<R>(), ctx_->stream>>>(
-                    d_desc_, d_mtiles_, segs + j, MeasOut{});
+            k_meas_loops<R, ROUND><<<lg, dim3(MEAS_SITES, 3 * meas_groups_), loops_smem_bytes(meas_groups_), ctx_->stream>>>(
+                d_desc_, d_mtiles_, tiles + j);
+            k_meas_planes<R, ROUND, OUT><<<pg, unit_sites_, planes_smem_bytes<R>(unit_sites_), ctx_->stream>>>(
+                d_desc_, members, d_sel_, units + j, out);
         }
     }
 
     int capture_one(bool step, int nseg, cudaGraphExec_t* out) {
         cudaGraph_t graph = nullptr;
         LGF_CUDA_TRY(ctx_, cudaStreamBeginCapture(ctx_->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = step ? launch_stages(nseg) : launch_measurement(nseg);
+        int rc = step ? launch_stages(nseg) : launch_measurement(nseg, meas_small_);
         cudaError_t e = cudaStreamEndCapture(ctx_->stream, &graph);
         if (rc != LGF_OK) {
             if (graph) cudaGraphDestroy(graph);
@@ -609,11 +674,13 @@ private:
     long long mtiles_cap_ = 0, rtiles_cap_ = 0;
     int jobs_cap_ = 0;
     int ntiles_ = 0;
-    int stage_grid_max_ = 1, meas_grid_max_ = 1;
+    int stage_grid_max_ = 1, small_grid_max_ = 1, loops_grid_max_ = 1, planes_grid_max_ = 1;
+    int meas_groups_ = LOOP_MAX_GROUPS, unit_sites_ = PLANE_MAX_SITES;  // tiles per loops block, sites per plane unit
     int slots_;                                   // launch slots per kernel (member_runs)
     int stage_nseg_ = 1, meas_nseg_ = 1;           // launch segments in use
+    bool meas_small_ = false;                      // some measured lattice takes the one-launch kernel
     int2* d_seg_ = nullptr;                        // the stage's launch segments
-    std::vector<cudaGraphExec_t> step_execs_, meas_execs_;  // by segment count
+    std::vector<cudaGraphExec_t> step_execs_, meas_execs_;  // by segment count (and small lattices)
 };
 
 GroupBase* make_group(lgf_ctx* ctx, int precision, const TileShape& shape, int max_members, long long max_tiles,
@@ -810,47 +877,6 @@ int download_links(lgf_ctx* ctx, const LatticeBuf& b, double* host) {
 using namespace lgf;
 
 
-// One measurement-kernel pass over a single lattice with per-site (and,
-// when asked, per (site, plane) F / F^) outputs; no reduction.
-template <typename R> static int single_lattice_measure(lgf_ctx* ctx, LatticeBuf& b, const MeasOut& out) {
-    std::vector<int4> mt;
-    for (int t = 0; t < b.g.n[0]; ++t)
-        for (int c = 0; c < b.nchunk; ++c) mt.push_back(make_int4(0, t, c, 0));
-    const int n = (int)mt.size();
-    LatDesc<R> d{};
-    d.g = b.g;
-    d.U0 = (cplx<R>*)b.U[0];
-    d.partial = b.partial;
-    d.nchunk = b.nchunk;
-    void* ddesc = nullptr;
-    int4* dmt = nullptr;
-    int2* dn = nullptr;
-    const int2 seg = make_int2(0, n);
-    cudaError_t e = prepare_measure_kernel<R, true>();
-    if (e == cudaSuccess) e = cudaMalloc(&ddesc, sizeof d);
-    if (e == cudaSuccess) e = cudaMalloc(&dmt, sizeof(int4) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&dn, sizeof(int2));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ddesc, &d, sizeof d, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dmt, mt.data(), sizeof(int4) * n, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dn, &seg, sizeof(int2), cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) {
-        k_measure<R, true><<<std::min(n, 4 * ctx->sm_count), dim3(MEAS_SITES, MEAS_WARPS), measure_smem_bytes<R, true>(),
-                             ctx->stream>>>((const LatDesc<R>*)ddesc, dmt, dn, out);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(ddesc);
-    cudaFree(dmt);
-    cudaFree(dn);
-    if (e != cudaSuccess) return set_error(ctx, LGF_ECUDA, "measurement pass failed: %s", cudaGetErrorString(e));
-    return LGF_OK;
-}
-
-static int single_measure(lgf_ctx* ctx, LatticeBuf& b, const MeasOut& out) {
-    return b.prec == LGF_PREC_FP64 ? single_lattice_measure<double>(ctx, b, out)
-                                   : single_lattice_measure<float>(ctx, b, out);
-}
-
 // =================================================================== C ABI
 extern "C" {
 
@@ -977,6 +1003,17 @@ static int lattice_group(lgf_lattice* lat, GroupBase** out) {
     return LGF_OK;
 }
 
+// One measurement pass over a lattice's links with per-site (and, when asked,
+// per (site, plane) F / F^) outputs.
+static int single_measure(lgf_lattice* lat, const MeasSites& out) {
+    GroupBase* grp = nullptr;
+    int rc = lattice_group(lat, &grp);
+    if (rc == LGF_OK) rc = grp->launch_sites(out);
+    if (rc != LGF_OK) return rc;
+    LGF_CUDA_TRY(lat->ctx, cudaStreamSynchronize(lat->ctx->stream));
+    return LGF_OK;
+}
+
 static int fetch_meas(lgf_ctx* ctx, const LatticeBuf& b, int nmeas, std::vector<double>& host) {
     const size_t per = 2 + 2 * (size_t)b.g.n[0];
     host.resize(per * std::max(nmeas, 1));
@@ -1094,15 +1131,14 @@ int lgf_site_densities(lgf_lattice* lat, double* e_site, double* q_site) {
     if (!lat) return LGF_EINVAL;
     lgf_ctx* ctx = lat->ctx;
     cudaSetDevice(ctx->device);
-    LatticeBuf& b = lat->buf;
-    const size_t V = (size_t)b.g.V;
+    const size_t V = (size_t)lat->buf.g.V;
     double *de = nullptr, *dq = nullptr;
     LGF_CUDA_TRY(ctx, cudaMalloc(&de, V * sizeof(double)));
     cudaError_t e = cudaMalloc(&dq, V * sizeof(double));
-    MeasOut mo{};
+    MeasSites mo{};
     mo.e = de;
     mo.q = dq;
-    int rc = e == cudaSuccess ? single_measure(ctx, b, mo)
+    int rc = e == cudaSuccess ? single_measure(lat, mo)
                               : set_error(ctx, LGF_ENOMEM, "site density buffers: %s", cudaGetErrorString(e));
     if (rc == LGF_OK && e_site) e = cudaMemcpy(e_site, de, V * sizeof(double), cudaMemcpyDeviceToHost);
     if (rc == LGF_OK && e == cudaSuccess && q_site) e = cudaMemcpy(q_site, dq, V * sizeof(double), cudaMemcpyDeviceToHost);
@@ -1116,15 +1152,15 @@ int lgf_measure_flowed(lgf_lattice* lat, double* E_improved, double* Q_clover) {
     if (!lat) return LGF_EINVAL;
     lgf_ctx* ctx = lat->ctx;
     cudaSetDevice(ctx->device);
-    LatticeBuf& b = lat->buf;
-    const size_t V = (size_t)b.g.V;
+    const size_t V = (size_t)lat->buf.g.V;
     double *de = nullptr, *dq = nullptr;
     LGF_CUDA_TRY(ctx, cudaMalloc(&de, V * sizeof(double)));
     cudaError_t e = cudaMalloc(&dq, V * sizeof(double));
-    MeasOut mo{};
-    mo.e_imp = de;
-    mo.q_clov = dq;
-    int rc = e == cudaSuccess ? single_measure(ctx, b, mo)
+    MeasSites mo{};
+    mo.e = de;
+    mo.q = dq;
+    mo.swap = 1;  // e with the improved F, q with the clover F
+    int rc = e == cudaSuccess ? single_measure(lat, mo)
                               : set_error(ctx, LGF_ENOMEM, "density buffers: %s", cudaGetErrorString(e));
     std::vector<double> he(V), hq(V);
     if (rc == LGF_OK) e = cudaMemcpy(he.data(), de, V * sizeof(double), cudaMemcpyDeviceToHost);
@@ -1241,15 +1277,14 @@ int lgf_debug_fields(lgf_lattice* lat, double* clover_F, double* improved_F) {
     if (!lat) return LGF_EINVAL;
     lgf_ctx* ctx = lat->ctx;
     cudaSetDevice(ctx->device);
-    LatticeBuf& b = lat->buf;
-    const size_t bytes = (size_t)b.g.V * 6 * 18 * sizeof(double);
+    const size_t bytes = (size_t)lat->buf.g.V * 6 * 18 * sizeof(double);
     double2 *dc = nullptr, *di = nullptr;
     LGF_CUDA_TRY(ctx, cudaMalloc(&dc, bytes));
     cudaError_t e = cudaMalloc(&di, bytes);
-    MeasOut mo{};
+    MeasSites mo{};
     mo.dbg_clover = dc;
     mo.dbg_improved = di;
-    int rc = e == cudaSuccess ? single_measure(ctx, b, mo)
+    int rc = e == cudaSuccess ? single_measure(lat, mo)
                               : set_error(ctx, LGF_ENOMEM, "debug field buffers: %s", cudaGetErrorString(e));
     if (rc == LGF_OK && clover_F) e = cudaMemcpy(clover_F, dc, bytes, cudaMemcpyDeviceToHost);
     if (rc == LGF_OK && e == cudaSuccess && improved_F) e = cudaMemcpy(improved_F, di, bytes, cudaMemcpyDeviceToHost);

@@ -10,7 +10,7 @@
 #include <vector>
 
 #include "../../include/lgf_b200.h"
-#include "lgf_kernels.cuh"
+#include "lgf_measure.cuh"
 
 // NVTX ranges around the host-side launch points (RK3 steps, stages,
 // measurements), visible on an Nsight timeline; header-only NVTX is a no-op
@@ -39,7 +39,7 @@ struct TileShape {
     int stage_order = 1;          // 0: blocks of x1 rows swept through x0; 1: x1 columns per CTA
     double stage_budget = 8.0 * (1 << 20);  // blocked order: stage bytes per row block and slice
     double meas_budget = 2.0 * (1 << 20);   // measurement: link bytes per row block and slice
-    int meas_split = 2;           // measurement warps per plane (1: 6-warp blocks, 2: 12-warp blocks)
+    int meas_split = 2;           // measurement blocks (1: 6 warps, 2: 12 warps)
     bool operator==(const TileShape& o) const {
         return threads == o.threads && stage_order == o.stage_order && stage_budget == o.stage_budget &&
                meas_budget == o.meas_budget && meas_split == o.meas_split;
@@ -174,12 +174,14 @@ public:
     // the subset of members measured by the next measurement launch
     virtual int set_measured(const std::vector<int>& which) = 0;
     virtual int launch_step() = 0;       // one RK3 step of every member (3 stage launches)
-    virtual int launch_measure() = 0;    // measurement of the measured subset (3 launches)
+    virtual int launch_measure() = 0;    // measurement of the measured subset
+    virtual int launch_sites(const MeasSites& out) = 0;  // the same pass with per-site outputs, no reduction
     virtual int launch_one(int k) = 0;   // one kernel alone: stage k+1 (k<3) or the measurement kernel
     virtual int capture() = 0;           // capture step and measurement graphs
     virtual int replay_step() = 0;       // graph launch (captures on first use)
     virtual int replay_measure() = 0;
     virtual int launches_per_step() const = 0;
+    virtual int launches_per_measure() const = 0;
     virtual int threads() const = 0;
     virtual const TileShape& shape() const = 0;
 };

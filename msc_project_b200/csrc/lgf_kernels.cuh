@@ -8,9 +8,10 @@
 //                      (LGF/Field/SU3_field.cpp:519-530), HermTrLessExp
 //                      (LGF/Math/SU3_mat.cpp:216-289) and the three update
 //                      loops of GradientFlow::flow (GradientFlow.cpp:22-54).
-//   k_measure<R>       clover F (E) and improved F (q) for every site and plane,
-//                      per-site e(x), q(x), warp-shuffle block partials by
-//                      x0 slice.  Replaces EnergyDensity::calculate and
+//   k_measure<R>       small lattices: clover F (E) and improved F (q) for every
+//                      site and plane in one launch, per-site e(x), q(x),
+//                      warp-shuffle block partials by x0 slice (the others:
+//                      lgf_measure.cuh).  Replaces EnergyDensity::calculate and
 //                      TopologicalCharge::calculate (Observables/*.cpp) and the
 //                      loop averages of SU3_field.cpp:533-792.
 //   k_reduce_slices / k_reduce_total
@@ -38,9 +39,6 @@
 #endif
 #ifndef LGF_STAGE_MINB
 #define LGF_STAGE_MINB 1
-#endif
-#ifndef LGF_MEAS_QSPLIT
-#define LGF_MEAS_QSPLIT 2  // default measurement warps per plane (the four quadrants split between them)
 #endif
 
 namespace lgf {
@@ -218,30 +216,31 @@ struct PlanePos { int s, xm, xn; };
 #define LGF_MEAS_ROW3 1  // path products of the measurement rebuild their third row (mul_nn_su3)
 #endif
 
-template <typename R> struct Plane {
+// Links are read in R and multiplied in D.
+template <typename R, typename D = R> struct Plane {
     const cplx<R>* __restrict__ U;
     int V, mu, nu;
     Dir dm, dn;  // .x unused: positions carry their own coordinates
 
     // the link of one step from p and the new position; adjoint for a backward step
-    __device__ __forceinline__ su3<R> step(PlanePos& p, bool along_mu, int sign) const {
+    __device__ __forceinline__ su3<D> step(PlanePos& p, bool along_mu, int sign) const {
         const Dir& d = along_mu ? dm : dn;
         int& xc = along_mu ? p.xm : p.xn;
         const int dir = along_mu ? mu : nu;
         if (sign > 0) {
-            su3<R> l = load_link(U, V, dir, p.s);
+            su3<D> l = su3_cast<D>(load_link(U, V, dir, p.s));
             p.s = (xc == d.n - 1) ? p.s - (d.n - 1) * d.stride : p.s + d.stride;
             xc = wrap_inc(xc, d.n);
             return l;
         }
         p.s = (xc == 0) ? p.s + (d.n - 1) * d.stride : p.s - d.stride;
         xc = wrap_dec(xc, d.n);
-        su3<R> l = load_link(U, V, dir, p.s);
-        su3<R> a;
+        su3<D> l = su3_cast<D>(load_link(U, V, dir, p.s));
+        su3<D> a;
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) a.m[3 * r + c] = cmk<R>(l.m[3 * c + r].re, -l.m[3 * c + r].im);
+            for (int c = 0; c < 3; ++c) a.m[3 * r + c] = cmk<D>(l.m[3 * c + r].re, -l.m[3 * c + r].im);
         return a;
     }
     // move p by count steps without loading links
@@ -259,19 +258,19 @@ template <typename R> struct Plane {
         }
     }
     // P <- P * (link of one step from p)
-    __device__ __forceinline__ void ext(su3<R>& P, PlanePos& p, bool along_mu, int sign) const {
+    __device__ __forceinline__ void ext(su3<D>& P, PlanePos& p, bool along_mu, int sign) const {
         const Dir& d = along_mu ? dm : dn;
         int& xc = along_mu ? p.xm : p.xn;
         const int dir = along_mu ? mu : nu;
         if (sign > 0) {
-            const su3<R> l = load_link(U, V, dir, p.s);
+            const su3<D> l = su3_cast<D>(load_link(U, V, dir, p.s));
             p.s = (xc == d.n - 1) ? p.s - (d.n - 1) * d.stride : p.s + d.stride;
             xc = wrap_inc(xc, d.n);
             P = LGF_MEAS_ROW3 ? mul_nn_su3(P, l) : mul_nn(P, l);
         } else {
             p.s = (xc == 0) ? p.s + (d.n - 1) * d.stride : p.s - d.stride;
             xc = wrap_dec(xc, d.n);
-            const su3<R> l = load_link(U, V, dir, p.s);
+            const su3<D> l = su3_cast<D>(load_link(U, V, dir, p.s));
             P = LGF_MEAS_ROW3 ? mul_na_su3(P, l) : mul_na(P, l);
         }
     }
@@ -420,16 +419,10 @@ template <typename R> struct PathStash {
     }
 };
 
-constexpr int MEAS_QSPLIT = LGF_MEAS_QSPLIT;
-constexpr int MEAS_WARPS = 6 * MEAS_QSPLIT;  // warp y: plane y % 6, quadrants of part y / 6
-// resident measurement blocks per SM the launch bounds ask for (caps the
-// registers): one block of 12 warps with the quadrants split, else two of 6
-template <int QS> struct MeasMinBlocks { static constexpr int value = QS == 2 ? 1 : 2; };
-
 // Shared memory of one measurement block: the straight lines of length 2 and
 // 3 from each of its 32 sites in the 8 signed directions (every plane and
 // quadrant of the site reuses them), then the per-plane results.
-template <typename R, bool OUT> struct MeasSmem {
+template <typename R> struct MeasSmem {
     union {
         R line[8][2][2 * MEAS_STASH_ENTRIES][MEAS_SITES];  // [2*dir + (sign<0)][length-2][real of entry][site]
         struct {                       // after the lines are dead: the second quadrant half's sums
@@ -440,36 +433,34 @@ template <typename R, bool OUT> struct MeasSmem {
     R acc[meas_smem_acc<R>() ? 16 : 1][meas_smem_acc<R>() ? MEAS_ACC_STRIDE : 1];  // G, Fhat columns (LGF_MEAS_SMEM_ACC)
     typename vec2_of<R>::type stash[2][MEAS_STASH_ENTRIES][MEAS_ACC_STRIDE];  // two paths per thread (PathStash)
     alg<R> F[6][MEAS_SITES];          // improved F per plane
-    alg<R> C[OUT ? 6 : 1][MEAS_SITES];  // clover F per plane (single-lattice passes only)
     double E[6][MEAS_SITES];
 };
 
-// Optional per-site / per-(site, plane) outputs of a measurement pass (all
-// null in the flow).  e, q: the densities of E and Q; e_imp, q_clov: the
-// energy density with the improved F (ImprovedEnergyDensity.cpp:13-20) and
-// the charge density with the clover F (UnImprovedTopologicalCharge.cpp:11-16);
-// dbg_*: F and F^ as Hermitian 3x3 matrices per (site, plane).
-struct MeasOut {
+// What a measurement pass may write besides the sums (single-lattice calls;
+// all null in the flow): e, q the site densities; swap: e with the improved F
+// and q with the clover F (ImprovedEnergyDensity.cpp:13-20,
+// UnImprovedTopologicalCharge.cpp:11-16); dbg_*: F and F^ as Hermitian 3x3
+// matrices per (site, plane).
+struct MeasSites {
     double* e;
     double* q;
-    double* e_imp;
-    double* q_clov;
+    int swap;
     double2* dbg_clover;
     double2* dbg_improved;
 };
 
 // A line is only ever extended (the left operand of a product that rebuilds
 // the third row), so like a parked path it keeps its first two rows.
-template <typename R, bool OUT>
-__device__ __forceinline__ void store_line(MeasSmem<R, OUT>* sm, int sdir, int len, int lane, const su3<R>& L) {
+template <typename R>
+__device__ __forceinline__ void store_line(MeasSmem<R>* sm, int sdir, int len, int lane, const su3<R>& L) {
 #pragma unroll
     for (int k = 0; k < MEAS_STASH_ENTRIES; ++k) {
         sm->line[sdir][len - 2][2 * k][lane] = L.m[k].re;
         sm->line[sdir][len - 2][2 * k + 1][lane] = L.m[k].im;
     }
 }
-template <typename R, bool OUT>
-__device__ __forceinline__ su3<R> load_line(const MeasSmem<R, OUT>* sm, int sdir, int len, int lane) {
+template <typename R>
+__device__ __forceinline__ su3<R> load_line(const MeasSmem<R>* sm, int sdir, int len, int lane) {
     su3<R> L;
 #pragma unroll
     for (int k = 0; k < 9; ++k)
@@ -478,10 +469,6 @@ __device__ __forceinline__ su3<R> load_line(const MeasSmem<R, OUT>* sm, int sdir
                      : cmk<R>(R(0), R(0));  // never read: the next product rebuilds the row
     return L;
 }
-
-#ifndef LGF_MEAS_REUSE
-#define LGF_MEAS_REUSE 1  // paths extended from parked shorter paths: 12 products per quadrant instead of 15
-#endif
 
 // Quadrants [qa, qb) of plane (mu, nu) at the thread's site, using the
 // block's shared lines: G = the sum of the 1x1 leaves' projections, Fhat =
@@ -496,12 +483,10 @@ __device__ __forceinline__ su3<R> load_line(const MeasSmem<R, OUT>* sm, int sdir
 // 12 matrix products and 14 global link loads per quadrant; the paths that
 // are extended after other work are parked in the thread's shared-memory
 // column (PathStash: Pm(1,1), Pm(2,1), Pn(1,2)), and the leaves are added in
-// the order (1,1) | (2,1), (3,1), (1,2), (1,3), (2,2), the order of the
-// 15-product form (LGF_MEAS_REUSE=0), whose every product it repeats: both
-// give the same bits.
-template <typename R, bool OUT, typename Acc>
+// the order (1,1) | (2,1), (3,1), (1,2), (1,3), (2,2).
+template <typename R, typename Acc>
 __device__ __forceinline__ void plane_fields_body(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c,
-                                                  int mu, int nu, const MeasSmem<R, OUT>* sm, int lane, int qa, int qb,
+                                                  int mu, int nu, const MeasSmem<R>* sm, int lane, int qa, int qb,
                                                   Acc G, Acc Fhat, PathStash<R> sa, PathStash<R> sb) {
     Plane<R> P;
     P.U = U;
@@ -523,162 +508,95 @@ __device__ __forceinline__ void plane_fields_body(const cplx<R>* __restrict__ U,
         const int sn = (q == 0 || q == 2) ? 1 : -1;
         const R sg = (q == 0 || q == 3) ? R(1) : R(-1);
         const int sdm = 2 * mu + (sm_ < 0 ? 1 : 0), sdn = 2 * nu + (sn < 0 ? 1 : 0);
-        if (LGF_MEAS_REUSE) {
-            // (1,1)
-            PlanePos pn = x0;
-            su3<R> Pn = P.step(pn, false, sn);
-            P.ext(Pn, pn, true, sm_);  // Pn(1,1)
-            PlanePos pm = x0;
-            su3<R> Pm = P.step(pm, true, sm_);
-            P.ext(Pm, pm, false, sn);  // Pm(1,1), pm at x + m + n
-            leaf_acc(Pn, Pm, sg, G);
-            sa.put(Pm);
-            // (2,1)
-            P.ext(Pn, pn, true, sm_);  // Pn(2,1)
-            PlanePos p21 = x0;
-            P.advance(p21, true, sm_, 2);
-            Pm = load_line(sm, sdm, 2, lane);
-            P.ext(Pm, p21, false, sn);  // Pm(2,1), p21 at x + 2m + n
-            leaf_acc(Pn, Pm, sg * k12, Fhat);
-            sb.put(Pm);
-            // (3,1)
-            P.ext(Pn, pn, true, sm_);  // Pn(3,1)
-            PlanePos p31 = x0;
-            P.advance(p31, true, sm_, 3);
-            Pm = load_line(sm, sdm, 3, lane);
-            P.ext(Pm, p31, false, sn);  // Pm(3,1)
-            leaf_acc(Pn, Pm, sg * k13, Fhat);
-            // (1,2)
-            Pm = sa.get();
-            P.ext(Pm, pm, false, sn);  // Pm(1,2)
-            PlanePos p12 = x0;
-            P.advance(p12, false, sn, 2);
-            Pn = load_line(sm, sdn, 2, lane);
-            P.ext(Pn, p12, true, sm_);  // Pn(1,2), p12 at x + 2n + m
-            leaf_acc(Pn, Pm, sg * k12, Fhat);
-            sa.put(Pn);
-            // (1,3)
-            P.ext(Pm, pm, false, sn);  // Pm(1,3)
-            PlanePos p13 = x0;
-            P.advance(p13, false, sn, 3);
-            Pn = load_line(sm, sdn, 3, lane);
-            P.ext(Pn, p13, true, sm_);  // Pn(1,3)
-            leaf_acc(Pn, Pm, sg * k13, Fhat);
-            // (2,2)
-            Pn = sa.get();
-            P.ext(Pn, p12, true, sm_);  // Pn(2,2)
-            Pm = sb.get();
-            P.ext(Pm, p21, false, sn);  // Pm(2,2)
-            leaf_acc(Pn, Pm, sg * k22, Fhat);
-            continue;
-        }
-        // row: (1,1), (2,1), (3,1)
+        // (1,1)
         PlanePos pn = x0;
-        su3<R> Rn = P.step(pn, false, sn);
-        P.ext(Rn, pn, true, sm_);  // Pn(1,1)
-        {
-            PlanePos q2 = x0;
-            su3<R> Pm = P.step(q2, true, sm_);
-            P.ext(Pm, q2, false, sn);  // Pm(1,1)
-            leaf_acc(Rn, Pm, sg, G);
-        }
-        P.ext(Rn, pn, true, sm_);  // Pn(2,1)
-        {
-            PlanePos q2 = x0;
-            P.advance(q2, true, sm_, 2);
-            su3<R> Pm = load_line(sm, sdm, 2, lane);
-            P.ext(Pm, q2, false, sn);  // Pm(2,1)
-            leaf_acc(Rn, Pm, sg * k12, Fhat);
-        }
-        P.ext(Rn, pn, true, sm_);  // Pn(3,1)
-        {
-            PlanePos q2 = x0;
-            P.advance(q2, true, sm_, 3);
-            su3<R> Pm = load_line(sm, sdm, 3, lane);
-            P.ext(Pm, q2, false, sn);  // Pm(3,1)
-            leaf_acc(Rn, Pm, sg * k13, Fhat);
-        }
-        // column: (1,2), (1,3)
-        {
-            PlanePos qm = x0;
-            su3<R> Lm = P.step(qm, true, sm_);
-            P.ext(Lm, qm, false, sn);
-            P.ext(Lm, qm, false, sn);  // Pm(1,2)
-            PlanePos q2 = x0;
-            P.advance(q2, false, sn, 2);
-            su3<R> Pn = load_line(sm, sdn, 2, lane);
-            P.ext(Pn, q2, true, sm_);  // Pn(1,2)
-            leaf_acc(Pn, Lm, sg * k12, Fhat);
-            P.ext(Lm, qm, false, sn);  // Pm(1,3)
-            PlanePos q3 = x0;
-            P.advance(q3, false, sn, 3);
-            Pn = load_line(sm, sdn, 3, lane);
-            P.ext(Pn, q3, true, sm_);  // Pn(1,3)
-            leaf_acc(Pn, Lm, sg * k13, Fhat);
-        }
+        su3<R> Pn = P.step(pn, false, sn);
+        P.ext(Pn, pn, true, sm_);  // Pn(1,1)
+        PlanePos pm = x0;
+        su3<R> Pm = P.step(pm, true, sm_);
+        P.ext(Pm, pm, false, sn);  // Pm(1,1), pm at x + m + n
+        leaf_acc(Pn, Pm, sg, G);
+        sa.put(Pm);
+        // (2,1)
+        P.ext(Pn, pn, true, sm_);  // Pn(2,1)
+        PlanePos p21 = x0;
+        P.advance(p21, true, sm_, 2);
+        Pm = load_line(sm, sdm, 2, lane);
+        P.ext(Pm, p21, false, sn);  // Pm(2,1), p21 at x + 2m + n
+        leaf_acc(Pn, Pm, sg * k12, Fhat);
+        sb.put(Pm);
+        // (3,1)
+        P.ext(Pn, pn, true, sm_);  // Pn(3,1)
+        PlanePos p31 = x0;
+        P.advance(p31, true, sm_, 3);
+        Pm = load_line(sm, sdm, 3, lane);
+        P.ext(Pm, p31, false, sn);  // Pm(3,1)
+        leaf_acc(Pn, Pm, sg * k13, Fhat);
+        // (1,2)
+        Pm = sa.get();
+        P.ext(Pm, pm, false, sn);  // Pm(1,2)
+        PlanePos p12 = x0;
+        P.advance(p12, false, sn, 2);
+        Pn = load_line(sm, sdn, 2, lane);
+        P.ext(Pn, p12, true, sm_);  // Pn(1,2), p12 at x + 2n + m
+        leaf_acc(Pn, Pm, sg * k12, Fhat);
+        sa.put(Pn);
+        // (1,3)
+        P.ext(Pm, pm, false, sn);  // Pm(1,3)
+        PlanePos p13 = x0;
+        P.advance(p13, false, sn, 3);
+        Pn = load_line(sm, sdn, 3, lane);
+        P.ext(Pn, p13, true, sm_);  // Pn(1,3)
+        leaf_acc(Pn, Pm, sg * k13, Fhat);
         // (2,2)
-        {
-            PlanePos q2 = x0;
-            P.advance(q2, false, sn, 2);
-            su3<R> Pn = load_line(sm, sdn, 2, lane);
-            P.ext(Pn, q2, true, sm_);
-            P.ext(Pn, q2, true, sm_);  // Pn(2,2)
-            PlanePos qm = x0;
-            P.advance(qm, true, sm_, 2);
-            su3<R> Pm = load_line(sm, sdm, 2, lane);
-            P.ext(Pm, qm, false, sn);
-            P.ext(Pm, qm, false, sn);  // Pm(2,2)
-            leaf_acc(Pn, Pm, sg * k22, Fhat);
-        }
+        Pn = sa.get();
+        P.ext(Pn, p12, true, sm_);  // Pn(2,2)
+        Pm = sb.get();
+        P.ext(Pm, p21, false, sn);  // Pm(2,2)
+        leaf_acc(Pn, Pm, sg * k22, Fhat);
     }
 }
 
-template <typename R, bool OUT>
+template <typename R>
 __device__ __forceinline__ void plane_fields_smem(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c,
-                                                  int mu, int nu, MeasSmem<R, OUT>* sm, int lane, int qa, int qb,
+                                                  int mu, int nu, MeasSmem<R>* sm, int lane, int qa, int qb,
                                                   alg<R>& Greg, alg<R>& Fhreg) {
     const int column = threadIdx.y * MEAS_SITES + lane;
     const PathStash<R> sa{&sm->stash[0][0][column]}, sb{&sm->stash[1][0][column]};
     if constexpr (meas_smem_acc<R>()) {
         R* col = &sm->acc[0][column];
         const SmemAcc<R> G{col}, Fhat{col + 8 * MEAS_ACC_STRIDE};
-        plane_fields_body<R, OUT>(U, g, s, c, mu, nu, sm, lane, qa, qb, G, Fhat, sa, sb);
+        plane_fields_body<R>(U, g, s, c, mu, nu, sm, lane, qa, qb, G, Fhat, sa, sb);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             Greg.v[k] = G.get(k);
             Fhreg.v[k] = Fhat.get(k);
         }
     } else {
-        plane_fields_body<R, OUT>(U, g, s, c, mu, nu, sm, lane, qa, qb, RegAcc<R>{Greg}, RegAcc<R>{Fhreg}, sa, sb);
+        plane_fields_body<R>(U, g, s, c, mu, nu, sm, lane, qa, qb, RegAcc<R>{Greg}, RegAcc<R>{Fhreg}, sa, sb);
     }
 }
 
-// Measurement tile = (lattice, x0 slice, chunk of 32 consecutive sites of the
-// slice); 6 x QS warps: warp y takes plane y % 6 and the quadrants of part
-// y / 6 (QS = 1: all four; QS = 2: two each).  Phase 0: the block's lines
-// (warp w builds the lines of signed direction w, w + 6 QS, ...) into shared
-// memory.  Phase 1: the
-// quadrant sums of every (site, plane); with two parts the second part's sums
+// Measurement of small lattices in one launch (small_measure, lgf_measure.cuh).
+// Tile = (lattice, x0 slice, chunk of 32 consecutive sites of the slice); 12
+// warps: warp y takes plane y % 6 and two of the four quadrants (part y / 6).
+// Phase 0: the block's lines (a warp per signed direction) into shared memory.
+// Phase 1: the quadrant sums of every (site, plane); the second part's sums
 // meet the first's in the (then dead) line storage, in a fixed order, for F
-// and F^.  Phase 2: the six planes meet in shared
-// memory for e(x) and q(x); the tile's sums go to the lattice's
-// partial[slice * nchunk + chunk] (double2).  The optional outputs of
-// MeasOut (single-lattice passes) receive per-site densities and per
-// (site, plane) F and F^.
+// and F^.  Phase 2: the six planes meet in shared memory for e(x) and q(x);
+// the tile's sums go to the lattice's partial[slice * nchunk + chunk].
 //   e(x) = sum_{mu<nu} ReTr(F F)                 (EnergyDensity.cpp:13-20)
 //   q(x) = ReTr(F^32 F^01) + ReTr(F^31 F^20) + ReTr(F^30 F^12)
 //        = -T(23,01) + T(13,02) - T(03,12),  T(a,b) = ReTr(F^a F^b)
 //                                             (TopologicalCharge.cpp:11-16)
-template <typename R, bool OUT = false, int QS = MEAS_QSPLIT>
-__global__ void __launch_bounds__(MEAS_SITES * 6 * QS, MeasMinBlocks<QS>::value) k_measure(const LatDesc<R>* __restrict__ descs,
-                                                                           const int4* __restrict__ mtiles,
-                                                                           const int2* __restrict__ seg,
-                                                                           MeasOut out) {
+constexpr int MEAS_WARPS = 12;
+template <typename R, bool OUT>
+__global__ void __launch_bounds__(MEAS_SITES * MEAS_WARPS, 1) k_measure(const LatDesc<R>* __restrict__ descs,
+                                                                       const int4* __restrict__ mtiles,
+                                                                       const int2* __restrict__ seg, MeasSites out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    MeasSmem<R, OUT>* sm = reinterpret_cast<MeasSmem<R, OUT>*>(smem_raw);
+    MeasSmem<R>* sm = reinterpret_cast<MeasSmem<R>*>(smem_raw);
     const int lane = threadIdx.x, w = threadIdx.y, p = w % 6, part = w / 6;
-    constexpr int NW = 6 * QS;  // warps of the block
-    const int qa = part * 2, qb = qa + 2;  // QS = 2: this warp's quadrant half
     const int2 r = *seg;  // this launch's tiles: mtiles[r.x, r.x + r.y)
     for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
         const int4 tile = mtiles[ti];
@@ -691,8 +609,8 @@ __global__ void __launch_bounds__(MEAS_SITES * 6 * QS, MeasMinBlocks<QS>::value)
         const Coord c = site_coord(g, s);
         const cplx<R>* __restrict__ U = d->U0;
         // phase 0: lines of length 2 and 3 in the 8 signed directions
-        for (int sdir = w; sdir < 8; sdir += NW) {
-            const int dir = sdir >> 1, sign = (sdir & 1) ? -1 : 1;
+        if (w < 8) {
+            const int dir = w >> 1, sign = (w & 1) ? -1 : 1;
             Plane<R> L;
             L.U = U;
             L.V = g.V;
@@ -703,61 +621,41 @@ __global__ void __launch_bounds__(MEAS_SITES * 6 * QS, MeasMinBlocks<QS>::value)
             PlanePos y = {s, L.dm.x, L.dm.x};
             su3<R> acc = L.step(y, true, sign);
             L.ext(acc, y, true, sign);
-            store_line(sm, sdir, 2, lane, acc);
+            store_line(sm, w, 2, lane, acc);
             L.ext(acc, y, true, sign);
-            store_line(sm, sdir, 3, lane, acc);
+            store_line(sm, w, 3, lane, acc);
         }
         __syncthreads();
-        // phase 1: this thread's plane and quadrants; with one warp per plane
-        // the two quadrant halves are still summed apart and then added, the
-        // order two warps per plane use, so both give the same bits
+        // phase 1: this thread's plane and quadrants
         alg<R> G, Fh;
-        if (valid) {
-            if (QS == 1) {
-#pragma unroll 1
-                for (int h = 0; h < 2; ++h) {
-                    alg<R> G1, F1;
-                    plane_fields_smem<R, OUT>(U, g, s, c, c_plane_mu[p], c_plane_nu[p], sm, lane, 2 * h, 2 * h + 2, G1, F1);
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        G.v[k] = h ? G.v[k] + G1.v[k] : G1.v[k];
-                        Fh.v[k] = h ? Fh.v[k] + F1.v[k] : F1.v[k];
-                    }
-                }
-            } else {
-                plane_fields_smem<R, OUT>(U, g, s, c, c_plane_mu[p], c_plane_nu[p], sm, lane, qa, qb, G, Fh);
-            }
+        if (valid) plane_fields_smem<R>(U, g, s, c, c_plane_mu[p], c_plane_nu[p], sm, lane, 2 * part, 2 * part + 2, G, Fh);
+        __syncthreads();  // every warp is done with the lines
+        if (part == 1 && valid) {
+            sm->part.G[p][lane] = G;
+            sm->part.Fh[p][lane] = Fh;
         }
-        if (QS == 2) {
-            __syncthreads();  // every warp is done with the lines
-            if (part == 1 && valid) {
-                sm->part.G[p][lane] = G;
-                sm->part.Fh[p][lane] = Fh;
-            }
-            __syncthreads();
-            if (part == 0 && valid) {
-                const alg<R> G1 = sm->part.G[p][lane], F1 = sm->part.Fh[p][lane];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    G.v[k] += G1.v[k];
-                    Fh.v[k] += F1.v[k];
-                }
-            }
-        }
+        __syncthreads();
         if (part == 0 && valid) {
+            const alg<R> G1 = sm->part.G[p][lane], F1 = sm->part.Fh[p][lane];
             alg<R> F11;
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
+                G.v[k] += G1.v[k];
+                Fh.v[k] += F1.v[k];
                 F11.v[k] = R(0.25) * G.v[k];
                 Fh.v[k] = fma(R(19.0 / 36.0), G.v[k], Fh.v[k]);
             }
-            sm->F[p][lane] = Fh;
-            sm->E[p][lane] = retr_hh(F11, F11);
             if (OUT) {
-                sm->C[p][lane] = F11;
                 if (out.dbg_clover) store_alg_as_herm(out.dbg_clover + ((size_t)s * 6 + p) * 9, F11);
                 if (out.dbg_improved) store_alg_as_herm(out.dbg_improved + ((size_t)s * 6 + p) * 9, Fh);
+                if (out.swap) {
+                    const alg<R> z = F11;
+                    F11 = Fh;
+                    Fh = z;
+                }
             }
+            sm->F[p][lane] = Fh;
+            sm->E[p][lane] = retr_hh(F11, F11);
         }
         __syncthreads();
         // phase 2: the site's e(x), q(x) and the tile's sums
@@ -768,17 +666,10 @@ __global__ void __launch_bounds__(MEAS_SITES * 6 * QS, MeasMinBlocks<QS>::value)
                     (sm->E[4][lane] + sm->E[5][lane]);
                 q = -retr_hh(sm->F[5][lane], sm->F[0][lane]) + retr_hh(sm->F[4][lane], sm->F[1][lane]) -
                     retr_hh(sm->F[2][lane], sm->F[3][lane]);
-                if (OUT && out.e) out.e[s] = e;
-                if (OUT && out.q) out.q[s] = q;
-                if (OUT && out.e_imp) {
-                    double ei = 0.0;
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) ei += retr_hh(sm->F[k][lane], sm->F[k][lane]);
-                    out.e_imp[s] = ei;
+                if (OUT) {
+                    if (out.e) out.e[s] = e;
+                    if (out.q) out.q[s] = q;
                 }
-                if (OUT && out.q_clov)
-                    out.q_clov[s] = -retr_hh(sm->C[5][lane], sm->C[0][lane]) + retr_hh(sm->C[4][lane], sm->C[1][lane]) -
-                                    retr_hh(sm->C[2][lane], sm->C[3][lane]);
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -791,13 +682,9 @@ __global__ void __launch_bounds__(MEAS_SITES * 6 * QS, MeasMinBlocks<QS>::value)
     }
 }
 
-// Dynamic shared memory of k_measure<R> (above 48 KB for double: the
-// attribute must be raised once per device before the first launch).
-template <typename R, bool OUT = false> inline size_t measure_smem_bytes() { return sizeof(MeasSmem<R, OUT>); }
-template <typename R, bool OUT = false, int QS = MEAS_QSPLIT> inline cudaError_t prepare_measure_kernel() {
-    return cudaFuncSetAttribute(k_measure<R, OUT, QS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(MeasSmem<R, OUT>));
-}
+// Dynamic shared memory of k_measure<R> (above 48 KB: raised with the kernel's
+// attribute before the first launch).
+template <typename R> inline size_t measure_smem_bytes() { return sizeof(MeasSmem<R>); }
 
 constexpr int RED_THREADS = 256;
 

@@ -55,6 +55,12 @@ template <typename R> __host__ __device__ __forceinline__ cplx<R> ccfma(cplx<R> 
 
 template <typename R> struct su3 { cplx<R> m[9]; };
 
+template <typename D, typename R> __host__ __device__ __forceinline__ su3<D> su3_cast(const su3<R>& a) {
+    su3<D> b;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) b.m[k] = cmk<D>((D)a.m[k].re, (D)a.m[k].im);
+    return b;
+}
 template <typename R> __host__ __device__ __forceinline__ void su3_zero(su3<R>& a) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) a.m[k] = cmk<R>(R(0), R(0));

@@ -9,7 +9,7 @@
 //   stage:       block size {128, 256, 384},
 //                then the tile order {x1 columns per CTA, row blocks through
 //                x0}, then (row blocks) the block budget {2, 8, 32 MB};
-//   measurement: warps per plane {2, 1}, then the block budget {2, 8, 64 MB}.
+//   measurement: blocks of {12, 6} warps, then the block budget {2, 8, 64 MB}.
 // The winner is recorded in the context and used by every later group whose
 // largest lattice falls in the same volume class (within a factor of two).
 // No candidate changes a result: only block shapes and tile order differ.
@@ -108,10 +108,9 @@ int tune_shape(lgf_ctx* ctx, int prec, const int shape[4], TileShape* best) {
             t.stage_budget = mb * MB;
             try_stage(t);
         }
-    // ---- measurement kernel alone, starting from whole-slice blocks (the
-    // fewest DRAM bytes: 1.16x the link bytes against 2.05x for 2 MB blocks
-    // on 24^3x48); smaller blocks replace them only when 2% faster (on 48^4
-    // whole slices no longer fit L2 and are 45% slower)
+    // ---- measurement kernels alone, starting from whole-slice blocks (the
+    // fewest DRAM bytes for the loops' links); smaller blocks replace them
+    // only when 2% faster
     cur.meas_budget = 64.0 * MB;
     float meas_ms = 0.f;
     if (rc == LGF_OK) rc = time_shape(ctx, prec, b, cur, 3, 1, &probe);
