@@ -148,6 +148,13 @@ static void check_tiles(const Geom& g) {
     for (int T : {32, 64, 96}) {
         std::set<int> want;
         for (int s0 = 0; s0 < g.V; s0 += T) want.insert(s0);
+        {
+            std::vector<int2> tiles;
+            append_site_tiles(tiles, 2, g, T);
+            std::multiset<int> got;
+            for (const int2& t : tiles) got.insert(t.y);
+            CHECK(got.size() == want.size() && std::set<int>(got.begin(), got.end()) == want);
+        }
         for (double budget : {1.0e3, 2.0e4, 3.0e5, 8.0e6}) {
             std::vector<int2> tiles;
             append_stage_tiles(tiles, 3, g, T, budget, bps_stage);

@@ -8,6 +8,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <new>
 #include <string>
@@ -250,7 +251,7 @@ public:
           int slots)
         : ctx_(ctx), shape_(shape), threads_(shape.threads), max_members_(max_members), max_tiles_(max_tiles),
           dynamic_(dynamic), per_volume_(per_volume), slots_(std::max(1, std::min(slots, max_members))),
-          step_execs_(slots_ + 1, nullptr), meas_execs_(2 * (slots_ + 1), nullptr) {}
+          meas_execs_(2 * (slots_ + 1), nullptr) {}
     ~Group() override {
         cudaStreamSynchronize(ctx_->stream);  // the lists are in use until then
         drop_graphs();
@@ -267,20 +268,27 @@ public:
 
     int init() {
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_desc_, sizeof(LatDesc<R>) * max_members_));
-        LGF_CUDA_TRY(ctx_, cudaMalloc(&d_tiles_, sizeof(int2) * max_tiles_));
+        // a lattice takes staple tiles, or plaquette and update tiles
+        const long long cap_sites = max_tiles_ * (threads_ / 4);
+        tiles_cap_ = std::max(max_tiles_, sizeof(R) == sizeof(float) ? cap_sites / PLAQ_SITES + cap_sites / UPDATE_SITES + 2 * max_members_ : 0LL);
+        LGF_CUDA_TRY(ctx_, cudaMalloc(&d_tiles_, sizeof(int2) * tiles_cap_));
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_counts_, sizeof(int) * 4));
-        LGF_CUDA_TRY(ctx_, cudaMalloc(&d_seg_, sizeof(int2) * slots_));
+        LGF_CUDA_TRY(ctx_, cudaMalloc(&d_seg_, sizeof(int2) * 3 * slots_));
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_sel_, sizeof(int) * sel_ints(max_members_)));
         LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_counts_, 0, sizeof(int) * 4, ctx_->stream));
-        LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_seg_, 0, sizeof(int2) * slots_, ctx_->stream));
         LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_sel_, 0, sizeof(int) * sel_ints(max_members_), ctx_->stream));
         int nb = 0;
         LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_stage<R, 1>, threads_, 0));
         stage_grid_max_ = std::max(1, nb) * ctx_->sm_count;
+        if constexpr (sizeof(R) == sizeof(float)) {
+            LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_plaquettes<R, 1>, 6 * PLAQ_SITES, 0));
+            plaq_grid_max_ = std::max(1, nb) * ctx_->sm_count;
+            LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_update<R, 1>, 4 * UPDATE_SITES, 0));
+            update_grid_max_ = std::max(1, nb) * ctx_->sm_count;
+        }
         // Measurement blocks: 4 tiles (loops) and 384 sites (planes) per block,
         // halved for one-warp-per-plane shapes, and smaller for lattices that
         // would not give every SM a block.
-        const long long cap_sites = max_tiles_ * (threads_ / 4);
         meas_groups_ = shape_.meas_split == 2 ? LOOP_MAX_GROUPS : LOOP_MAX_GROUPS / 2;
         while (meas_groups_ > 1 && cap_sites < (long long)MEAS_SITES * meas_groups_ * ctx_->sm_count) meas_groups_ /= 2;
         unit_sites_ = shape_.meas_split == 2 ? PLANE_MAX_SITES : PLANE_MAX_SITES / 2;
@@ -316,7 +324,6 @@ public:
         std::vector<int4> mtiles;
         seg_off_.assign(members.size(), 0);
         seg_len_.assign(members.size(), 0);
-        std::vector<int> stage_len(members.size(), 0);
         for (size_t i = 0; i < members.size(); ++i) {
             const LatticeBuf& b = *members[i];
             LatDesc<R>& d = h_desc_[i];
@@ -330,22 +337,45 @@ public:
             d.meas = b.meas;
             d.slot = b.slot;
             d.nchunk = b.nchunk;
-            d.eps = (R)b.eps;
-            // a tile is threads_/4 consecutive sites with all four link directions;
-            // per site a stage reads and writes 4 links and 4 su(3) accumulators
+            d.eps = b.eps;
             const TileShape ls = list_shape(b.g.V);
-            const size_t t0 = tiles.size();
-            if (!(ls.stage_order == 1 && append_stage_tiles_columns(tiles, (int)i, b.g, threads_ / 4, stage_grid_max_)))
-                append_stage_tiles(tiles, (int)i, b.g, threads_ / 4, ls.stage_budget, 4.0 * (2 * 18 + 8) * sizeof(R));
-            stage_len[i] = (int)(tiles.size() - t0);
             // this member's segment of the measurement list
             seg_off_[i] = (int)mtiles.size();
             append_measure_tiles(mtiles, (int)i, b.g, ls.meas_budget, 4.0 * 18 * sizeof(R));
             seg_len_[i] = (int)mtiles.size() - seg_off_[i];
         }
-        if ((long long)tiles.size() > max_tiles_)
+        // the stage's launches: a launch per run of whole members with the
+        // staple form, two (plaquettes, update) per run with the plaquette form
+        std::vector<int2> segs;
+        stage_nseg_ = plaq_nseg_ = 0;
+        for (int form = 0; form < 2; ++form) {
+            std::vector<int> which, len;
+            for (size_t i = 0; i < members.size(); ++i) {
+                if (plaquette_stage<R>(members[i]->g) != (form == 1)) continue;
+                which.push_back((int)i);
+                len.push_back((members[i]->g.V + threads_ / 4 - 1) / (threads_ / 4));
+            }
+            if (which.empty()) continue;
+            size_t m = 0;
+            long long pos = 0;
+            for (const int2& run : member_runs(len, slots_, 8LL * stage_grid_max_)) {
+                const size_t m0 = m;
+                while (m < which.size() && pos < (long long)run.x + run.y) pos += len[m++];
+                for (int part = 0; part <= form; ++part) {
+                    const int first = (int)tiles.size();
+                    for (size_t k = m0; k < m; ++k) {
+                        const Geom& g = members[which[k]]->g;
+                        if (form == 1) append_site_tiles(tiles, which[k], g, part ? UPDATE_SITES : PLAQ_SITES);
+                        else append_staple_tiles(tiles, which[k], g);
+                    }
+                    segs.push_back(make_int2(first, (int)tiles.size() - first));
+                }
+                ++(form ? plaq_nseg_ : stage_nseg_);
+            }
+        }
+        if ((long long)tiles.size() > tiles_cap_)
             return set_error(ctx_, LGF_EINVAL, "work list of %zu tiles exceeds the group capacity %lld", tiles.size(),
-                             max_tiles_);
+                             tiles_cap_);
         const long long mt = (long long)mtiles.size();
         if (mt > mtiles_cap_) {
             if (captured()) return set_error(ctx_, LGF_EINVAL, "measurement list grew after capture");
@@ -370,13 +400,11 @@ public:
             LGF_CUDA_TRY(ctx_, cudaMalloc(&d_jobs_, sizeof(int) * jobs_cap_));
         }
         ntiles_ = (int)tiles.size();
-        // the stage's launch segments (unused slots empty)
-        std::vector<int2> segs = member_runs(stage_len, slots_, 8LL * stage_grid_max_);
-        stage_nseg_ = (int)segs.size();
-        segs.resize(slots_, make_int2(0, 0));
+        seg_tiles_.clear();
+        for (const int2& q : segs) seg_tiles_.push_back(q.y);
         // one page-locked area carries the descriptors, both tile lists and the segments
         const size_t bd = align16(sizeof(LatDesc<R>) * members.size()), bt = align16(sizeof(int2) * tiles.size()),
-                     bm = align16(sizeof(int4) * mtiles.size()), bs = sizeof(int2) * slots_;
+                     bm = align16(sizeof(int4) * mtiles.size()), bs = sizeof(int2) * segs.size();
         std::lock_guard<std::mutex> lk(ctx_->list_mu);
         char* h = nullptr;
         LGF_CUDA_TRY(ctx_, ctx_->list_stage.acquire(bd + bt + bm + bs, &h));
@@ -393,13 +421,13 @@ public:
         if (mt)
             LGF_CUDA_TRY(ctx_, cudaMemcpyAsync(d_all_mtiles_, h + bd + bt, sizeof(int4) * mtiles.size(),
                                                cudaMemcpyHostToDevice, ctx_->stream));
-        LGF_CUDA_TRY(ctx_, cudaMemcpyAsync(d_seg_, h + bd + bt + bm, bs, cudaMemcpyHostToDevice, ctx_->stream));
+        if (bs) LGF_CUDA_TRY(ctx_, cudaMemcpyAsync(d_seg_, h + bd + bt + bm, bs, cudaMemcpyHostToDevice, ctx_->stream));
         LGF_CUDA_TRY(ctx_, ctx_->list_stage.release(ctx_->stream));
         return LGF_OK;
     }
 
     int set_eps(const std::vector<double>& eps) override {
-        for (size_t i = 0; i < h_desc_.size() && i < eps.size(); ++i) h_desc_[i].eps = (R)eps[i];
+        for (size_t i = 0; i < h_desc_.size() && i < eps.size(); ++i) h_desc_[i].eps = eps[i];
         if (h_desc_.empty()) return LGF_OK;
         std::lock_guard<std::mutex> lk(ctx_->list_mu);
         char* h = nullptr;
@@ -484,13 +512,13 @@ public:
         return LGF_OK;
     }
 
-    int launch_step() override { return launch_stages(stage_nseg_); }
+    int launch_step() override { return launch_stages(stage_nseg_, plaq_nseg_); }
 
     // a single kernel: k = 0..2 stage k+1, k = 3 the measurement kernel alone
     // (every launch segment of it)
     int launch_one(int k) override {
         if (k < 3) {
-            for (int j = 0; j < stage_nseg_; ++j) launch_stage(k + 1, j);
+            launch_stage(k + 1, stage_nseg_, plaq_nseg_);
         } else {
             launch_measure_kernels<false>(meas_nseg_, meas_small_, MeasSites{});
         }
@@ -510,16 +538,16 @@ public:
     // drop the graphs and capture those of the current segment counts
     int capture() override {
         drop_graphs();
-        int rc = capture_one(true, stage_nseg_, &step_execs_[stage_nseg_]);
+        int rc = capture_one(true, 0, &step_execs_[step_graph()]);
         if (rc != LGF_OK) return rc;
         return capture_one(false, meas_nseg_, &meas_execs_[meas_graph()]);
     }
     // graph launch; a graph per count of launch segments, captured on first use
     int replay_step() override {
         NvtxRange r("lgf.rk3_step");
-        cudaGraphExec_t& g = step_execs_[stage_nseg_];
+        cudaGraphExec_t& g = step_execs_[step_graph()];
         if (!g) {
-            int rc = capture_one(true, stage_nseg_, &g);
+            int rc = capture_one(true, 0, &g);
             if (rc != LGF_OK) return rc;
         }
         LGF_CUDA_TRY(ctx_, cudaGraphLaunch(g, ctx_->stream));
@@ -535,13 +563,12 @@ public:
         LGF_CUDA_TRY(ctx_, cudaGraphLaunch(g, ctx_->stream));
         return LGF_OK;
     }
-    int launches_per_step() const override { return 3; }
+    int launches_per_step() const override { return 3 * (stage_nseg_ + 2 * plaq_nseg_); }
     int launches_per_measure() const override { return (meas_small_ ? 1 : 0) + (meas_nseg_ ? 5 : 0) + 2; }
     int threads() const override { return threads_; }
     const TileShape& shape() const override { return shape_; }
 
 private:
-    int stage_grid() const { return dynamic_ ? stage_grid_max_ : std::max(1, std::min(ntiles_, stage_grid_max_)); }
     // a measurement kernel's grid: its persistent grid, or fewer blocks when its lists are shorter
     int meas_grid(long long work, int grid_max) const {
         return dynamic_ ? grid_max : (int)std::max(1LL, std::min(work, (long long)grid_max));
@@ -562,29 +589,49 @@ private:
     size_t sel_ints(int n) const { return (size_t)sel_fields() + (size_t)SEL_FIELDS * std::max(n, 1); }
     int meas_graph() const { return 2 * meas_nseg_ + (meas_small_ ? 1 : 0); }
     bool captured() const {
-        for (auto g : step_execs_) if (g) return true;
+        for (auto& g : step_execs_) if (g.second) return true;
         for (auto g : meas_execs_) if (g) return true;
         return false;
     }
     void drop_graphs() {
-        for (auto& g : step_execs_) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+        for (auto& g : step_execs_) if (g.second) cudaGraphExecDestroy(g.second);
+        step_execs_.clear();
         for (auto& g : meas_execs_) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     }
 
-    // stage S over launch segment j of the tile list
-    void launch_stage(int S, int j) {
-        const int grid = stage_grid();
-        const int2* seg = d_seg_ + j;
-        if (S == 1) k_rk3_stage<R, 1><<<grid, threads_, 0, ctx_->stream>>>(d_desc_, d_tiles_, seg);
-        if (S == 2) k_rk3_stage<R, 2><<<grid, threads_, 0, ctx_->stream>>>(d_desc_, d_tiles_, seg);
-        if (S == 3) k_rk3_stage<R, 3><<<grid, threads_, 0, ctx_->stream>>>(d_desc_, d_tiles_, seg);
+    // the staple tiles of lattice i in its work order: threads_/4 consecutive
+    // sites with all four link directions; per site a stage reads and writes 4
+    // links and 4 su(3) accumulators
+    void append_staple_tiles(std::vector<int2>& tiles, int i, const Geom& g) const {
+        const TileShape ls = list_shape(g.V);
+        if (!(ls.stage_order == 1 && append_stage_tiles_columns(tiles, i, g, threads_ / 4, stage_grid_max_)))
+            append_stage_tiles(tiles, i, g, threads_ / 4, ls.stage_budget, 4.0 * (2 * 18 + 8) * sizeof(R));
     }
-    int launch_stages(int nseg) {
+    // a stage launch's grid: persistent, or fewer blocks when its list is shorter
+    int stage_grid(int j, int most) const { return dynamic_ ? most : std::max(1, std::min(seg_tiles_[j], most)); }
+    int step_graph() const { return stage_nseg_ * (slots_ + 1) + plaq_nseg_; }
+    // stage S: n launches of the staple form, then np pairs of the plaquette form
+    template <int S> void launch_stage_of(int n, int np) {
+        int j = 0;
+        for (; j < n; ++j)
+            k_rk3_stage<R, S><<<stage_grid(j, stage_grid_max_), threads_, 0, ctx_->stream>>>(d_desc_, d_tiles_, d_seg_ + j);
+        if constexpr (sizeof(R) == sizeof(float))
+            for (; j < n + 2 * np; j += 2) {
+                k_rk3_plaquettes<R, S><<<stage_grid(j, plaq_grid_max_), 6 * PLAQ_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, d_seg_ + j);
+                k_rk3_update<R, S><<<stage_grid(j + 1, update_grid_max_), 4 * UPDATE_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, d_seg_ + j + 1);
+            }
+    }
+    void launch_stage(int S, int n, int np) {
+        if (S == 1) launch_stage_of<1>(n, np);
+        if (S == 2) launch_stage_of<2>(n, np);
+        if (S == 3) launch_stage_of<3>(n, np);
+    }
+    int launch_stages(int n, int np) {
         if (!dynamic_ && ntiles_ == 0) return LGF_OK;
         static const char* names[3] = {"lgf.rk3_stage1", "lgf.rk3_stage2", "lgf.rk3_stage3"};
         for (int S = 1; S <= 3; ++S) {
             NvtxRange r(names[S - 1]);
-            for (int j = 0; j < nseg; ++j) launch_stage(S, j);
+            launch_stage(S, n, np);
         }
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
@@ -628,7 +675,7 @@ private:
     int capture_one(bool step, int nseg, cudaGraphExec_t* out) {
         cudaGraph_t graph = nullptr;
         LGF_CUDA_TRY(ctx_, cudaStreamBeginCapture(ctx_->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = step ? launch_stages(nseg) : launch_measurement(nseg, meas_small_);
+        int rc = step ? launch_stages(stage_nseg_, plaq_nseg_) : launch_measurement(nseg, meas_small_);
         cudaError_t e = cudaStreamEndCapture(ctx_->stream, &graph);
         if (rc != LGF_OK) {
             if (graph) cudaGraphDestroy(graph);
@@ -677,10 +724,14 @@ private:
     int stage_grid_max_ = 1, small_grid_max_ = 1, loops_grid_max_ = 1, planes_grid_max_ = 1;
     int meas_groups_ = LOOP_MAX_GROUPS, unit_sites_ = PLANE_MAX_SITES;  // tiles per loops block, sites per plane unit
     int slots_;                                   // launch slots per kernel (member_runs)
-    int stage_nseg_ = 1, meas_nseg_ = 1;           // launch segments in use
+    int stage_nseg_ = 0, plaq_nseg_ = 0, meas_nseg_ = 1;  // launch segments in use (staple and plaquette form, measurement)
     bool meas_small_ = false;                      // some measured lattice takes the one-launch kernel
     int2* d_seg_ = nullptr;                        // the stage's launch segments
-    std::vector<cudaGraphExec_t> step_execs_, meas_execs_;  // by segment count (and small lattices)
+    long long tiles_cap_ = 0;                      // capacity of d_tiles_
+    int plaq_grid_max_ = 1, update_grid_max_ = 1;
+    std::vector<int> seg_tiles_;                   // tiles of each stage launch
+    std::map<int, cudaGraphExec_t> step_execs_;    // by launch counts (step_graph)
+    std::vector<cudaGraphExec_t> meas_execs_;      // by segment count (and small lattices)
 };
 
 GroupBase* make_group(lgf_ctx* ctx, int precision, const TileShape& shape, int max_members, long long max_tiles,
@@ -1261,10 +1312,15 @@ int lgf_debug_gradient(lgf_lattice* lat, double* Z) {
     const size_t bytes = (size_t)b.g.V * 4 * 18 * sizeof(double);
     double2* d = nullptr;
     LGF_CUDA_TRY(ctx, cudaMalloc(&d, bytes));
-    if (b.prec == LGF_PREC_FP64)
-        k_debug_gradient<double><<<blocks_for(4LL * b.g.V, 128), 128, 0, ctx->stream>>>((const cplx<double>*)b.U[0], b.g, d);
-    else
-        k_debug_gradient<float><<<blocks_for(4LL * b.g.V, 128), 128, 0, ctx->stream>>>((const cplx<float>*)b.U[0], b.g, d);
+    // (the plaquette form's fields go to the ring's second buffer, free between flows)
+    const dim3 gp(blocks_for(b.g.V, 128), 6), gl(blocks_for(b.g.V, 128), 4);
+    if (b.prec == LGF_PREC_FP64) {
+        k_debug_gradient<double><<<gl, 128, 0, ctx->stream>>>((const cplx<double>*)b.U[0], (const double*)b.U[1], b.g, d);
+    } else {
+        if (plaquette_stage<float>(b.g))
+            k_debug_plaquettes<float><<<gp, 128, 0, ctx->stream>>>((const cplx<float>*)b.U[0], b.g, (float*)b.U[1]);
+        k_debug_gradient<float><<<gl, 128, 0, ctx->stream>>>((const cplx<float>*)b.U[0], (const float*)b.U[1], b.g, d);
+    }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(Z, d, bytes, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);

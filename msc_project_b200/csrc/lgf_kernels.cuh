@@ -1,6 +1,7 @@
 // sm_100a kernels of the Wilson-flow engine.
 //
-//   k_rk3_stage<R,S>   one fused Luscher RK3 stage for every link: staple,
+//   k_rk3_stage<R,S>   one fused Luscher RK3 stage for every link (FP64; FP32:
+//                      k_rk3_plaquettes + k_rk3_update): staple,
 //                      projected force Z, su(3) accumulator update,
 //                      Cayley-Hamilton exponential, link update (ping-pong).
 //                      Replaces Wilson::calculate_FlowGradient
@@ -78,9 +79,6 @@ __device__ __forceinline__ su3<R> staple_sum(const cplx<R>* __restrict__ U, cons
     return S;
 }
 
-#ifndef LGF_TA_ONLY
-#define LGF_TA_ONLY 1  // the force's product forms only the entries its projection reads
-#endif
 // ta_part(A B, s) computing only what the projection reads: the imaginary
 // parts of the diagonal and the three off-diagonal pairs (90 real
 // operations instead of 108 for the full product)
@@ -118,7 +116,7 @@ __device__ __forceinline__ alg<R> flow_gradient(const cplx<R>* __restrict__ U, c
                                                 int mu, su3<R>& u_out) {
     const su3<R> S = staple_sum<R>(U, g, s, c, mu);
     u_out = load_link(U, g.V, mu, s);
-    return LGF_TA_ONLY ? ta_of_product(u_out, S, R(-0.5)) : ta_part(mul_nn(u_out, S), R(-0.5));
+    return ta_of_product(u_out, S, R(-0.5));
 }
 
 // Device descriptor of one resident lattice.  Every flow launch works on a
@@ -135,62 +133,8 @@ template <typename R> struct LatDesc {
     double* meas;         // [capacity * (2 + 2 N0)] measurement results
     int* slot;            // next measurement slot
     int nchunk;           // measurement blocks per x0 slice
-    R eps;
+    double eps;
 };
-
-// One RK3 stage (low-storage form of the reference's integrator):
-//   S=1:  A = Z0;                    U1 = exp(eps/4 Z0) U0
-//   S=2:  A = 8/9 Z1 - 17/36 A;      U2 = exp(eps A) U1
-//   S=3:                             U3 = exp(eps (3/4 Z2 - A)) U2
-// which equals GradientFlow.cpp:27-50 term by term.  Input and output are
-// different buffers of the ring (every thread reads neighbours of the input).
-// Persistent: blocks stride over one segment of the tile list (seg = first
-// tile, count); tile = (lattice, first site).
-// A tile of T threads (T a multiple of 128) covers T/4 consecutive sites with
-// all four directions: warp w handles mu = w % 4 for the 32 sites of group
-// w / 4, so the four link directions of a site range are read together and
-// every load of a warp covers 32 consecutive sites.
-template <typename R> struct StageMaxThreads { static constexpr int value = LGF_STAGE_MAXT_F; };
-template <> struct StageMaxThreads<double> { static constexpr int value = LGF_STAGE_MAXT_D; };
-
-template <typename R, int S>
-__global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_rk3_stage(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
-                                                   const int2* __restrict__ seg) {
-    const int2 r = *seg;  // this launch's tiles: tiles[r.x, r.x + r.y)
-    for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
-        const int2 tile = tiles[ti];
-        const LatDesc<R>* d = descs + tile.x;
-        const Geom g = d->g;
-        const int mu = (threadIdx.x >> 5) & 3;
-        const int s = tile.y + ((threadIdx.x >> 7) << 5) + (threadIdx.x & 31);
-        if (s >= g.V) continue;
-        const cplx<R>* Uin = S == 1 ? d->U0 : (S == 2 ? d->U1 : d->U2);
-        cplx<R>* Uout = S == 1 ? d->U1 : (S == 2 ? d->U2 : d->U0);
-        R* A = d->A;
-        const R eps = d->eps;
-        const Coord c = site_coord(g, s);
-        su3<R> u;
-        const alg<R> Z = flow_gradient<R>(Uin, g, s, c, mu, u);
-        alg<R> X;
-        if (S == 1) {
-            store_alg(A, g.V, mu, s, Z);
-            X = alg_scale(R(0.25) * eps, Z);
-        } else if (S == 2) {
-            const alg<R> a = load_alg(A, g.V, mu, s);
-            const alg<R> an = alg_axpby(R(8.0 / 9.0), Z, R(-17.0 / 36.0), a);
-            store_alg(A, g.V, mu, s, an);
-            X = alg_scale(eps, an);
-        } else {
-            const alg<R> a = load_alg(A, g.V, mu, s);
-            const alg<R> dd = alg_axpby(R(3.0 / 4.0), Z, R(-1.0), a);
-            X = alg_scale(eps, dd);
-        }
-        const su3<R> E = expm_alg(X);
-        // the stored link is the full product (rebuilding its third row from
-        // the first two would let their rounding drift into it step after step)
-        store_link(Uout, g.V, mu, s, mul_nn(E, u));
-    }
-}
 
 // ---------------------------------------------------------- Wilson loops
 // The clover-type averages of the reference (SU3_field.cpp:533-792) are sums
@@ -325,6 +269,279 @@ template <typename R, typename Acc> __device__ __forceinline__ void leaf_acc(con
     }
 }
 
+__device__ __constant__ int c_plane_mu[6] = {0, 0, 0, 1, 1, 2};
+__device__ __constant__ int c_plane_nu[6] = {1, 2, 3, 2, 3, 3};
+
+// ---------------------------------------------------------------- fields
+// Hermitian traceless field of 8 coordinates per site in 32-site blocks:
+// double2 pairs or float4 quads, planes of 32 sites.
+constexpr int FIELD_REALS = 8 * LAYOUT_BLOCK;  // one field of one block
+template <typename R, bool RO> __device__ __forceinline__ alg<R> get_field(const R* p) {
+    alg<R> z;
+    if constexpr (sizeof(R) == sizeof(double)) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const double2* a = reinterpret_cast<const double2*>(p) + q * LAYOUT_BLOCK;
+            const double2 v = RO ? __ldg(a) : *a;
+            z.v[2 * q] = v.x;
+            z.v[2 * q + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const float4* a = reinterpret_cast<const float4*>(p) + q * LAYOUT_BLOCK;
+            const float4 v = RO ? __ldg(a) : *a;
+            z.v[4 * q] = v.x;
+            z.v[4 * q + 1] = v.y;
+            z.v[4 * q + 2] = v.z;
+            z.v[4 * q + 3] = v.w;
+        }
+    }
+    return z;
+}
+template <typename R> __device__ __forceinline__ void put_field(R* p, const alg<R>& z) {
+    if constexpr (sizeof(R) == sizeof(double)) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            reinterpret_cast<double2*>(p)[q * LAYOUT_BLOCK] = make_double2(z.v[2 * q], z.v[2 * q + 1]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            reinterpret_cast<float4*>(p)[q * LAYOUT_BLOCK] = make_float4(z.v[4 * q], z.v[4 * q + 1], z.v[4 * q + 2], z.v[4 * q + 3]);
+    }
+}
+
+// c F[A B^dag], computed in D and returned in R
+template <typename R, typename D> __device__ __forceinline__ alg<R> leaf(const su3<D>& A, const su3<D>& B, D c) {
+    alg<D> F;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) F.v[k] = D(0);
+    leaf_acc(A, B, c, RegAcc<D>{F});
+    alg<R> z;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) z.v[k] = (R)F.v[k];
+    return z;
+}
+
+// U^dag H U of a Hermitian traceless H, in the same 8 coordinates: column by
+// column, Y = H U_col (30 operations) and the entries of U^dag Y at and above
+// the diagonal; the last diagonal entry follows from the trace.
+template <typename R> __device__ __forceinline__ alg<R> shift(const alg<R>& h, const su3<R>& U) {
+    const R a0 = h.v[0], a1 = h.v[1], a2 = -(h.v[0] + h.v[1]);
+    const cplx<R> q01 = cmk<R>(h.v[2], h.v[3]), q02 = cmk<R>(h.v[4], h.v[5]), q12 = cmk<R>(h.v[6], h.v[7]);
+    alg<R> z;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const cplx<R> u0 = U.m[c], u1 = U.m[3 + c], u2 = U.m[6 + c];
+        const cplx<R> y0 = cfma(q02, u2, cfma(q01, u1, cmk<R>(a0 * u0.re, a0 * u0.im)));
+        const cplx<R> y1 = cfma(q12, u2, ccfma(q01, u0, cmk<R>(a1 * u1.re, a1 * u1.im)));
+        const cplx<R> y2 = ccfma(q12, u1, ccfma(q02, u0, cmk<R>(a2 * u2.re, a2 * u2.im)));
+        if (c < 2) {
+            R d = u0.re * y0.re;
+            d = fma(u0.im, y0.im, d);
+            d = fma(u1.re, y1.re, d);
+            d = fma(u1.im, y1.im, d);
+            d = fma(u2.re, y2.re, d);
+            z.v[c] = fma(u2.im, y2.im, d);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (r >= c) continue;
+            cplx<R> w = ccmul(U.m[r], y0);
+            w = ccfma(U.m[3 + r], y1, w);
+            w = ccfma(U.m[6 + r], y2, w);
+            const int o = 2 * (r + c);  // 01 -> 2, 02 -> 4, 12 -> 6
+            z.v[o] = w.re;
+            z.v[o + 1] = w.im;
+        }
+    }
+    return z;
+}
+template <typename R> __device__ __forceinline__ alg<R> alg_add(const alg<R>& x, const alg<R>& y) {
+    alg<R> z;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) z.v[k] = x.v[k] + y.v[k];
+    return z;
+}
+
+// ------------------------------------------------------------------ stage
+// One RK3 stage (low-storage form of the reference's integrator):
+//   S=1:  A = Z0;                    U1 = exp(eps/4 Z0) U0
+//   S=2:  A = 8/9 Z1 - 17/36 A;      U2 = exp(eps A) U1
+//   S=3:                             U3 = exp(eps (3/4 Z2 - A)) U2
+// which equals GradientFlow.cpp:27-50 term by term.  Input and output are
+// different buffers of the ring (every thread reads neighbours of the input).
+template <typename R, int S> __device__ __forceinline__ const cplx<R>* stage_in(const LatDesc<R>* d) { return S == 1 ? d->U0 : (S == 2 ? d->U1 : d->U2); }
+template <typename R, int S> __device__ __forceinline__ cplx<R>* stage_out(const LatDesc<R>* d) { return S == 1 ? d->U1 : (S == 2 ? d->U2 : d->U0); }
+template <typename R, int S> __device__ __forceinline__ R* stage_free(const LatDesc<R>* d) { return reinterpret_cast<R*>(S == 1 ? d->U2 : (S == 2 ? d->U0 : d->U1)); }
+
+// accumulator, exponential and link update of link (s, mu) with force Z and
+// link u.  The integrator's coefficients and eps are applied in double for
+// both precisions: in float they round by up to 2e-8 of themselves, the same
+// way at every step, which is a flow time off by as much.
+template <typename R, int S>
+__device__ __forceinline__ void update_link(R* A, cplx<R>* Uout, double eps, int V, int s, int mu, const alg<R>& Z, const su3<R>& u) {
+    alg<double> X = alg_cast<double>(Z);
+    if (S == 1) {
+        store_alg(A, V, mu, s, Z);
+        X = alg_scale(0.25 * eps, X);
+    } else if (S == 2) {
+        X = alg_axpby(8.0 / 9.0, X, -17.0 / 36.0, alg_cast<double>(load_alg(A, V, mu, s)));
+        store_alg(A, V, mu, s, alg_cast<R>(X));
+        X = alg_scale(eps, X);
+    } else {
+        X = alg_axpby(3.0 / 4.0, X, -1.0, alg_cast<double>(load_alg(A, V, mu, s)));
+        X = alg_scale(eps, X);
+    }
+    // the stored link is the full product (rebuilding its third row from
+    // the first two would let their rounding drift into it step after step)
+    store_link(Uout, V, mu, s, exp_times(X, u));
+}
+
+// Staple form: FP64, and small FP32 lattices (plaquette_stage).
+// Persistent: blocks stride over one segment of the tile list (seg = first
+// tile, count); tile = (lattice, first site).
+// A tile of T threads (T a multiple of 128) covers T/4 consecutive sites with
+// all four directions: warp w handles mu = w % 4 for the 32 sites of group
+// w / 4, so the four link directions of a site range are read together and
+// every load of a warp covers 32 consecutive sites.
+template <typename R> struct StageMaxThreads { static constexpr int value = LGF_STAGE_MAXT_F; };
+template <> struct StageMaxThreads<double> { static constexpr int value = LGF_STAGE_MAXT_D; };
+
+template <typename R, int S>
+__global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_rk3_stage(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
+                                                   const int2* __restrict__ seg) {
+    const int2 r = *seg;  // this launch's tiles: tiles[r.x, r.x + r.y)
+    for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
+        const int2 tile = tiles[ti];
+        const LatDesc<R>* d = descs + tile.x;
+        const Geom g = d->g;
+        const int mu = (threadIdx.x >> 5) & 3;
+        const int s = tile.y + ((threadIdx.x >> 7) << 5) + (threadIdx.x & 31);
+        if (s >= g.V) continue;
+        const cplx<R>* Uin = stage_in<R, S>(d);
+        cplx<R>* Uout = stage_out<R, S>(d);
+        R* A = d->A;
+        const double eps = d->eps;
+        const Coord c = site_coord(g, s);
+        su3<R> u;
+        const alg<R> Z = flow_gradient<R>(Uin, g, s, c, mu, u);
+        update_link<R, S>(A, Uout, eps, g.V, s, mu, Z, u);
+    }
+}
+
+// Plaquette form: FP32 lattices above the small ones.
+//
+// The force of link (x, mu) sums the six plaquettes that contain the link,
+// projected: Z = -i sum_nu F[W_+nu] + F[W_-nu] with W based at x and starting
+// along mu.  Every plaquette belongs to four links.  With its projection
+// P_mn(y) = F[m(y) n(y+m) (n(y) m(y+n))^dag] at its lowest corner (m < n), and
+// T_d the covariant shift of a projection (shift()),
+//     link (x, m):  F[W_+n] + F[W_-n] =   P_mn(x) - T_n P_mn(x)
+//     link (x, n):  F[W_+m] + F[W_-m] = -(P_mn(x) - T_m P_mn(x)),
+// so a site's six plaquettes (two products and a projection each) and twelve
+// shifts replace its 24 staples: 4600 instead of 6500 operations per site and
+// stage.  The plaquettes make a launch of their own and go to the ring's free
+// buffer (stage S reads U_{S-1}, writes U_S; six fields of 8 reals take two
+// thirds of the third), which costs 384 (FP64: 768) bytes of traffic per site.
+// FP32, bound by instruction issue, gains: one B200, us per step (3 stages),
+// 24^3x48 803 -> 665, 32^4 1251 -> 1023, 48^4 6900 -> 5500, 16^4 89 -> 77,
+// 6x10x14x18 35 -> 31.
+// FP64, where both forms are bound by L2 latency and bandwidth (plaquettes
+// 153 us at 0.49 of the FP64 pipe, update 278 us at 0.45 with DRAM at 5 TB/s,
+// 24^3x48), does not: 1197 -> 1153, and 48^4 10160 -> 11700; keeping a chunk
+// of x0 slices' plaquettes in L2 with a launch per chunk was slower still
+// (1350 in chunks of 256 MB, 1570 of 64 MB).
+constexpr int PLAQ_SITES = 32;    // sites of a plaquette tile: a warp per plane
+constexpr int UPDATE_SITES = 32;  // sites of an update tile: a warp per direction
+template <typename R> __device__ __forceinline__ R* plaq_field(R* K, int p, int s) {
+    return K + ((size_t)(s / LAYOUT_BLOCK) * 6 + p) * FIELD_REALS + (s % LAYOUT_BLOCK) * (16 / sizeof(R));
+}
+// index of plane (a, b), a < b, in the order 01 02 03 12 13 23
+__host__ __device__ __forceinline__ int plane_index(int a, int b) { return a == 0 ? b - 1 : a + b; }
+
+template <typename R>
+__device__ __forceinline__ void plaquette_at(const cplx<R>* __restrict__ U, R* __restrict__ K, const Geom& g, int s, const Coord& c, int p) {
+    const int m = c_plane_mu[p], n = c_plane_nu[p];
+    const int xpm = fwd(s, dir_of(g, c, m)), xpn = fwd(s, dir_of(g, c, n));
+    const su3<R> a = mul_nn_su3(load_link(U, g.V, m, s), load_link(U, g.V, n, xpm));
+    const su3<R> b = mul_nn_su3(load_link(U, g.V, n, s), load_link(U, g.V, m, xpn));
+    put_field(plaq_field(K, p, s), leaf<R>(a, b, R(1)));
+}
+
+// Z(x, mu) from the plaquettes, in the coordinates of an su(3) element:
+// X = -i F has (Im X00, Im X11) = -(F00, F11) and X_ij = (Im F_ij, -Re F_ij)
+template <typename R>
+__device__ __forceinline__ alg<R> force_at(const cplx<R>* __restrict__ U, const R* __restrict__ K, const Geom& g, int s, const Coord& c,
+                                           int mu) {
+    alg<R> f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) f.v[k] = R(0);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+        const int nu = (mu + i) & 3;
+        const int p = mu < nu ? plane_index(mu, nu) : plane_index(nu, mu);
+        const R sg = mu < nu ? R(1) : R(-1);
+        const int xmn = bwd(s, dir_of(g, c, nu));
+        const alg<R> t = shift(get_field<R, true>(plaq_field(K, p, xmn)), load_link(U, g.V, nu, xmn));
+        const alg<R> k0 = get_field<R, true>(plaq_field(K, p, s));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f.v[k] = fma(sg, k0.v[k] - t.v[k], f.v[k]);
+    }
+    alg<R> z;
+    z.v[0] = -f.v[0];
+    z.v[1] = -f.v[1];
+#pragma unroll
+    for (int k = 2; k < 8; k += 2) {
+        z.v[k] = f.v[k + 1];
+        z.v[k + 1] = -f.v[k];
+    }
+    return z;
+}
+
+// 24 warps of 80 registers per SM (30 of 64 registers: 16^4 5% slower)
+template <typename R, int S>
+__global__ void __launch_bounds__(6 * PLAQ_SITES, 4) k_rk3_plaquettes(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
+                                                                     const int2* __restrict__ seg) {
+    const int2 r = *seg;  // this launch's tiles: tiles[r.x, r.x + r.y)
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
+        const int2 tile = tiles[ti];
+        const LatDesc<R>* d = descs + tile.x;
+        const Geom g = d->g;
+        const int s = tile.y + (w / 6) * 32 + lane;
+        if (s < g.V) plaquette_at<R>(stage_in<R, S>(d), stage_free<R, S>(d), g, s, site_coord(g, s), w % 6);
+    }
+}
+
+// 24 warps of 80 registers per SM (20 of 95: 24^3x48 2% slower per step, 16 of 115: 6%)
+template <typename R, int S>
+__global__ void __launch_bounds__(4 * UPDATE_SITES, 6) k_rk3_update(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
+                                                                   const int2* __restrict__ seg) {
+    const int2 r = *seg;
+    const int mu = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
+        const int2 tile = tiles[ti];
+        const LatDesc<R>* d = descs + tile.x;
+        const Geom g = d->g;
+        const int s = tile.y + lane;
+        if (s >= g.V) continue;
+        const cplx<R>* Uin = stage_in<R, S>(d);
+        const alg<R> Z = force_at<R>(Uin, stage_free<R, S>(d), g, s, site_coord(g, s), mu);
+        update_link<R, S>(d->A, stage_out<R, S>(d), d->eps, g.V, s, mu, Z, load_link(Uin, g.V, mu, s));
+    }
+}
+
+// Whether a lattice's stages take the plaquette form.  Small FP32 lattices do
+// not: their two short launches cost more than the operations they save (8^4:
+// 22.6 against 18.5 us per step; from 15120 sites on, 31 against 35, they do).
+// The rule reads the lattice alone, so a lattice gives the same bits in every
+// group.
+constexpr int PLAQ_MIN_SITES = 8192;
+template <typename R> __host__ __device__ __forceinline__ bool plaquette_stage(const Geom& g) {
+    return sizeof(R) == sizeof(float) && g.V >= PLAQ_MIN_SITES;
+}
+
 template <typename R> __device__ __forceinline__ void store_alg_as_antiherm(double2* dst, const alg<R>& z) {
     const double v0 = z.v[0], v1 = z.v[1];
     dst[0] = make_double2(0.0, v0);
@@ -349,9 +566,6 @@ template <typename R> __device__ __forceinline__ void store_alg_as_herm(double2*
     dst[5] = make_double2(f.v[6], f.v[7]);
     dst[7] = make_double2(f.v[6], -(double)f.v[7]);
 }
-
-__device__ __constant__ int c_plane_mu[6] = {0, 0, 0, 1, 1, 2};
-__device__ __constant__ int c_plane_nu[6] = {1, 2, 3, 2, 3, 3};
 
 constexpr int MEAS_SITES = 32;  // sites per measurement block (x) ; planes in y
 
@@ -946,15 +1160,20 @@ __global__ void __launch_bounds__(256) k_unitarity(const cplx<R>* __restrict__ U
 }
 
 // ---------------------------------------------------- per-function debug
-// flow gradient Z(x, mu) for every link, file order [s][mu][9] (double2)
+// the plaquettes of every site and plane, as a stage's K tiles write them
 template <typename R>
-__global__ void k_debug_gradient(const cplx<R>* __restrict__ U, Geom g, double2* __restrict__ out) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 4 * g.V) return;
-    const int mu = t / g.V, s = t - mu * g.V;
+__global__ void k_debug_plaquettes(const cplx<R>* __restrict__ U, Geom g, R* __restrict__ K) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < g.V) plaquette_at<R>(U, K, g, s, site_coord(g, s), blockIdx.y);
+}
+// flow gradient Z(x, mu) for every link, file order [s][mu][9] (double2), in the lattice's stage form
+template <typename R>
+__global__ void k_debug_gradient(const cplx<R>* __restrict__ U, const R* __restrict__ K, Geom g, double2* __restrict__ out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x, mu = blockIdx.y;
+    if (s >= g.V) return;
     const Coord c = site_coord(g, s);
     su3<R> u;
-    const alg<R> Z = flow_gradient<R>(U, g, s, c, mu, u);
+    const alg<R> Z = plaquette_stage<R>(g) ? force_at<R>(U, K, g, s, c, mu) : flow_gradient<R>(U, g, s, c, mu, u);
     store_alg_as_antiherm(out + ((size_t)s * 4 + mu) * 9, Z);
 }
 
@@ -973,7 +1192,7 @@ __global__ void k_debug_exp(const double2* __restrict__ in, double2* __restrict_
     x.v[5] = (R)m[2].y;
     x.v[6] = (R)m[5].x;
     x.v[7] = (R)m[5].y;
-    const su3<R> e = expm_alg(x);
+    const su3<R> e = expm_alg<R>(x);
 #pragma unroll
     for (int k = 0; k < 9; ++k) out[(size_t)t * 9 + k] = make_double2(e.m[k].re, e.m[k].im);
 }

@@ -43,7 +43,6 @@ namespace lgf {
 
 constexpr int LOOP_SHAPES = 6;                     // (1,1) (2,1) (3,1) (1,2) (1,3) (2,2)
 constexpr int LOOP_FIELDS = 3 * LOOP_SHAPES;       // of one round
-constexpr int FIELD_REALS = 8 * LAYOUT_BLOCK;      // one field of one 32-site block
 static_assert(LOOP_FIELDS * FIELD_REALS == 2 * 36 * 2 * LAYOUT_BLOCK, "U1..U2 hold one round's fields");
 
 // planes of a round, and the shapes' weights in F^ (F = G / 4, F^ = 19/36 G +
@@ -60,94 +59,6 @@ template <typename R> __device__ __forceinline__ R* loop_field(R* W, int f, int 
 template <typename R> __device__ __forceinline__ R* acc_field(R* A, int f, int s) {
     return A + ((size_t)(s / LAYOUT_BLOCK) * 4 + f) * FIELD_REALS + (s % LAYOUT_BLOCK) * (16 / sizeof(R));
 }
-template <typename R, bool RO> __device__ __forceinline__ alg<R> get_field(const R* p) {
-    alg<R> z;
-    if constexpr (sizeof(R) == sizeof(double)) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const double2* a = reinterpret_cast<const double2*>(p) + q * LAYOUT_BLOCK;
-            const double2 v = RO ? __ldg(a) : *a;
-            z.v[2 * q] = v.x;
-            z.v[2 * q + 1] = v.y;
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const float4* a = reinterpret_cast<const float4*>(p) + q * LAYOUT_BLOCK;
-            const float4 v = RO ? __ldg(a) : *a;
-            z.v[4 * q] = v.x;
-            z.v[4 * q + 1] = v.y;
-            z.v[4 * q + 2] = v.z;
-            z.v[4 * q + 3] = v.w;
-        }
-    }
-    return z;
-}
-template <typename R> __device__ __forceinline__ void put_field(R* p, const alg<R>& z) {
-    if constexpr (sizeof(R) == sizeof(double)) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            reinterpret_cast<double2*>(p)[q * LAYOUT_BLOCK] = make_double2(z.v[2 * q], z.v[2 * q + 1]);
-    } else {
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-            reinterpret_cast<float4*>(p)[q * LAYOUT_BLOCK] = make_float4(z.v[4 * q], z.v[4 * q + 1], z.v[4 * q + 2], z.v[4 * q + 3]);
-    }
-}
-
-// c F[A B^dag], computed in D and returned in R
-template <typename R, typename D> __device__ __forceinline__ alg<R> leaf(const su3<D>& A, const su3<D>& B, D c) {
-    alg<D> F;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) F.v[k] = D(0);
-    leaf_acc(A, B, c, RegAcc<D>{F});
-    alg<R> z;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) z.v[k] = (R)F.v[k];
-    return z;
-}
-
-// U^dag H U of a Hermitian traceless H, in the same 8 coordinates: column by
-// column, Y = H U_col (30 operations) and the entries of U^dag Y at and above
-// the diagonal; the last diagonal entry follows from the trace.
-template <typename R> __device__ __forceinline__ alg<R> shift(const alg<R>& h, const su3<R>& U) {
-    const R a0 = h.v[0], a1 = h.v[1], a2 = -(h.v[0] + h.v[1]);
-    const cplx<R> q01 = cmk<R>(h.v[2], h.v[3]), q02 = cmk<R>(h.v[4], h.v[5]), q12 = cmk<R>(h.v[6], h.v[7]);
-    alg<R> z;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const cplx<R> u0 = U.m[c], u1 = U.m[3 + c], u2 = U.m[6 + c];
-        const cplx<R> y0 = cfma(q02, u2, cfma(q01, u1, cmk<R>(a0 * u0.re, a0 * u0.im)));
-        const cplx<R> y1 = cfma(q12, u2, ccfma(q01, u0, cmk<R>(a1 * u1.re, a1 * u1.im)));
-        const cplx<R> y2 = ccfma(q12, u1, ccfma(q02, u0, cmk<R>(a2 * u2.re, a2 * u2.im)));
-        if (c < 2) {
-            R d = u0.re * y0.re;
-            d = fma(u0.im, y0.im, d);
-            d = fma(u1.re, y1.re, d);
-            d = fma(u1.im, y1.im, d);
-            d = fma(u2.re, y2.re, d);
-            z.v[c] = fma(u2.im, y2.im, d);
-        }
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            if (r >= c) continue;
-            cplx<R> w = ccmul(U.m[r], y0);
-            w = ccfma(U.m[3 + r], y1, w);
-            w = ccfma(U.m[6 + r], y2, w);
-            const int o = 2 * (r + c);  // 01 -> 2, 02 -> 4, 12 -> 6
-            z.v[o] = w.re;
-            z.v[o + 1] = w.im;
-        }
-    }
-    return z;
-}
-template <typename R> __device__ __forceinline__ alg<R> alg_add(const alg<R>& x, const alg<R>& y) {
-    alg<R> z;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) z.v[k] = x.v[k] + y.v[k];
-    return z;
-}
-
 // ------------------------------------------------------------------- loops
 // H_ab of the round's three planes: one thread per site and plane, warp w of
 // a block takes plane w % 3 of tile group w / 3 (a tile = 32 sites; adjacent

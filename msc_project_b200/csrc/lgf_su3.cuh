@@ -360,10 +360,6 @@ __device__ __forceinline__ void ch_coefficients(double c0, double c1, cplx<doubl
     }
 }
 
-#ifndef LGF_HERM_EXP
-#define LGF_HERM_EXP 1  // exp(iQ) = f0 + f1 Q + f2 Q^2 assembled from Q's Hermitian structure
-#endif
-
 // f0 + f1 Q + f2 Q^2 for Hermitian traceless Q (diagonal a_i real, upper
 // triangle q_ij, lower conj(q_ij)), using that structure: the diagonal of
 // Q^2 is a sum of squares, Q^2_01 = -a2 q01 + q02 conj(q12),
@@ -399,10 +395,10 @@ __device__ __forceinline__ su3<R> exp_assemble_herm(const herm_d& h, cplx<double
     return E;
 }
 
-// exp(X) for X in su(3) given by 8 coordinates; the result in precision R.
-// c0, c1 and the coefficients are computed in double from the (possibly
-// float) coordinates; the matrix assembly f0 + f1 Q + f2 Q^2 runs in R.
-template <typename R> __device__ __forceinline__ su3<R> expm_alg(const alg<R>& x) {
+// exp(X) - c for X in su(3) given by 8 coordinates (float or double); the result in precision R.
+// c0, c1 and the coefficients are computed in double, and c (0 or 1) is taken
+// from f0 there; the matrix assembly f0 + f1 Q + f2 Q^2 runs in R.
+template <typename R, typename X> __device__ __forceinline__ su3<R> expm_alg(const alg<X>& x, double c = 0.0) {
     const herm_d h = herm_from_alg(x);
     const double n01 = h.q01.re * h.q01.re + h.q01.im * h.q01.im;
     const double n02 = h.q02.re * h.q02.re + h.q02.im * h.q02.im;
@@ -414,49 +410,31 @@ template <typename R> __device__ __forceinline__ su3<R> expm_alg(const alg<R>& x
     const double c0 = h.a0 * h.a1 * h.a2 + 2.0 * re3 - h.a0 * n12 - h.a1 * n02 - h.a2 * n01;
     cplx<double> f0, f1, f2;
     ch_coefficients(c0, c1, f0, f1, f2);
-
-    if (LGF_HERM_EXP) return exp_assemble_herm<R>(h, f0, f1, f2);
-    // Q and Q^2 in precision R (Q Hermitian traceless)
-    su3<R> Q;
-    Q.m[0] = cmk<R>((R)h.a0, R(0));
-    Q.m[4] = cmk<R>((R)h.a1, R(0));
-    Q.m[8] = cmk<R>((R)h.a2, R(0));
-    Q.m[1] = cmk<R>((R)h.q01.re, (R)h.q01.im);
-    Q.m[2] = cmk<R>((R)h.q02.re, (R)h.q02.im);
-    Q.m[5] = cmk<R>((R)h.q12.re, (R)h.q12.im);
-    Q.m[3] = cmk<R>(Q.m[1].re, -Q.m[1].im);
-    Q.m[6] = cmk<R>(Q.m[2].re, -Q.m[2].im);
-    Q.m[7] = cmk<R>(Q.m[5].re, -Q.m[5].im);
-    // Q^2 is Hermitian: compute the diagonal and the upper triangle
-    su3<R> Q2;
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = r; c < 3; ++c) {
-            cplx<R> s = cmul(Q.m[3 * r], Q.m[c]);
-            s = cfma(Q.m[3 * r + 1], Q.m[3 + c], s);
-            s = cfma(Q.m[3 * r + 2], Q.m[6 + c], s);
-            Q2.m[3 * r + c] = s;
-        }
-    Q2.m[0].im = R(0);
-    Q2.m[4].im = R(0);
-    Q2.m[8].im = R(0);
-    Q2.m[3] = cmk<R>(Q2.m[1].re, -Q2.m[1].im);
-    Q2.m[6] = cmk<R>(Q2.m[2].re, -Q2.m[2].im);
-    Q2.m[7] = cmk<R>(Q2.m[5].re, -Q2.m[5].im);
-
-    const cplx<R> F0 = cmk<R>((R)f0.re, (R)f0.im);
-    const cplx<R> F1 = cmk<R>((R)f1.re, (R)f1.im);
-    const cplx<R> F2 = cmk<R>((R)f2.re, (R)f2.im);
-    su3<R> E;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) E.m[k] = cfma(Q2.m[k], F2, cmul(Q.m[k], F1));
-    E.m[0] = cadd(E.m[0], F0);
-    E.m[4] = cadd(E.m[4], F0);
-    E.m[8] = cadd(E.m[8], F0);
-    return E;
+    f0.re -= c;
+    return exp_assemble_herm<R>(h, f0, f1, f2);
 }
 
+// exp(X) u.  Double: the product with exp(X).  Float: u + (exp(X) - 1) u, whose
+// product is small against u, so a step's rounding is that of one addition
+// instead of a whole product of unit-size entries.
+template <typename R> __device__ __forceinline__ su3<R> exp_times(const alg<double>& x, const su3<R>& u) {
+    if constexpr (sizeof(R) == sizeof(double)) {
+        const su3<R> E = expm_alg<R>(x);
+        return mul_nn(E, u);
+    } else {
+        const su3<R> D = expm_alg<R>(x, 1.0);
+        su3<R> p = mul_nn(D, u);
+        su3_addto(p, u);
+        return p;
+    }
+}
+
+template <typename D, typename R> __device__ __forceinline__ alg<D> alg_cast(const alg<R>& x) {
+    alg<D> z;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) z.v[k] = (D)x.v[k];
+    return z;
+}
 template <typename R> __device__ __forceinline__ alg<R> alg_axpby(R a, const alg<R>& x, R b, const alg<R>& y) {
     alg<R> z;
 #pragma unroll

@@ -90,6 +90,11 @@ inline bool append_stage_tiles_columns(std::vector<int2>& tiles, int i, const Ge
     return true;
 }
 
+// tiles of T consecutive sites of lattice i, in site order
+inline void append_site_tiles(std::vector<int2>& tiles, int i, const Geom& g, int T) {
+    for (long long s = 0; s < g.V; s += T) tiles.push_back(make_int2(i, (int)s));
+}
+
 // measurement tiles (lattice, slice, chunk of the slice) of lattice i; a
 // chunk is a 32-site strip or a 4 x 8 patch (meas_patched, lgf_kernels.cuh)
 inline void append_measure_tiles(std::vector<int4>& tiles, int i, const Geom& g, double budget,
