@@ -156,12 +156,40 @@ template <typename R> struct LatDesc {
 // 40 for separate loops.
 struct PlanePos { int s, xm, xn; };
 
-#ifndef LGF_MEAS_ROW3
-#define LGF_MEAS_ROW3 1  // path products of the measurement rebuild their third row (mul_nn_su3)
-#endif
-
-// Links are read in R and multiplied in D.
-template <typename R, typename D = R> struct Plane {
+// A link of the device layout, or (FILE, double) of file-order links: entry k
+// at (s * 4 + mu) * 9 + k.  There a lane's link is 144 contiguous bytes and
+// the next lane's 576 further on, so a plain 16-byte load of a warp touches 32
+// cache lines and takes the L1 as many cycles.  Two lanes therefore read their
+// two links together, 32 contiguous bytes of one link at a time (16 lines per
+// load), and exchange halves by a shuffle: every lane of the warp must call.
+__device__ __forceinline__ cplx<double> shfl_xor_c(cplx<double> z, int mask) {
+    return cmk<double>(__shfl_xor_sync(0xffffffffu, z.re, mask), __shfl_xor_sync(0xffffffffu, z.im, mask));
+}
+__device__ __forceinline__ cplx<double> pick(bool c, cplx<double> a, cplx<double> b) { return cmk<double>(c ? a.re : b.re, c ? a.im : b.im); }
+template <bool FILE, typename R> __device__ __forceinline__ su3<R> load_link_from(const cplx<R>* __restrict__ U, int V, int mu, int s) {
+    if constexpr (FILE) {
+        static_assert(sizeof(R) == sizeof(double), "file-order links are double");
+        const bool odd = threadIdx.x & 1;
+        const int other = __shfl_xor_sync(0xffffffffu, s, 1);
+        const cplx<R>* even_link = U + ((size_t)(odd ? other : s) * 4 + mu) * 9 + (odd ? 1 : 0);
+        const cplx<R>* odd_link = U + ((size_t)(odd ? s : other) * 4 + mu) * 9 + (odd ? 1 : 0);
+        su3<R> a;
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {  // this lane's entry (k, or k + 1 on odd lanes) of both links
+            const cplx<R> e = ldc(even_link + k), o = ldc(odd_link + k);
+            const cplx<R> r = shfl_xor_c(pick(odd, e, o), 1);
+            a.m[k] = pick(odd, r, e);
+            a.m[k + 1] = pick(odd, o, r);
+        }
+        a.m[8] = ldc(U + ((size_t)s * 4 + mu) * 9 + 8);
+        return a;
+    } else {
+        return load_link(U, V, mu, s);
+    }
+}
+// Links are read in R and multiplied in D; FILE: U is in file order instead of
+// the device layout.
+template <typename R, typename D = R, bool FILE = false> struct Plane {
     const cplx<R>* __restrict__ U;
     int V, mu, nu;
     Dir dm, dn;  // .x unused: positions carry their own coordinates
@@ -172,14 +200,14 @@ template <typename R, typename D = R> struct Plane {
         int& xc = along_mu ? p.xm : p.xn;
         const int dir = along_mu ? mu : nu;
         if (sign > 0) {
-            su3<D> l = su3_cast<D>(load_link(U, V, dir, p.s));
+            su3<D> l = su3_cast<D>(load_link_from<FILE>(U, V, dir, p.s));
             p.s = (xc == d.n - 1) ? p.s - (d.n - 1) * d.stride : p.s + d.stride;
             xc = wrap_inc(xc, d.n);
             return l;
         }
         p.s = (xc == 0) ? p.s + (d.n - 1) * d.stride : p.s - d.stride;
         xc = wrap_dec(xc, d.n);
-        su3<D> l = su3_cast<D>(load_link(U, V, dir, p.s));
+        su3<D> l = su3_cast<D>(load_link_from<FILE>(U, V, dir, p.s));
         su3<D> a;
 #pragma unroll
         for (int r = 0; r < 3; ++r)
@@ -207,15 +235,15 @@ template <typename R, typename D = R> struct Plane {
         int& xc = along_mu ? p.xm : p.xn;
         const int dir = along_mu ? mu : nu;
         if (sign > 0) {
-            const su3<D> l = su3_cast<D>(load_link(U, V, dir, p.s));
+            const su3<D> l = su3_cast<D>(load_link_from<FILE>(U, V, dir, p.s));
             p.s = (xc == d.n - 1) ? p.s - (d.n - 1) * d.stride : p.s + d.stride;
             xc = wrap_inc(xc, d.n);
-            P = LGF_MEAS_ROW3 ? mul_nn_su3(P, l) : mul_nn(P, l);
+            P = mul_nn_su3(P, l);
         } else {
             p.s = (xc == 0) ? p.s + (d.n - 1) * d.stride : p.s - d.stride;
             xc = wrap_dec(xc, d.n);
-            const su3<D> l = su3_cast<D>(load_link(U, V, dir, p.s));
-            P = LGF_MEAS_ROW3 ? mul_na_su3(P, l) : mul_na(P, l);
+            const su3<D> l = su3_cast<D>(load_link_from<FILE>(U, V, dir, p.s));
+            P = mul_na_su3(P, l);
         }
     }
 };
@@ -608,7 +636,7 @@ template <typename R> constexpr bool meas_smem_acc() { return LGF_MEAS_SMEM_ACC 
 // extended by one more link.  Only its first two rows are kept when the
 // extension rebuilds the third (mul_nn_su3 / mul_na_su3 read rows 0 and 1 of
 // their left operand), so a parked path is exactly the one put there.
-constexpr int MEAS_STASH_ENTRIES = LGF_MEAS_ROW3 ? 6 : 9;
+constexpr int MEAS_STASH_ENTRIES = 6;
 template <typename R> struct PathStash {
     typename vec2_of<R>::type* p;  // entry k at p[k * MEAS_ACC_STRIDE]
     __device__ __forceinline__ void put(const su3<R>& P) const {
@@ -698,11 +726,11 @@ __device__ __forceinline__ su3<R> load_line(const MeasSmem<R>* sm, int sdir, int
 // are extended after other work are parked in the thread's shared-memory
 // column (PathStash: Pm(1,1), Pm(2,1), Pn(1,2)), and the leaves are added in
 // the order (1,1) | (2,1), (3,1), (1,2), (1,3), (2,2).
-template <typename R, typename Acc>
+template <typename R, bool FILE, typename Acc>
 __device__ __forceinline__ void plane_fields_body(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c,
                                                   int mu, int nu, const MeasSmem<R>* sm, int lane, int qa, int qb,
                                                   Acc G, Acc Fhat, PathStash<R> sa, PathStash<R> sb) {
-    Plane<R> P;
+    Plane<R, R, FILE> P;
     P.U = U;
     P.V = g.V;
     P.mu = mu;
@@ -771,7 +799,7 @@ __device__ __forceinline__ void plane_fields_body(const cplx<R>* __restrict__ U,
     }
 }
 
-template <typename R>
+template <typename R, bool FILE>
 __device__ __forceinline__ void plane_fields_smem(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c,
                                                   int mu, int nu, MeasSmem<R>* sm, int lane, int qa, int qb,
                                                   alg<R>& Greg, alg<R>& Fhreg) {
@@ -780,14 +808,14 @@ __device__ __forceinline__ void plane_fields_smem(const cplx<R>* __restrict__ U,
     if constexpr (meas_smem_acc<R>()) {
         R* col = &sm->acc[0][column];
         const SmemAcc<R> G{col}, Fhat{col + 8 * MEAS_ACC_STRIDE};
-        plane_fields_body<R>(U, g, s, c, mu, nu, sm, lane, qa, qb, G, Fhat, sa, sb);
+        plane_fields_body<R, FILE>(U, g, s, c, mu, nu, sm, lane, qa, qb, G, Fhat, sa, sb);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             Greg.v[k] = G.get(k);
             Fhreg.v[k] = Fhat.get(k);
         }
     } else {
-        plane_fields_body<R>(U, g, s, c, mu, nu, sm, lane, qa, qb, RegAcc<R>{Greg}, RegAcc<R>{Fhreg}, sa, sb);
+        plane_fields_body<R, FILE>(U, g, s, c, mu, nu, sm, lane, qa, qb, RegAcc<R>{Greg}, RegAcc<R>{Fhreg}, sa, sb);
     }
 }
 
@@ -804,94 +832,99 @@ __device__ __forceinline__ void plane_fields_smem(const cplx<R>* __restrict__ U,
 //        = -T(23,01) + T(13,02) - T(03,12),  T(a,b) = ReTr(F^a F^b)
 //                                             (TopologicalCharge.cpp:11-16)
 constexpr int MEAS_WARPS = 12;
+template <typename R, bool OUT, bool FILE>
+__device__ __forceinline__ void measure_tile(MeasSmem<R>* sm, const cplx<R>* __restrict__ U, const Geom& g, int slice, int chunk,
+                                             double2* __restrict__ partial, int nchunk, const MeasSites& out) {
+    const int lane = threadIdx.x, w = threadIdx.y, p = w % 6, part = w / 6;
+    const int off = meas_site_offset(g, meas_patched(g), chunk, lane);
+    const bool valid = off < g.Vs;
+    const int s = slice * g.Vs + (valid ? off : 0);
+    const Coord c = site_coord(g, s);
+    // phase 0: lines of length 2 and 3 in the 8 signed directions
+    if (w < 8) {
+        const int dir = w >> 1, sign = (w & 1) ? -1 : 1;
+        Plane<R, R, FILE> L;
+        L.U = U;
+        L.V = g.V;
+        L.mu = dir;
+        L.nu = dir;
+        L.dm = dir_of(g, c, dir);
+        L.dn = L.dm;
+        PlanePos y = {s, L.dm.x, L.dm.x};
+        su3<R> acc = L.step(y, true, sign);
+        L.ext(acc, y, true, sign);
+        store_line(sm, w, 2, lane, acc);
+        L.ext(acc, y, true, sign);
+        store_line(sm, w, 3, lane, acc);
+    }
+    __syncthreads();
+    // phase 1: this thread's plane and quadrants
+    alg<R> G, Fh;
+    if (FILE || valid) plane_fields_smem<R, FILE>(  // (file-order loads need the whole warp)
+        U, g, s, c, c_plane_mu[p], c_plane_nu[p], sm, lane, 2 * part, 2 * part + 2, G, Fh);
+    __syncthreads();  // every warp is done with the lines
+    if (part == 1 && valid) {
+        sm->part.G[p][lane] = G;
+        sm->part.Fh[p][lane] = Fh;
+    }
+    __syncthreads();
+    if (part == 0 && valid) {
+        const alg<R> G1 = sm->part.G[p][lane], F1 = sm->part.Fh[p][lane];
+        alg<R> F11;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            G.v[k] += G1.v[k];
+            Fh.v[k] += F1.v[k];
+            F11.v[k] = R(0.25) * G.v[k];
+            Fh.v[k] = fma(R(19.0 / 36.0), G.v[k], Fh.v[k]);
+        }
+        if (OUT) {
+            if (out.dbg_clover) store_alg_as_herm(out.dbg_clover + ((size_t)s * 6 + p) * 9, F11);
+            if (out.dbg_improved) store_alg_as_herm(out.dbg_improved + ((size_t)s * 6 + p) * 9, Fh);
+            if (out.swap) {
+                const alg<R> z = F11;
+                F11 = Fh;
+                Fh = z;
+            }
+        }
+        sm->F[p][lane] = Fh;
+        sm->E[p][lane] = retr_hh(F11, F11);
+    }
+    __syncthreads();
+    // phase 2: the site's e(x), q(x) and the tile's sums
+    if (w == 0) {
+        double e = 0.0, q = 0.0;
+        if (valid) {
+            e = ((sm->E[0][lane] + sm->E[1][lane]) + (sm->E[2][lane] + sm->E[3][lane])) +
+                (sm->E[4][lane] + sm->E[5][lane]);
+            q = -retr_hh(sm->F[5][lane], sm->F[0][lane]) + retr_hh(sm->F[4][lane], sm->F[1][lane]) -
+                retr_hh(sm->F[2][lane], sm->F[3][lane]);
+            if (OUT) {
+                if (out.e) out.e[s] = e;
+                if (out.q) out.q[s] = q;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            e += __shfl_xor_sync(0xffffffffu, e, o);
+            q += __shfl_xor_sync(0xffffffffu, q, o);
+        }
+        if (lane == 0) partial[slice * nchunk + chunk] = make_double2(e, q);
+    }
+}
+
 template <typename R, bool OUT>
 __global__ void __launch_bounds__(MEAS_SITES * MEAS_WARPS, 1) k_measure(const LatDesc<R>* __restrict__ descs,
                                                                        const int4* __restrict__ mtiles,
                                                                        const int2* __restrict__ seg, MeasSites out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MeasSmem<R>* sm = reinterpret_cast<MeasSmem<R>*>(smem_raw);
-    const int lane = threadIdx.x, w = threadIdx.y, p = w % 6, part = w / 6;
     const int2 r = *seg;  // this launch's tiles: mtiles[r.x, r.x + r.y)
     for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
         const int4 tile = mtiles[ti];
         const LatDesc<R>* d = descs + tile.x;
         const Geom g = d->g;
-        const int slice = tile.y, chunk = tile.z;
-        const int off = meas_site_offset(g, meas_patched(g), chunk, lane);
-        const bool valid = off < g.Vs;
-        const int s = slice * g.Vs + (valid ? off : 0);
-        const Coord c = site_coord(g, s);
-        const cplx<R>* __restrict__ U = d->U0;
-        // phase 0: lines of length 2 and 3 in the 8 signed directions
-        if (w < 8) {
-            const int dir = w >> 1, sign = (w & 1) ? -1 : 1;
-            Plane<R> L;
-            L.U = U;
-            L.V = g.V;
-            L.mu = dir;
-            L.nu = dir;
-            L.dm = dir_of(g, c, dir);
-            L.dn = L.dm;
-            PlanePos y = {s, L.dm.x, L.dm.x};
-            su3<R> acc = L.step(y, true, sign);
-            L.ext(acc, y, true, sign);
-            store_line(sm, w, 2, lane, acc);
-            L.ext(acc, y, true, sign);
-            store_line(sm, w, 3, lane, acc);
-        }
-        __syncthreads();
-        // phase 1: this thread's plane and quadrants
-        alg<R> G, Fh;
-        if (valid) plane_fields_smem<R>(U, g, s, c, c_plane_mu[p], c_plane_nu[p], sm, lane, 2 * part, 2 * part + 2, G, Fh);
-        __syncthreads();  // every warp is done with the lines
-        if (part == 1 && valid) {
-            sm->part.G[p][lane] = G;
-            sm->part.Fh[p][lane] = Fh;
-        }
-        __syncthreads();
-        if (part == 0 && valid) {
-            const alg<R> G1 = sm->part.G[p][lane], F1 = sm->part.Fh[p][lane];
-            alg<R> F11;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                G.v[k] += G1.v[k];
-                Fh.v[k] += F1.v[k];
-                F11.v[k] = R(0.25) * G.v[k];
-                Fh.v[k] = fma(R(19.0 / 36.0), G.v[k], Fh.v[k]);
-            }
-            if (OUT) {
-                if (out.dbg_clover) store_alg_as_herm(out.dbg_clover + ((size_t)s * 6 + p) * 9, F11);
-                if (out.dbg_improved) store_alg_as_herm(out.dbg_improved + ((size_t)s * 6 + p) * 9, Fh);
-                if (out.swap) {
-                    const alg<R> z = F11;
-                    F11 = Fh;
-                    Fh = z;
-                }
-            }
-            sm->F[p][lane] = Fh;
-            sm->E[p][lane] = retr_hh(F11, F11);
-        }
-        __syncthreads();
-        // phase 2: the site's e(x), q(x) and the tile's sums
-        if (w == 0) {
-            double e = 0.0, q = 0.0;
-            if (valid) {
-                e = ((sm->E[0][lane] + sm->E[1][lane]) + (sm->E[2][lane] + sm->E[3][lane])) +
-                    (sm->E[4][lane] + sm->E[5][lane]);
-                q = -retr_hh(sm->F[5][lane], sm->F[0][lane]) + retr_hh(sm->F[4][lane], sm->F[1][lane]) -
-                    retr_hh(sm->F[2][lane], sm->F[3][lane]);
-                if (OUT) {
-                    if (out.e) out.e[s] = e;
-                    if (out.q) out.q[s] = q;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                e += __shfl_xor_sync(0xffffffffu, e, o);
-                q += __shfl_xor_sync(0xffffffffu, q, o);
-            }
-            if (lane == 0) d->partial[slice * d->nchunk + chunk] = make_double2(e, q);
-        }
+        measure_tile<R, OUT, false>(sm, d->U0, g, tile.y, tile.z, d->partial, d->nchunk, out);
         __syncthreads();
     }
 }

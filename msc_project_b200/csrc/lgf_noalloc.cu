@@ -42,113 +42,19 @@ static __device__ __align__(256) double2 g_noalloc_scratch[NOALLOC_MAX_PARTIALS 
 std::mutex g_noalloc_mu;
 double2* g_noalloc_addr[NOALLOC_MAX_DEVICES] = {};
 
-// one link in the caller's file order: double2 L[(s*4 + mu)*9 + k]
-__device__ __forceinline__ su3<double> file_link(const double2* __restrict__ L, int s, int mu) {
-    su3<double> a;
-    const double2* p = L + ((size_t)s * 4 + mu) * 9;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        const double2 v = __ldg(p + k);
-        a.m[k] = cmk<double>(v.x, v.y);
-    }
-    return a;
-}
-
-// The a x b loops of the clover-type averages, walked over file-order links
-// (same quadrants and orientation as the engine's measurement kernel).
-template <int A, int B>
-__device__ __forceinline__ void leaves_file(const double2* __restrict__ L, const Geom& g, int s, const Coord& c, int mu,
-                                            int nu, su3<double>& sum) {
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        int y = s, ymu = c.x[mu], ynu = c.x[nu];
-        bool first = true;
-        su3<double> acc;
-        auto step = [&](int dir, int sign) {
-            int& yc = (dir == mu) ? ymu : ynu;
-            if (sign > 0) {
-                const su3<double> l = file_link(L, y, dir);
-                y = fwd(g, y, dir, yc);
-                yc = wrap_inc(yc, g.n[dir]);
-                acc = first ? l : mul_nn(acc, l);
-            } else {
-                y = bwd(g, y, dir, yc);
-                yc = wrap_dec(yc, g.n[dir]);
-                const su3<double> l = file_link(L, y, dir);
-                if (first) {
-#pragma unroll
-                    for (int r = 0; r < 3; ++r)
-#pragma unroll
-                        for (int cc = 0; cc < 3; ++cc) acc.m[3 * r + cc] = cmk<double>(l.m[3 * cc + r].re, -l.m[3 * cc + r].im);
-                } else {
-                    acc = mul_na(acc, l);
-                }
-            }
-            first = false;
-        };
-        auto seg = [&](int dir, int sign, int len) {
-            for (int i = 0; i < len; ++i) step(dir, sign);
-        };
-        if (q == 0) { seg(nu, +1, B); seg(mu, +1, A); seg(nu, -1, B); seg(mu, -1, A); }
-        else if (q == 1) { seg(mu, +1, A); seg(nu, -1, B); seg(mu, -1, A); seg(nu, +1, B); }
-        else if (q == 2) { seg(mu, -1, A); seg(nu, +1, B); seg(mu, +1, A); seg(nu, -1, B); }
-        else { seg(nu, -1, B); seg(mu, -1, A); seg(nu, +1, B); seg(mu, +1, A); }
-        su3_addto(sum, acc);
-    }
-}
-
-__device__ __forceinline__ void plane_fields_file(const double2* __restrict__ L, const Geom& g, int s, const Coord& c,
-                                                  int mu, int nu, alg<double>& F11, alg<double>& Fhat) {
-    su3<double> C;
-    su3_zero(C);
-    leaves_file<1, 1>(L, g, s, c, mu, nu, C);
-    F11 = field_strength(C, 0.25);
-    Fhat = alg_scale(19.0 / 9.0, F11);
-    su3_zero(C);
-    leaves_file<2, 2>(L, g, s, c, mu, nu, C);
-    Fhat = alg_axpby(1.0, Fhat, 1.0 / 36.0, field_strength(C, 0.25));
-    su3_zero(C);
-    leaves_file<1, 2>(L, g, s, c, mu, nu, C);
-    leaves_file<2, 1>(L, g, s, c, mu, nu, C);
-    Fhat = alg_axpby(1.0, Fhat, -32.0 / 45.0, field_strength(C, 1.0 / 8.0));
-    su3_zero(C);
-    leaves_file<1, 3>(L, g, s, c, mu, nu, C);
-    leaves_file<3, 1>(L, g, s, c, mu, nu, C);
-    Fhat = alg_axpby(1.0, Fhat, 1.0 / 15.0, field_strength(C, 1.0 / 8.0));
-}
-
-// grid (nchunk, N0), block (32 sites, 6 planes); partials[slice*nchunk + chunk]
-__global__ void __launch_bounds__(MEAS_SITES * 6) k_noalloc_measure(const double2* __restrict__ L, Geom g,
-                                                                    double2* __restrict__ partials) {
-    __shared__ alg<double> sF[6][MEAS_SITES];
-    __shared__ double sE[6][MEAS_SITES];
-    const int lane = threadIdx.x, p = threadIdx.y;
-    const int slice = blockIdx.y, chunk = blockIdx.x;
-    const int off = chunk * MEAS_SITES + lane;
-    const bool valid = off < g.Vs;
-    const int s = slice * g.Vs + (valid ? off : 0);
-    if (valid) {
-        const Coord c = site_coord(g, s);
-        alg<double> F11, Fh;
-        plane_fields_file(L, g, s, c, c_plane_mu[p], c_plane_nu[p], F11, Fh);
-        sF[p][lane] = Fh;
-        sE[p][lane] = retr_hh(F11, F11);
-    }
-    __syncthreads();
-    if (p == 0) {
-        double e = 0.0, q = 0.0;
-        if (valid) {
-            e = ((sE[0][lane] + sE[1][lane]) + (sE[2][lane] + sE[3][lane])) + (sE[4][lane] + sE[5][lane]);
-            q = -retr_hh(sF[5][lane], sF[0][lane]) + retr_hh(sF[4][lane], sF[1][lane]) -
-                retr_hh(sF[2][lane], sF[3][lane]);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            e += __shfl_xor_sync(0xffffffffu, e, o);
-            q += __shfl_xor_sync(0xffffffffu, q, o);
-        }
-        if (lane == 0) partials[slice * gridDim.x + chunk] = make_double2(e, q);
-    }
+// Grid (nchunk, N0), one 32-site tile per block: the one-launch measurement
+// (measure_tile) reading the caller's file-order links in place.  The fixed
+// scratch has no room for the loops' projections that lgf_measure.cuh shares
+// between sites.  Bound by link loads (load_link_from<true>): 14 per plane and
+// quadrant with shared paths instead of 40 for separate loops.  One B200, all
+// launches on 32x16^3: 2.81 ms with separate loops, 1.40 with shared paths and
+// a 16-byte load per lane, 1.20 with links read by lane pairs (1.24 by fours:
+// the selects cost more than the lines they save).
+__global__ void __launch_bounds__(MEAS_SITES * MEAS_WARPS, 1) k_noalloc_measure(const cplx<double>* __restrict__ L, Geom g,
+                                                                               double2* __restrict__ partials) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    measure_tile<double, false, true>(reinterpret_cast<MeasSmem<double>*>(smem_raw), L, g, blockIdx.y, blockIdx.x, partials,
+                                      gridDim.x, MeasSites{});
 }
 
 // one block per slice: fixed-order sums, then out = [E, Q, E_slice, Q_slice]
@@ -205,7 +111,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_noalloc_total(const double2* __
     }
 }
 
-// device address of the scratch array on the current device (looked up once)
+// device address of the scratch array on the current device (looked up once,
+// with the measurement kernel's shared-memory limit raised there)
 int noalloc_scratch(int dev, double2** out) {
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     if (!g_noalloc_addr[dev]) {
@@ -213,6 +120,11 @@ int noalloc_scratch(int dev, double2** out) {
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || !p) {
             if (e != cudaSuccess) cudaGetLastError();  // this lookup's own error
+            return LGF_ECUDA;
+        }
+        e = cudaFuncSetAttribute(k_noalloc_measure, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)measure_smem_bytes<double>());
+        if (e != cudaSuccess) {
+            cudaGetLastError();
             return LGF_ECUDA;
         }
         g_noalloc_addr[dev] = (double2*)p;
@@ -252,7 +164,8 @@ extern "C" int lgf_measure_noalloc(const double* links, const int shape[4], doub
     double2* partials = scratch;
     double2* slice_sums = scratch + NOALLOC_MAX_PARTIALS;
     cudaStream_t st = (cudaStream_t)stream;
-    k_noalloc_measure<<<dim3(nchunk, g.n[0]), dim3(MEAS_SITES, 6), 0, st>>>((const double2*)links, g, partials);
+    k_noalloc_measure<<<dim3(nchunk, g.n[0]), dim3(MEAS_SITES, MEAS_WARPS), measure_smem_bytes<double>(), st>>>(
+        (const cplx<double>*)links, g, partials);
     k_noalloc_slices<<<g.n[0], RED_THREADS, 0, st>>>(partials, nchunk, g, slice_sums, out);
     k_noalloc_total<<<1, RED_THREADS, 0, st>>>(slice_sums, g, out);
     // nothing was pending at entry, so an error now comes from these launches
