@@ -50,10 +50,10 @@ int validate_job(lgf_ctx* ctx, const lgf_job& j) {
 TileShape shape_for(lgf_ctx* ctx, int prec, const int shape[4]) {
     const long long V = 1LL * shape[0] * shape[1] * shape[2] * shape[3];
     if (has_tuned(ctx, prec, V)) return tuned_shape(ctx, prec, V);
-    TileShape best = default_shape(prec);
+    TileShape best = default_shape(prec, V);
     if (tune_shape(ctx, prec, shape, &best) != LGF_OK) {
         ctx->err.clear();
-        return default_shape(prec);
+        return default_shape(prec, V);
     }
     return best;
 }
@@ -92,7 +92,7 @@ int run_wave(lgf_ctx* ctx, int prec, std::vector<JobRun*>& runs, GroupBase* grp,
         members.push_back(&r->buf);
         eps.push_back(r->job->flow.eps);
         r->buf.eps = r->job->flow.eps;
-        LGF_CUDA_TRY(ctx, cudaMemsetAsync(r->buf.slot, 0, sizeof(int), ctx->stream));
+        LGF_CUDA_TRY(ctx, cudaMemsetAsync(r->buf.slot, 0, 2 * sizeof(int), ctx->stream));
         r->t = r->job->flow.t0;
     }
     int rc = grp->set_members(members);

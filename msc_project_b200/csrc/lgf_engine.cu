@@ -55,23 +55,20 @@ size_t footprint_bytes(const int shape[4], int precision, int meas_slots) {
     return b;
 }
 
-// Stage block size until the autotuner has run: FP64 256 threads (64 sites x 4
-// directions: one block per SM whose eight warps share their neighbours in
-// L1; 9% faster per stage than 128 on 24^3x48, 19% per job on 48^4), FP32 128
-// (three blocks per SM; 256 is 20% slower).
-#ifndef LGF_FP64_THREADS
-#define LGF_FP64_THREADS 384
-#endif
-#ifndef LGF_FP32_THREADS
-#define LGF_FP32_THREADS 128
-#endif
-int default_threads(int precision) { return precision == LGF_PREC_FP64 ? LGF_FP64_THREADS : LGF_FP32_THREADS; }
-
+// Stage block size until the autotuner has run: FP64 384 threads (96 adjacent
+// sites share their neighbours in L1; 7% faster per stage than 256 on 24^3x48
+// and 48^4), FP32 128.  A lattice too small to fill the SMs evenly with 96-site
+// tiles takes 32-site ones: the SM with the most tiles sets the time, so the
+// smaller tiles are taken where they cut that SM's sites by over a tenth
+// (8^4: 33 -> 23 us per step, 12^4 60 -> 54; 16^4, at 448 against 480 sites,
+// 140 either way).
 int stage_max_threads(int precision) { return precision == LGF_PREC_FP64 ? LGF_STAGE_MAXT_D : LGF_STAGE_MAXT_F; }
 
-TileShape default_shape(int precision) {
+TileShape default_shape(int precision, long long volume) {
+    const long long sms = 148;
+    auto most_sites = [&](long long tile) { return ((volume + tile - 1) / tile + sms - 1) / sms * tile; };
     TileShape t;
-    t.threads = default_threads(precision);
+    t.threads = precision == LGF_PREC_FP64 && 10 * most_sites(32) > 9 * most_sites(96) ? 384 : 128;
     return t;
 }
 
@@ -85,7 +82,7 @@ static const lgf_ctx::Tuned* find_tuned(const lgf_ctx* ctx, int precision, long 
 
 TileShape tuned_shape(const lgf_ctx* ctx, int precision, long long volume) {
     const lgf_ctx::Tuned* t = find_tuned(ctx, precision, volume);
-    return t ? t->shape : default_shape(precision);
+    return t ? t->shape : default_shape(precision, volume);
 }
 
 bool has_tuned(const lgf_ctx* ctx, int precision, long long volume) { return find_tuned(ctx, precision, volume) != nullptr; }
@@ -132,7 +129,7 @@ int buf_alloc(lgf_ctx* ctx, LatticeBuf& b, const int shape[4], int precision, in
     if (e == cudaSuccess) e = cudaMalloc(&b.A, Vp * 4 * 8 * rs);
     if (e == cudaSuccess) e = cudaMalloc(&b.partial, (size_t)b.g.n[0] * b.nchunk * sizeof(double2));
     if (e == cudaSuccess) e = cudaMalloc(&b.slice_sums, (size_t)b.g.n[0] * sizeof(double2));
-    if (e == cudaSuccess) e = cudaMalloc(&b.slot, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&b.slot, 2 * sizeof(int));
     if (e == cudaSuccess) {
         b.meas_cap = std::max(meas_slots, 1);
         e = cudaMalloc(&b.meas, (size_t)b.meas_cap * (2 + 2 * (size_t)b.g.n[0]) * sizeof(double));
@@ -157,7 +154,7 @@ size_t placed_bytes(const int shape[4], int precision, int meas_slots) {
     const size_t nchunk = ((size_t)shape[1] * shape[2] * shape[3] + MEAS_SITES - 1) / MEAS_SITES;
     return align256(3 * Vp * 4 * 18 * rs) + align256(Vp * 4 * 8 * rs) +
            align256((size_t)shape[0] * nchunk * sizeof(double2)) + align256((size_t)shape[0] * sizeof(double2)) +
-           align256(sizeof(int)) + align256((size_t)std::max(meas_slots, 1) * (2 + 2 * (size_t)shape[0]) * sizeof(double));
+           align256(2 * sizeof(int)) + align256((size_t)std::max(meas_slots, 1) * (2 + 2 * (size_t)shape[0]) * sizeof(double));
 }
 
 void buf_place(LatticeBuf& b, const int shape[4], int precision, int meas_slots, void* mem) {
@@ -180,7 +177,7 @@ void buf_place(LatticeBuf& b, const int shape[4], int precision, int meas_slots,
     b.slice_sums = (double2*)p;
     p += align256((size_t)b.g.n[0] * sizeof(double2));
     b.slot = (int*)p;
-    p += align256(sizeof(int));
+    p += align256(2 * sizeof(int));
     b.meas_cap = std::max(meas_slots, 1);
     b.meas = (double*)p;
 }
@@ -216,18 +213,16 @@ int count_measurements(const lgf_flow_opts& o) {
 //          then per selected member k: member, segment offset, tiles, first
 //          output tile, N0, first output slice]
 // Outputs: mtiles (the selected segments back to back), rtiles (member, t)
-// for t < N0, jobs[k] = member, counts = {tiles, slices, nsel}.  Grid
+// for t < N0, counts = {tiles, slices}.  Grid
 // (max(nsel, 1), any): block (k, y) copies a share of segment k.
 constexpr int SEL_HEADER = 4, SEL_SEGS = 2, SEL_FIELDS = 6;  // ints; int2 segments before the launch segments; ints
 __global__ void __launch_bounds__(256) k_select_measure(const int* __restrict__ sel, int fields,
                                                         const int4* __restrict__ all, int4* __restrict__ mtiles,
-                                                        int2* __restrict__ rtiles, int* __restrict__ jobs,
-                                                        int* __restrict__ counts) {
+                                                        int2* __restrict__ rtiles, int* __restrict__ counts) {
     const int nsel = sel[0];
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         counts[0] = sel[1];
         counts[1] = sel[2];
-        counts[2] = nsel;
     }
     const int k = blockIdx.x;
     if (k >= nsel) return;
@@ -235,10 +230,8 @@ __global__ void __launch_bounds__(256) k_select_measure(const int* __restrict__ 
     const int member = f[0], off = f[1], n = f[2], mstart = f[3], n0 = f[4], rstart = f[5];
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n; i += gridDim.y * blockDim.x)
         mtiles[mstart + i] = all[off + i];
-    if (blockIdx.y == 0) {
+    if (blockIdx.y == 0)
         for (int t = threadIdx.x; t < n0; t += blockDim.x) rtiles[rstart + t] = make_int2(member, t);
-        if (threadIdx.x == 0) jobs[k] = member;
-    }
 }
 
 static inline size_t align16(size_t n) { return (n + 15) & ~size_t(15); }
@@ -260,7 +253,6 @@ public:
         cudaFree(d_mtiles_);
         cudaFree(d_all_mtiles_);
         cudaFree(d_rtiles_);
-        cudaFree(d_jobs_);
         cudaFree(d_counts_);
         cudaFree(d_seg_);
         cudaFree(d_sel_);
@@ -272,10 +264,10 @@ public:
         const long long cap_sites = max_tiles_ * (threads_ / 4);
         tiles_cap_ = std::max(max_tiles_, sizeof(R) == sizeof(float) ? cap_sites / PLAQ_SITES + cap_sites / UPDATE_SITES + 2 * max_members_ : 0LL);
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_tiles_, sizeof(int2) * tiles_cap_));
-        LGF_CUDA_TRY(ctx_, cudaMalloc(&d_counts_, sizeof(int) * 4));
+        LGF_CUDA_TRY(ctx_, cudaMalloc(&d_counts_, sizeof(int) * 2));
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_seg_, sizeof(int2) * 3 * slots_));
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_sel_, sizeof(int) * sel_ints(max_members_)));
-        LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_counts_, 0, sizeof(int) * 4, ctx_->stream));
+        LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_counts_, 0, sizeof(int) * 2, ctx_->stream));
         LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_sel_, 0, sizeof(int) * sel_ints(max_members_), ctx_->stream));
         int nb = 0;
         LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_stage<R, 1>, threads_, 0));
@@ -306,11 +298,9 @@ public:
             // largest resident set the tile capacity allows (x0 extents <= 256)
             mtiles_cap_ = max_tiles_ * threads_ / (4 * MEAS_SITES) + 256LL * max_members_;
             rtiles_cap_ = 256LL * max_members_;
-            jobs_cap_ = max_members_;
             LGF_CUDA_TRY(ctx_, cudaMalloc(&d_mtiles_, sizeof(int4) * mtiles_cap_));
             LGF_CUDA_TRY(ctx_, cudaMalloc(&d_all_mtiles_, sizeof(int4) * mtiles_cap_));
             LGF_CUDA_TRY(ctx_, cudaMalloc(&d_rtiles_, sizeof(int2) * rtiles_cap_));
-            LGF_CUDA_TRY(ctx_, cudaMalloc(&d_jobs_, sizeof(int) * jobs_cap_));
         }
         return LGF_OK;
     }
@@ -389,15 +379,12 @@ public:
         }
         long long rt = 0;
         for (auto* b : members) rt += b->g.n[0];
-        if (rt > rtiles_cap_ || (long long)members.size() > jobs_cap_) {
+        if (rt > rtiles_cap_) {
             if (captured()) return set_error(ctx_, LGF_EINVAL, "reduction list grew after capture");
             LGF_CUDA_TRY(ctx_, cudaStreamSynchronize(ctx_->stream));
             cudaFree(d_rtiles_);
-            cudaFree(d_jobs_);
             rtiles_cap_ = std::max(rt, (long long)max_members_ * 64);
-            jobs_cap_ = max_members_;
             LGF_CUDA_TRY(ctx_, cudaMalloc(&d_rtiles_, sizeof(int2) * rtiles_cap_));
-            LGF_CUDA_TRY(ctx_, cudaMalloc(&d_jobs_, sizeof(int) * jobs_cap_));
         }
         ntiles_ = (int)tiles.size();
         seg_tiles_.clear();
@@ -472,7 +459,7 @@ public:
                 tu[round] += plane_units(members_[i]->g, round, unit_sites_);
             }
         }
-        if (tm > mtiles_cap_ || tr > rtiles_cap_ || (long long)which.size() > jobs_cap_ ||
+        if (tm > mtiles_cap_ || tr > rtiles_cap_ ||
             std::max(tu[0], tu[1]) > (1LL << 31) - 1024)
             return set_error(ctx_, LGF_EINVAL, "measurement list exceeds capacity");
         sel[0] = (int)which.size();
@@ -507,7 +494,7 @@ public:
             LGF_CUDA_TRY(ctx_, ctx_->list_stage.release(ctx_->stream));
         }
         k_select_measure<<<dim3(std::max<int>(1, (int)which.size()), 16), 256, 0, ctx_->stream>>>(
-            d_sel_, sel_fields(), d_all_mtiles_, d_mtiles_, d_rtiles_, d_jobs_, d_counts_ + 1);
+            d_sel_, sel_fields(), d_all_mtiles_, d_mtiles_, d_rtiles_, d_counts_);
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
     }
@@ -564,7 +551,7 @@ public:
         return LGF_OK;
     }
     int launches_per_step() const override { return 3 * (stage_nseg_ + 2 * plaq_nseg_); }
-    int launches_per_measure() const override { return (meas_small_ ? 1 : 0) + (meas_nseg_ ? 5 : 0) + 2; }
+    int launches_per_measure() const override { return (meas_small_ ? 1 : 0) + (meas_nseg_ ? 4 * meas_nseg_ + 1 : 0) + 1; }
     int threads() const override { return threads_; }
     const TileShape& shape() const override { return shape_; }
 
@@ -639,10 +626,8 @@ private:
     int launch_measurement(int nseg, bool small) {
         NvtxRange r("lgf.measure_launch");
         const int rg = dynamic_ ? ctx_->sm_count : std::max(1, (int)std::min<long long>(rtiles_cap_, 4 * ctx_->sm_count));
-        const int jg = dynamic_ ? std::min(jobs_cap_, 4 * ctx_->sm_count) : std::max(1, (int)std::min<long long>(jobs_cap_, 4 * ctx_->sm_count));
         launch_measure_kernels<false>(nseg, small, MeasSites{});
-        k_reduce_slices<R><<<rg, RED_THREADS, 0, ctx_->stream>>>(d_desc_, d_rtiles_, d_counts_ + 2);
-        k_reduce_total<R><<<std::max(1, jg), RED_THREADS, 0, ctx_->stream>>>(d_desc_, d_jobs_, d_counts_ + 3);
+        k_reduce<R><<<rg, RED_THREADS, 0, ctx_->stream>>>(d_desc_, d_rtiles_, d_counts_ + 1);
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
     }
@@ -697,7 +682,7 @@ private:
     TileShape list_shape(long long V) const {
         if (!per_volume_) return shape_;
         const int prec = std::is_same<R, double>::value ? LGF_PREC_FP64 : LGF_PREC_FP32MIXED;
-        return has_tuned(ctx_, prec, V) ? tuned_shape(ctx_, prec, V) : default_shape(prec);
+        return has_tuned(ctx_, prec, V) ? tuned_shape(ctx_, prec, V) : default_shape(prec, V);
     }
 
     lgf_ctx* ctx_;
@@ -716,10 +701,8 @@ private:
     int4* d_all_mtiles_ = nullptr;  // every member's measurement tiles
     int* d_sel_ = nullptr;          // selection table of the next measurement
     int2* d_rtiles_ = nullptr;
-    int* d_jobs_ = nullptr;
-    int* d_counts_ = nullptr;  // (unused), nmtiles, nrtiles, njobs
+    int* d_counts_ = nullptr;  // nmtiles, nrtiles
     long long mtiles_cap_ = 0, rtiles_cap_ = 0;
-    int jobs_cap_ = 0;
     int ntiles_ = 0;
     int stage_grid_max_ = 1, small_grid_max_ = 1, loops_grid_max_ = 1, planes_grid_max_ = 1;
     int meas_groups_ = LOOP_MAX_GROUPS, unit_sites_ = PLANE_MAX_SITES;  // tiles per loops block, sites per plane unit
@@ -1104,7 +1087,7 @@ int lgf_flow(lgf_lattice* lat, const lgf_flow_opts* o, lgf_meas* out) {
     lat->buf.eps = o->eps;
     rc = grp->set_eps({o->eps});
     if (rc != LGF_OK) return rc;
-    LGF_CUDA_TRY(ctx, cudaMemsetAsync(lat->buf.slot, 0, sizeof(int), ctx->stream));
+    LGF_CUDA_TRY(ctx, cudaMemsetAsync(lat->buf.slot, 0, 2 * sizeof(int), ctx->stream));
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     LGF_CUDA_TRY(ctx, cudaEventCreate(&ev0));
     LGF_CUDA_TRY(ctx, cudaEventCreate(&ev1));
@@ -1248,7 +1231,7 @@ int lgf_profile_kernels(lgf_lattice* lat, double eps, int nrep, double ms[4]) {
     lat->buf.eps = eps;
     rc = grp->set_eps({eps});
     if (rc != LGF_OK) return rc;
-    LGF_CUDA_TRY(ctx, cudaMemsetAsync(lat->buf.slot, 0, sizeof(int), ctx->stream));
+    LGF_CUDA_TRY(ctx, cudaMemsetAsync(lat->buf.slot, 0, 2 * sizeof(int), ctx->stream));
     std::vector<cudaEvent_t> ev(2 * 4 * nrep);
     for (auto& e : ev) LGF_CUDA_TRY(ctx, cudaEventCreate(&e));
     double acc[4] = {0, 0, 0, 0};

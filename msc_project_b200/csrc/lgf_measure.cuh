@@ -21,7 +21,7 @@
 //   k_meas_planes<R, ROUND>   shifts along nu (from memory), then along mu
 //                             (through shared memory): F, F^, e and q terms
 //   k_meas_sites<R>           e(x), q(x) and their sums per 32-site chunk
-//   k_reduce_slices / k_reduce_total (lgf_kernels.cuh)
+//   k_reduce (lgf_kernels.cuh)
 //
 // A round handles three planes: round 0 (01), (02), (03), round 1 their
 // complements (23), (13), (12), whose q terms pair with round 0's F^.  The

@@ -292,7 +292,7 @@ int lgf_server::admit(ServeJob* j) {
     if (rc != LGF_OK) return rc;
     j->buf.eps = j->job.flow.eps;
     j->t = j->job.flow.t0;
-    LGF_CUDA_TRY(ctx, cudaMemsetAsync(j->buf.slot, 0, sizeof(int), adm));
+    LGF_CUDA_TRY(ctx, cudaMemsetAsync(j->buf.slot, 0, 2 * sizeof(int), adm));
     LGF_CUDA_TRY(ctx, cudaEventRecord(j->ready, adm));
     return LGF_OK;
 }
@@ -547,7 +547,7 @@ void lgf_server::run() {
 // measurement tuned (by under 2%) on 24^3x48 slowed a served mix of four
 // volumes by 12%.  Each job's work order is still its own class's tuned
 // order (the groups' per-volume lists).
-static TileShape serve_shape(const lgf_ctx*, int prec) { return default_shape(prec); }
+static TileShape serve_shape(const lgf_ctx*, int prec) { return default_shape(prec, 1LL << 40); }
 
 extern "C" {
 

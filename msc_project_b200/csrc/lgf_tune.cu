@@ -69,7 +69,7 @@ int tune_shape(lgf_ctx* ctx, int prec, const int shape[4], TileShape* best) {
     if (rc != LGF_OK) return rc;
     rc = launch_generate(ctx, b, 12345, 0.5);
     b.eps = 0.01;
-    TileShape cur = default_shape(prec);
+    TileShape cur = default_shape(prec, b.g.V);
     float cur_ms = 0.f;
     const double MB = double(1 << 20);
     // A candidate replaces the current shape only when it is more than 2%
