@@ -10,9 +10,13 @@
 // overrelaxation reflects the subgroup (:78-104).
 //
 // B200 mapping: one launch per (parity, direction) class updates all its links
-// in place in parallel -- the staple of a link reads only other directions and
-// opposite-parity links of its own direction, so the class has no internal
-// dependencies.  Random numbers come from a counter hash of (seed, class epoch,
+// in place in parallel, on a copy of the links in parity order -- the staple of
+// a link reads only other directions and opposite-parity links of its own
+// direction, so the class has no internal dependencies.  Measured per class
+// launch, FP64, against site order (same bits): 32x16^3 heatbath 40 -> 30 us,
+// overrelaxation 33 -> 22; 24^3x48 197 -> 145 and 169 -> 109; FP32 100 -> 100
+// and 68 -> 60 on 24^3x48; the copy there and back costs about three launches.
+//  Random numbers come from a counter hash of (seed, class epoch,
 // subgroup, site, draw), so results do not depend on the launch shape.  The
 // rejection loop is bounded (HB_MAX_ATTEMPTS); a subgroup whose draws all
 // fail is left unchanged and counted.  The reference seeds from
@@ -36,29 +40,107 @@ __device__ __forceinline__ double hb_draw(unsigned long long seed, unsigned long
     return unit_open(seed, base + (unsigned long long)k);
 }
 
-// site of parity p with index t among the V/2 sites of that parity
-// (N3 is even: every x0,x1,x2 row holds N3/2 sites of each parity)
-__device__ __forceinline__ int parity_site(const Geom& g, int p, int t) {
-    const int half3 = g.n[3] >> 1;
-    const int row = t / half3, k = t - row * half3;
-    const int x2 = row % g.n[2];
-    const int r1 = row / g.n[2];
-    const int x1 = r1 % g.n[1];
-    const int x0 = r1 / g.n[1];
-    const int x3 = 2 * k + ((p + x0 + x1 + x2) & 1);
-    return row * g.n[3] + x3;
+// Sweeps run on a copy of the links in parity order: the V/2 even sites, then
+// the odd ones, each in site order, in the same 32-site blocks.  A class
+// updates and reads whole runs of one parity there, where in site order every
+// second site of a run is of the other parity and half of each 32-byte sector
+// that a warp fetches goes unused -- and L2 bandwidth is what bounds a class
+// (32x16^3, FP64: 12 TB/s in site order).  The copy takes the ring's second
+// buffer, free between flows.
+//
+// N3 is even, so each (x0, x1, x2) row holds h = N3/2 sites of each parity:
+// site x of parity p is entry row * h + k of its parity, x3 = 2k + o with
+// o = (p + x0 + x1 + x2) & 1.  A step along x0, x1 or x2 keeps k and o; a step
+// along x3 flips o and moves k by one when it leaves the pair.
+struct ParitySite {
+    int x0, x1, x2;  // coordinates of the row
+    int row, k, o, p;
+};
+__host__ __device__ __forceinline__ ParitySite parity_site(const Geom& g, int p, int t) {
+    const int h = g.n[3] >> 1;
+    ParitySite a;
+    a.p = p;
+    a.row = t / h;
+    a.k = t - a.row * h;
+    a.x2 = a.row % g.n[2];
+    const int r1 = a.row / g.n[2];
+    a.x1 = r1 % g.n[1];
+    a.x0 = r1 / g.n[1];
+    a.o = (p + a.x0 + a.x1 + a.x2) & 1;
+    return a;
+}
+// entry of the parity-ordered links
+__host__ __device__ __forceinline__ int parity_index(const Geom& g, const ParitySite& a) {
+    return (a.p ? g.V >> 1 : 0) + a.row * (g.n[3] >> 1) + a.k;
+}
+__host__ __device__ __forceinline__ int site_index(const Geom& g, const ParitySite& a) { return a.row * g.n[3] + 2 * a.k + a.o; }
+__host__ __device__ __forceinline__ ParitySite parity_step(const Geom& g, ParitySite a, int d, int sign) {
+    a.p ^= 1;
+    if (d == 3) {
+        const int h = g.n[3] >> 1;
+        if (sign > 0 && a.o == 1) a.k = a.k == h - 1 ? 0 : a.k + 1;
+        if (sign < 0 && a.o == 0) a.k = a.k == 0 ? h - 1 : a.k - 1;
+        a.o ^= 1;
+        return a;
+    }
+    const int n = sel4(d, g.n[0], g.n[1], g.n[2], 0), x = sel4(d, a.x0, a.x1, a.x2, 0);
+    const int rows = d == 0 ? g.n[1] * g.n[2] : (d == 1 ? g.n[2] : 1);
+    const int move = sign > 0 ? (x == n - 1 ? 1 - n : 1) : (x == 0 ? n - 1 : -1);
+    a.row += move * rows;
+    if (d == 0) a.x0 += move;
+    if (d == 1) a.x1 += move;
+    if (d == 2) a.x2 += move;
+    return a;
 }
 
+// links of site order -> parity order (TO) or back
+template <typename R, bool TO>
+__global__ void __launch_bounds__(128) k_parity_order(const cplx<R>* __restrict__ in, cplx<R>* __restrict__ out, Geom g) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, mu = blockIdx.y;
+    if (t >= g.V) return;
+    const int half = g.V >> 1;
+    const ParitySite a = parity_site(g, t >= half, t >= half ? t - half : t);
+    const int s = site_index(g, a);
+    store_link(out, g.V, mu, TO ? t : s, load_link(in, g.V, mu, TO ? s : t));
+}
+
+// the staple sum of staple_sum() (same products in the same order) on parity-ordered links
 template <typename R>
-__global__ void __launch_bounds__(128) k_checkerboard(cplx<R>* __restrict__ U, Geom g, int mu, int parity, double beta,
-                                                      unsigned long long seed, unsigned long long epoch, int overrelax,
-                                                      unsigned int* __restrict__ failures) {
+__device__ __forceinline__ su3<R> staple_sum_parity(const cplx<R>* U, const Geom& g, const ParitySite& x, int mu) {
+    const int V = g.V;
+    su3<R> S;
+    su3_zero(S);
+    const int s = parity_index(g, x), xpm = parity_index(g, parity_step(g, x, mu, 1));
+#pragma unroll
+    for (int nu = 0; nu < 4; ++nu) {
+        if (nu == mu) continue;
+        const ParitySite m = parity_step(g, x, nu, -1);
+        const int xpn = parity_index(g, parity_step(g, x, nu, 1)), xmn = parity_index(g, m);
+        const int xmnpm = parity_index(g, parity_step(g, m, mu, 1));
+        {
+            const su3<R> t = mul_nn_su3(load_link(U, V, nu, s), load_link(U, V, mu, xpn));
+            acc_na(S, load_link(U, V, nu, xpm), t);
+        }
+        {
+            const su3<R> t = mul_nn_su3(load_link(U, V, mu, xmn), load_link(U, V, nu, xmnpm));
+            acc_an(S, t, load_link(U, V, nu, xmn));
+        }
+    }
+    return S;
+}
+
+// One (parity, direction) class.  MINB: resident blocks per SM that the
+// registers are capped for (heatbath_blocks).
+template <typename R, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_checkerboard(cplx<R>* U, Geom g, int mu, int parity, double beta,
+                                                            unsigned long long seed, unsigned long long epoch, int overrelax,
+                                                            unsigned int* __restrict__ failures) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (g.V >> 1)) return;
-    const int s = parity_site(g, parity, t);
-    const Coord c = site_coord(g, s);
-    const su3<R> A = staple_sum<R>(U, g, s, c, mu);
-    su3<R> u = load_link(U, g.V, mu, s);
+    const ParitySite x = parity_site(g, parity, t);
+    const int s = site_index(g, x), at = parity_index(g, x);  // the random numbers are keyed by the site
+    const su3<R> A = staple_sum_parity<R>(U, g, x, mu);
+    su3<R> u = load_link(U, g.V, mu, at);
 #pragma unroll 1
     for (int sg = 0; sg < 3; ++sg) {
         const int m = sg == 2 ? 1 : 0, n = sg == 0 ? 1 : 2;  // (0,1), (0,2), (1,2)
@@ -151,7 +233,7 @@ __global__ void __launch_bounds__(128) k_checkerboard(cplx<R>* __restrict__ U, G
             }
         }
     }
-    store_link(U, g.V, mu, s, u);
+    store_link(U, g.V, mu, at, u);
 }
 
 // Random SU(3) per link as a product of three random SU(2) subgroup elements
@@ -221,10 +303,16 @@ __global__ void __launch_bounds__(256) k_plaquette(const cplx<R>* __restrict__ U
                 const su3<R> b = load_link(U, g.V, nu, fwd(g, s, mu, c.x[mu]));
                 const su3<R> cc = load_link(U, g.V, mu, fwd(g, s, nu, c.x[nu]));
                 const su3<R> d = load_link(U, g.V, nu, s);
+                // ReTr U_mu(x) U_nu(x+mu) (U_nu(x) U_mu(x+nu))^dag: entry by entry, no third product
                 const su3<R> ab = mul_nn(a, b);
                 const su3<R> dc = mul_nn(d, cc);
-                const su3<R> p = mul_na(ab, dc);  // U_mu(x) U_nu(x+mu) (U_nu(x) U_mu(x+nu))^dag
-                acc += (double)p.m[0].re + (double)p.m[4].re + (double)p.m[8].re;
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    R row = R(0);
+#pragma unroll
+                    for (int k = 3 * r; k < 3 * r + 3; ++k) row = fma(ab.m[k].re, dc.m[k].re, fma(ab.m[k].im, dc.m[k].im, row));
+                    acc += (double)row;
+                }
             }
     }
     sh[threadIdx.x] = acc;
@@ -236,32 +324,48 @@ __global__ void __launch_bounds__(256) k_plaquette(const cplx<R>* __restrict__ U
     if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 
+// The class kernel for nb blocks.  FP64 at 3 blocks per SM (168 registers) runs
+// a full wave of blocks in 1/1.3 of the time of 4 (128 registers, some spills),
+// so 4 are taken where they save enough waves (32x16^3: one wave instead of
+// two, 22 against 24 us; 24^3x48: 6 of 3 beat 5 of 4).  FP32 takes 5 (96).
+template <typename R> auto heatbath_kernel(int nb, int sms) {
+    auto waves = [&](int per_sm) { return (nb + per_sm * sms - 1) / (per_sm * sms); };
+    if constexpr (sizeof(R) == sizeof(double)) return 10 * waves(3) > 13 * waves(4) ? k_checkerboard<R, 4> : k_checkerboard<R, 3>;
+    else return k_checkerboard<R, 5>;
+}
+
 // n_iter x (heatbath sweep unless or_only, then or_per_hb overrelaxation sweeps)
 template <typename R>
 int heatbath_impl(lgf_ctx* ctx, lgf_lattice* lat, double beta, int n_iter, int or_per_hb, unsigned long long seed,
                   unsigned long long* rejected, bool or_only) {
     LatticeBuf& b = lat->buf;
-    unsigned int* dfail = nullptr;
-    LGF_CUDA_TRY(ctx, cudaMalloc(&dfail, sizeof(unsigned int)));
-    cudaMemsetAsync(dfail, 0, sizeof(unsigned int), ctx->stream);
-    const int half = b.g.V / 2, th = 128, nb = (half + th - 1) / th;
+    unsigned int* dfail = reinterpret_cast<unsigned int*>(b.slot);  // (a flow resets its slot before it counts)
+    LGF_CUDA_TRY(ctx, cudaMemsetAsync(dfail, 0, sizeof(unsigned int), ctx->stream));
+    const int V = b.g.V, th = 128, nb = (V / 2 + th - 1) / th;
+    cplx<R>*U = (cplx<R>*)b.U[0], *P = (cplx<R>*)b.U[1];
+    const dim3 order((V + th - 1) / th, 4);
     cudaError_t e = cudaSuccess;
+    const bool any = n_iter > 0 && (!or_only || or_per_hb > 0);
+    if (any) k_parity_order<R, true><<<order, th, 0, ctx->stream>>>(U, P, b.g);
+    auto sweep_class = heatbath_kernel<R>(nb, ctx->sm_count);
     for (int it = 0; it < n_iter && e == cudaSuccess; ++it) {
         for (int sweep = or_only ? 1 : 0; sweep <= or_per_hb && e == cudaSuccess; ++sweep) {
             const int over = sweep > 0;
             for (int par = 0; par <= 1; ++par)
                 for (int mu = 0; mu < 4; ++mu) {
                     const unsigned long long epoch = lat->hb_epoch++;
-                    k_checkerboard<R><<<nb, th, 0, ctx->stream>>>((cplx<R>*)b.U[0], b.g, mu, par, beta, seed, epoch,
-                                                                  over, dfail);
+                    sweep_class<<<nb, th, 0, ctx->stream>>>(P, b.g, mu, par, beta, seed, epoch, over, dfail);
                 }
             e = cudaGetLastError();
         }
     }
+    if (any && e == cudaSuccess) {
+        k_parity_order<R, false><<<order, th, 0, ctx->stream>>>(P, U, b.g);
+        e = cudaGetLastError();
+    }
     unsigned int h = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, dfail, sizeof h, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(dfail);
     if (e != cudaSuccess) return set_error(ctx, LGF_ECUDA, "heatbath failed: %s", cudaGetErrorString(e));
     if (rejected) *rejected = h;
     return LGF_OK;
@@ -331,8 +435,7 @@ int lgf_plaquette(lgf_lattice* lat, double* avg) {
     cudaSetDevice(ctx->device);
     const Geom g = lat->buf.g;
     const int nb = (g.V + 255) / 256;
-    double* dp = nullptr;
-    LGF_CUDA_TRY(ctx, cudaMalloc(&dp, sizeof(double) * nb));
+    double* dp = (double*)lat->buf.U[1];  // the ring's second buffer, free between flows
     if (lat->buf.prec == LGF_PREC_FP64)
         k_plaquette<double><<<nb, 256, 0, ctx->stream>>>((const cplx<double>*)lat->buf.U[0], g, dp);
     else
@@ -341,7 +444,6 @@ int lgf_plaquette(lgf_lattice* lat, double* avg) {
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), dp, sizeof(double) * nb, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(dp);
     if (e != cudaSuccess) return set_error(ctx, LGF_ECUDA, "plaquette failed: %s", cudaGetErrorString(e));
     double sum = 0.0;
     for (double v : h) sum += v;
