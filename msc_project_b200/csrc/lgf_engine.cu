@@ -625,8 +625,11 @@ private:
     }
     int launch_measurement(int nseg, bool small) {
         NvtxRange r("lgf.measure_launch");
-        const int rg = dynamic_ ? ctx_->sm_count : std::max(1, (int)std::min<long long>(rtiles_cap_, 4 * ctx_->sm_count));
         launch_measure_kernels<false>(nseg, small, MeasSites{});
+        return launch_reduce();
+    }
+    int launch_reduce() override {
+        const int rg = dynamic_ ? ctx_->sm_count : std::max(1, (int)std::min<long long>(rtiles_cap_, 4 * ctx_->sm_count));
         k_reduce<R><<<rg, RED_THREADS, 0, ctx_->stream>>>(d_desc_, d_rtiles_, d_counts_ + 1);
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
@@ -869,14 +872,14 @@ int upload_links(lgf_ctx* ctx, LatticeBuf& b, const double* host) {
     return rc;
 }
 
-int download_links(lgf_ctx* ctx, const LatticeBuf& b, double* host) {
-    const size_t bytes = (size_t)b.g.V * 4 * 18 * sizeof(double);
-    char* stage = (char*)file_staging(b);
-    int rc = launch_to_file(ctx, b, (double*)stage);
-    if (rc != LGF_OK) return rc;
+// device -> host on the context's stream, complete on return: one DMA into
+// page-locked memory, else through the context's two pinned chunks, the host
+// copy of one overlapping the DMA of the other
+int copy_out(lgf_ctx* ctx, void* host, const void* dev, size_t bytes) {
+    const char* src = (const char*)dev;
     cudaError_t e = cudaSuccess;
     if (is_pinned(host)) {
-        e = cudaMemcpyAsync(host, stage, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+        e = cudaMemcpyAsync(host, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     } else {
         std::lock_guard<std::mutex> lk(ctx->pin_mu);
@@ -889,7 +892,7 @@ int download_links(lgf_ctx* ctx, const LatticeBuf& b, double* host) {
         const size_t nchunks = (bytes + PIN_CHUNK - 1) / PIN_CHUNK;
         auto issue = [&](size_t i) {
             const size_t off = i * PIN_CHUNK, n = std::min(PIN_CHUNK, bytes - off);
-            cudaError_t r = cudaMemcpyAsync(ctx->pin[i & 1], stage + off, n, cudaMemcpyDeviceToHost, ctx->stream);
+            cudaError_t r = cudaMemcpyAsync(ctx->pin[i & 1], src + off, n, cudaMemcpyDeviceToHost, ctx->stream);
             return r == cudaSuccess ? cudaEventRecord(ctx->pin_done[i & 1], ctx->stream) : r;
         };
         e = issue(0);
@@ -902,8 +905,14 @@ int download_links(lgf_ctx* ctx, const LatticeBuf& b, double* host) {
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     }
-    if (e != cudaSuccess) return set_error(ctx, LGF_ECUDA, "download failed: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return set_error(ctx, LGF_ECUDA, "copy to the host failed: %s", cudaGetErrorString(e));
     return LGF_OK;
+}
+
+int download_links(lgf_ctx* ctx, const LatticeBuf& b, double* host) {
+    double* stage = file_staging(b);
+    const int rc = launch_to_file(ctx, b, stage);
+    return rc == LGF_OK ? copy_out(ctx, host, stage, (size_t)b.g.V * 4 * 18 * sizeof(double)) : rc;
 }
 
 }  // namespace lgf
@@ -1038,15 +1047,16 @@ static int lattice_group(lgf_lattice* lat, GroupBase** out) {
 }
 
 // One measurement pass over a lattice's links with per-site (and, when asked,
-// per (site, plane) F / F^) outputs.
+// per (site, plane) F / F^) outputs, enqueued.
 static int single_measure(lgf_lattice* lat, const MeasSites& out) {
     GroupBase* grp = nullptr;
     int rc = lattice_group(lat, &grp);
-    if (rc == LGF_OK) rc = grp->launch_sites(out);
-    if (rc != LGF_OK) return rc;
-    LGF_CUDA_TRY(lat->ctx, cudaStreamSynchronize(lat->ctx->stream));
-    return LGF_OK;
+    return rc == LGF_OK ? grp->launch_sites(out) : rc;
 }
+
+// Where a pass leaves its site densities: the loops' scratch, dead once the
+// planes are done (and free in the one-launch measurement).
+static double* site_scratch(const LatticeBuf& b) { return (double*)b.U[1]; }
 
 static int fetch_meas(lgf_ctx* ctx, const LatticeBuf& b, int nmeas, std::vector<double>& host) {
     const size_t per = 2 + 2 * (size_t)b.g.n[0];
@@ -1166,52 +1176,35 @@ int lgf_site_densities(lgf_lattice* lat, double* e_site, double* q_site) {
     lgf_ctx* ctx = lat->ctx;
     cudaSetDevice(ctx->device);
     const size_t V = (size_t)lat->buf.g.V;
-    double *de = nullptr, *dq = nullptr;
-    LGF_CUDA_TRY(ctx, cudaMalloc(&de, V * sizeof(double)));
-    cudaError_t e = cudaMalloc(&dq, V * sizeof(double));
     MeasSites mo{};
-    mo.e = de;
-    mo.q = dq;
-    int rc = e == cudaSuccess ? single_measure(lat, mo)
-                              : set_error(ctx, LGF_ENOMEM, "site density buffers: %s", cudaGetErrorString(e));
-    if (rc == LGF_OK && e_site) e = cudaMemcpy(e_site, de, V * sizeof(double), cudaMemcpyDeviceToHost);
-    if (rc == LGF_OK && e == cudaSuccess && q_site) e = cudaMemcpy(q_site, dq, V * sizeof(double), cudaMemcpyDeviceToHost);
-    if (rc == LGF_OK && e != cudaSuccess) rc = set_error(ctx, LGF_ECUDA, "site densities copy: %s", cudaGetErrorString(e));
-    cudaFree(de);
-    cudaFree(dq);
+    mo.e = site_scratch(lat->buf);
+    mo.q = mo.e + V;
+    int rc = single_measure(lat, mo);
+    if (rc == LGF_OK && e_site) rc = copy_out(ctx, e_site, mo.e, V * sizeof(double));
+    if (rc == LGF_OK && q_site) rc = copy_out(ctx, q_site, mo.q, V * sizeof(double));
+    if (rc == LGF_OK && !e_site && !q_site) LGF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     return rc;
 }
 
+// The same pass with the two field strengths' parts swapped (e from the
+// improved F, q from the clover F), summed as a measurement is.
 int lgf_measure_flowed(lgf_lattice* lat, double* E_improved, double* Q_clover) {
     if (!lat) return LGF_EINVAL;
     lgf_ctx* ctx = lat->ctx;
     cudaSetDevice(ctx->device);
-    const size_t V = (size_t)lat->buf.g.V;
-    double *de = nullptr, *dq = nullptr;
-    LGF_CUDA_TRY(ctx, cudaMalloc(&de, V * sizeof(double)));
-    cudaError_t e = cudaMalloc(&dq, V * sizeof(double));
-    MeasSites mo{};
-    mo.e = de;
-    mo.q = dq;
-    mo.swap = 1;  // e with the improved F, q with the clover F
-    int rc = e == cudaSuccess ? single_measure(lat, mo)
-                              : set_error(ctx, LGF_ENOMEM, "density buffers: %s", cudaGetErrorString(e));
-    std::vector<double> he(V), hq(V);
-    if (rc == LGF_OK) e = cudaMemcpy(he.data(), de, V * sizeof(double), cudaMemcpyDeviceToHost);
-    if (rc == LGF_OK && e == cudaSuccess) e = cudaMemcpy(hq.data(), dq, V * sizeof(double), cudaMemcpyDeviceToHost);
-    cudaFree(de);
-    cudaFree(dq);
-    if (rc == LGF_OK && e != cudaSuccess) rc = set_error(ctx, LGF_ECUDA, "density copy: %s", cudaGetErrorString(e));
+    GroupBase* grp = nullptr;
+    int rc = lattice_group(lat, &grp);
     if (rc != LGF_OK) return rc;
-    // fixed-order sums in global site order (ImprovedEnergyDensity.cpp:26, UnImprovedTopologicalCharge.cpp:21)
-    double se = 0.0, sq = 0.0;
-    for (size_t i = 0; i < V; ++i) {
-        se += he[i];
-        sq += hq[i];
-    }
-    const double PI = 3.14159265358979323846;
-    if (E_improved) *E_improved = se * (1.0 / (double)V);
-    if (Q_clover) *Q_clover = sq * (1.0 / (4.0 * PI * PI));
+    LGF_CUDA_TRY(ctx, cudaMemsetAsync(lat->buf.slot, 0, 2 * sizeof(int), ctx->stream));
+    MeasSites mo{};
+    mo.swap = 1;
+    rc = grp->launch_sites(mo);
+    if (rc == LGF_OK) rc = grp->launch_reduce();
+    std::vector<double> h;
+    if (rc == LGF_OK) rc = fetch_meas(ctx, lat->buf, 1, h);
+    if (rc != LGF_OK) return rc;
+    if (E_improved) *E_improved = h[0];
+    if (Q_clover) *Q_clover = h[1];
     return LGF_OK;
 }
 
@@ -1325,7 +1318,8 @@ int lgf_debug_fields(lgf_lattice* lat, double* clover_F, double* improved_F) {
     mo.dbg_improved = di;
     int rc = e == cudaSuccess ? single_measure(lat, mo)
                               : set_error(ctx, LGF_ENOMEM, "debug field buffers: %s", cudaGetErrorString(e));
-    if (rc == LGF_OK && clover_F) e = cudaMemcpy(clover_F, dc, bytes, cudaMemcpyDeviceToHost);
+    if (rc == LGF_OK) e = cudaStreamSynchronize(ctx->stream);
+    if (rc == LGF_OK && e == cudaSuccess && clover_F) e = cudaMemcpy(clover_F, dc, bytes, cudaMemcpyDeviceToHost);
     if (rc == LGF_OK && e == cudaSuccess && improved_F) e = cudaMemcpy(improved_F, di, bytes, cudaMemcpyDeviceToHost);
     if (rc == LGF_OK && e != cudaSuccess) rc = set_error(ctx, LGF_ECUDA, "debug fields copy: %s", cudaGetErrorString(e));
     cudaFree(dc);

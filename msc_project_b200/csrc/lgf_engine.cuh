@@ -176,6 +176,7 @@ public:
     virtual int launch_step() = 0;       // one RK3 step of every member (3 stage launches)
     virtual int launch_measure() = 0;    // measurement of the measured subset
     virtual int launch_sites(const MeasSites& out) = 0;  // the same pass with per-site outputs, no reduction
+    virtual int launch_reduce() = 0;     // the reduction alone
     virtual int launch_one(int k) = 0;   // one kernel alone: stage k+1 (k<3) or the measurement kernel
     virtual int capture() = 0;           // capture step and measurement graphs
     virtual int replay_step() = 0;       // graph launch (captures on first use)
@@ -206,6 +207,7 @@ int upload_links(lgf_ctx* ctx, LatticeBuf& b, const double* host);
 // pageable memory has been copied to the context's pinned chunks on return
 int upload_links_on(lgf_ctx* ctx, LatticeBuf& b, const double* host, cudaStream_t st);
 int download_links(lgf_ctx* ctx, const LatticeBuf& b, double* host);
+int copy_out(lgf_ctx* ctx, void* host, const void* dev, size_t bytes);  // complete on return
 void release_pinned_chunks(lgf_ctx* ctx);
 
 // measurement schedule of FlowSavedGaugeConfigurations for one job
