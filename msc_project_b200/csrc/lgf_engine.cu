@@ -97,55 +97,32 @@ void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape
 }
 
 void buf_free(LatticeBuf& b) {
-    if (b.placed) {  // the memory belongs to the caller (a server's arena)
-        b = LatticeBuf();
-        return;
-    }
-    if (b.U[0]) cudaFree(b.U[0]);  // U[1], U[2] lie in the same allocation
-    if (b.A) cudaFree(b.A);
-    if (b.partial) cudaFree(b.partial);
-    if (b.slice_sums) cudaFree(b.slice_sums);
-    if (b.meas) cudaFree(b.meas);
-    if (b.slot) cudaFree(b.slot);
+    if (b.own_meas) cudaFree(b.meas);
+    if (b.block) cudaFree(b.block);  // null: the memory belongs to the caller (a server's arena, a batch)
     b = LatticeBuf();
 }
 
+// One device allocation per lattice: each cudaMalloc or cudaFree costs ~0.15 ms
+// and may stall behind other work on the device.
 int buf_alloc(lgf_ctx* ctx, LatticeBuf& b, const int shape[4], int precision, int meas_slots) {
-    b = LatticeBuf();
-    b.g = make_geom(shape);
-    b.prec = precision;
-    const size_t Vp = padded_sites((size_t)b.g.V);  // the layout's whole 32-site blocks
-    const size_t rs = real_size(precision);
-    b.nchunk = (b.g.Vs + MEAS_SITES - 1) / MEAS_SITES;
-    cudaError_t e = cudaSuccess;
-    // the link ring as one allocation: U1 (FP64) or U1..U2 (FP32) then spans
-    // at least V*4*18 doubles, the upload/download staging area
-    const size_t ring = Vp * 4 * 18 * rs;
-    e = cudaMalloc(&b.U[0], 3 * ring);
-    if (e == cudaSuccess) {
-        b.U[1] = (char*)b.U[0] + ring;
-        b.U[2] = (char*)b.U[0] + 2 * ring;
-    }
-    if (e == cudaSuccess) e = cudaMalloc(&b.A, Vp * 4 * 8 * rs);
-    if (e == cudaSuccess) e = cudaMalloc(&b.partial, (size_t)b.g.n[0] * b.nchunk * sizeof(double2));
-    if (e == cudaSuccess) e = cudaMalloc(&b.slice_sums, (size_t)b.g.n[0] * sizeof(double2));
-    if (e == cudaSuccess) e = cudaMalloc(&b.slot, 2 * sizeof(int));
-    if (e == cudaSuccess) {
-        b.meas_cap = std::max(meas_slots, 1);
-        e = cudaMalloc(&b.meas, (size_t)b.meas_cap * (2 + 2 * (size_t)b.g.n[0]) * sizeof(double));
-    }
+    void* block = nullptr;
+    const cudaError_t e = cudaMalloc(&block, placed_bytes(shape, precision, meas_slots));
     if (e != cudaSuccess) {
         cudaGetLastError();
-        buf_free(b);
+        b = LatticeBuf();
         return set_error(ctx, LGF_ENOMEM, "device allocation of a %dx%dx%dx%d lattice (%zu bytes) failed: %s",
                          shape[0], shape[1], shape[2], shape[3], footprint_bytes(shape, precision, meas_slots),
                          cudaGetErrorString(e));
     }
+    buf_place(b, shape, precision, meas_slots, block);
+    b.block = block;
     return LGF_OK;
 }
 
-// The same buffers laid out inside one block of caller memory, each part
-// starting on a 256-byte boundary (placed_bytes gives the block's size).
+// A lattice's buffers laid out inside one block of memory, each part starting
+// on a 256-byte boundary (placed_bytes gives the block's size).  The link ring
+// is one run: U1 (FP64) or U1..U2 (FP32) spans at least V*4*18 doubles, the
+// upload/download staging area.
 static inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
 size_t placed_bytes(const int shape[4], int precision, int meas_slots) {
@@ -161,7 +138,6 @@ void buf_place(LatticeBuf& b, const int shape[4], int precision, int meas_slots,
     b = LatticeBuf();
     b.g = make_geom(shape);
     b.prec = precision;
-    b.placed = true;
     const size_t Vp = padded_sites((size_t)b.g.V), rs = real_size(precision);
     b.nchunk = (b.g.Vs + MEAS_SITES - 1) / MEAS_SITES;
     char* p = (char*)mem;
@@ -184,15 +160,16 @@ void buf_place(LatticeBuf& b, const int shape[4], int precision, int meas_slots,
 
 int buf_grow_meas(lgf_ctx* ctx, LatticeBuf& b, int meas_slots) {
     if (meas_slots <= b.meas_cap) return LGF_OK;
-    if (b.placed) return set_error(ctx, LGF_EINVAL, "a placed lattice holds %d measurement slots", b.meas_cap);
+    if (!b.block) return set_error(ctx, LGF_EINVAL, "a placed lattice holds %d measurement slots", b.meas_cap);
     double* m = nullptr;
     cudaError_t e = cudaMalloc(&m, (size_t)meas_slots * (2 + 2 * (size_t)b.g.n[0]) * sizeof(double));
     if (e != cudaSuccess) {
         cudaGetLastError();
         return set_error(ctx, LGF_ENOMEM, "measurement buffer allocation failed: %s", cudaGetErrorString(e));
     }
-    cudaFree(b.meas);
+    if (b.own_meas) cudaFree(b.meas);
     b.meas = m;
+    b.own_meas = true;
     b.meas_cap = meas_slots;
     return LGF_OK;
 }

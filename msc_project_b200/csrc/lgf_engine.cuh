@@ -151,7 +151,8 @@ struct LatticeBuf {
     int* slot = nullptr;
     int nchunk = 0;
     double eps = 0.0;
-    bool placed = false;  // laid out in caller memory (buf_place): buf_free does not free it
+    void* block = nullptr;   // the allocation that holds everything; null: caller memory (buf_place), not freed
+    bool own_meas = false;   // meas has outgrown the block (buf_grow_meas)
 };
 
 int buf_alloc(lgf_ctx* ctx, LatticeBuf& b, const int shape[4], int precision, int meas_slots);
