@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_r
 // buffer (stage S reads U_{S-1}, writes U_S; six fields of 8 reals take two
 // thirds of the third), which costs 384 (FP64: 768) bytes of traffic per site.
 // FP32, bound by instruction issue, gains: one B200, us per step (3 stages),
-// 24^3x48 803 -> 665, 32^4 1251 -> 1023, 48^4 6900 -> 5500, 16^4 89 -> 77,
+// 24^3x48 803 -> 661, 32^4 1251 -> 1012, 48^4 6900 -> 5600, 16^4 89 -> 76,
 // 6x10x14x18 35 -> 31.
 // FP64, where both forms are bound by L2 latency and bandwidth (plaquettes
 // 153 us at 0.49 of the FP64 pipe, update 278 us at 0.45 with DRAM at 5 TB/s,
@@ -504,17 +504,28 @@ __device__ __forceinline__ alg<R> force_at(const cplx<R>* __restrict__ U, const 
     alg<R> f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) f.v[k] = R(0);
-#pragma unroll
-    for (int i = 1; i < 4; ++i) {
-        const int nu = (mu + i) & 3;
-        const int p = mu < nu ? plane_index(mu, nu) : plane_index(nu, mu);
+    const int n1 = (mu + 1) & 3, n2 = (mu + 2) & 3, n3 = (mu + 3) & 3;
+    auto plane = [&](int nu) { return mu < nu ? plane_index(mu, nu) : plane_index(nu, mu); };
+    auto H = [&](int nu, int at) { return get_field<R, true>(plaq_field(K, plane(nu), at)); };
+    const int b1 = bwd(s, dir_of(g, c, n1)), b2 = bwd(s, dir_of(g, c, n2)), b3 = bwd(s, dir_of(g, c, n3));
+    auto add = [&](int nu, const alg<R>& k0, const alg<R>& t) {
         const R sg = mu < nu ? R(1) : R(-1);
-        const int xmn = bwd(s, dir_of(g, c, nu));
-        const alg<R> t = shift(get_field<R, true>(plaq_field(K, p, xmn)), load_link(U, g.V, nu, xmn));
-        const alg<R> k0 = get_field<R, true>(plaq_field(K, p, s));
 #pragma unroll
         for (int k = 0; k < 8; ++k) f.v[k] = fma(sg, k0.v[k] - t.v[k], f.v[k]);
-    }
+    };
+    // the next direction's loads are issued before this one's shift
+    const su3<R> l1 = load_link(U, g.V, n1, b1);
+    const alg<R> h1 = H(n1, b1);
+    const su3<R> l2 = load_link(U, g.V, n2, b2);
+    const alg<R> h2 = H(n2, b2);
+    const alg<R> k1 = H(n1, s);
+    add(n1, k1, shift(h1, l1));
+    const su3<R> l3 = load_link(U, g.V, n3, b3);
+    const alg<R> h3 = H(n3, b3);
+    const alg<R> k2 = H(n2, s);
+    add(n2, k2, shift(h2, l2));
+    const alg<R> k3 = H(n3, s);
+    add(n3, k3, shift(h3, l3));
     alg<R> z;
     z.v[0] = -f.v[0];
     z.v[1] = -f.v[1];
@@ -541,9 +552,10 @@ __global__ void __launch_bounds__(6 * PLAQ_SITES, 4) k_rk3_plaquettes(const LatD
     }
 }
 
-// 24 warps of 80 registers per SM (20 of 95: 24^3x48 2% slower per step, 16 of 115: 6%)
+// 20 warps of 96 registers per SM (24 of 80 with each load beside its shift: 32^4 1030 us
+// per step instead of 1012; 16 of 127: 1037)
 template <typename R, int S>
-__global__ void __launch_bounds__(4 * UPDATE_SITES, 6) k_rk3_update(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
+__global__ void __launch_bounds__(4 * UPDATE_SITES, 5) k_rk3_update(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
                                                                    const int2* __restrict__ seg) {
     const int2 r = *seg;
     const int mu = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -30,12 +30,12 @@
 // stage 2 U2), and per 32-site block U1..U2 hold exactly 18 fields of 8 reals
 // (6 shapes x 3 planes) and A four: F^ of round 0's planes, and the e terms.
 //
-// One B200, whole measurement without the reductions, against one kernel that
-// builds every quadrant's loops at every site: FP64 16^4 0.357 -> 0.217 ms,
-// 24^3x48 3.58 -> 1.80 ms, 48^4 28.8 -> 14.9 ms; FP32-mixed 24^3x48 2.28 ->
-// 1.27 ms, 48^4 18.5 -> 9.9 ms.  24^3x48 FP64 in parts: loops 0.42 + 0.39 ms
-// (FP64 pipe 58-62% busy, then L2 latency), planes 0.50 + 0.45 ms (L2 and
-// DRAM latency: 1.3 KB read per site and plane; FP64 pipe 37-42%).
+// One B200, whole measurement without the reduction, against one kernel that
+// builds every quadrant's loops at every site: FP64 16^4 0.357 -> 0.21 ms,
+// 24^3x48 3.58 -> 1.75 ms, 48^4 28.8 -> 14.3 ms; FP32-mixed 24^3x48 2.28 ->
+// 1.22 ms, 48^4 18.5 -> 9.5 ms.  24^3x48 FP64 in parts: loops 0.43 + 0.41 ms
+// (FP64 pipe 58-62% busy, then L2 latency), planes 0.44 + 0.43 ms (1.3 KB read
+// per site and plane: 0.31 ms with every load in L1, 0.38 without arithmetic).
 #pragma once
 #include "lgf_kernels.cuh"
 
@@ -354,24 +354,36 @@ __global__ void __launch_bounds__(PLANE_MAX_SITES, plane_blocks<R>()) k_meas_pla
             const int s2 = xn >= 2 ? s - 2 * sn : s + (nn - 2) * sn;
             const int s3 = xn >= 3 ? s - 3 * sn : s + (nn - 3) * sn;
             const int f0 = j * LOOP_SHAPES;
-            su3<R> l = load_link(U, g.V, nu, s3);
-            alg<R> a = shift(get_field<R, true>(loop_field(W, f0 + 4, s3)), l);             // (1,3) at x - 3nu
-            l = load_link(U, g.V, nu, s2);
-            a = shift(alg_add(get_field<R, true>(loop_field(W, f0 + 3, s2)), a), l);          // (1,2) at x - 2nu
-            alg<R> b = shift(get_field<R, true>(loop_field(W, f0 + 5, s2)), l);               // (2,2) at x - 2nu
-            l = load_link(U, g.V, nu, s1);
-            a = shift(a, l);
-            F = alg_add(alg_add(get_field<R, true>(loop_field(W, f0 + 3, s)), get_field<R, true>(loop_field(W, f0 + 4, s))), a);
+            auto H = [&](int f, int q) { return get_field<R, true>(loop_field(W, f0 + f, q)); };
+            // each load is issued one or two shifts ahead of its use (loads beside
+            // their shifts: 500 + 459 us on 24^3x48 FP64 instead of 440 + 428)
+            const su3<R> l3 = load_link(U, g.V, nu, s3);
+            alg<R> a = H(4, s3);  // (1,3) at x - 3nu
+            const su3<R> l2 = load_link(U, g.V, nu, s2);
+            const alg<R> h3 = H(3, s2);  // (1,2) at x - 2nu
+            alg<R> b = H(5, s2);  // (2,2) at x - 2nu
+            a = shift(a, l3);
+            const su3<R> l1 = load_link(U, g.V, nu, s1);
+            const alg<R> h30 = H(3, s);
+            const alg<R> h40 = H(4, s);
+            a = shift(alg_add(h3, a), l2);
+            const alg<R> h11 = H(1, s1);  // (2,1) at x - nu
+            b = shift(b, l2);
+            const alg<R> h10 = H(1, s), h50 = H(5, s);
+            a = shift(a, l1);
+            F = alg_add(alg_add(h30, h40), a);
             f1.put(t, F);
-            a = shift(alg_add(get_field<R, true>(loop_field(W, f0 + 1, s1)), b), l);          // (2,1) at x - nu
-            a = alg_add(alg_add(get_field<R, true>(loop_field(W, f0 + 1, s)), get_field<R, true>(loop_field(W, f0 + 5, s))), a);
+            const alg<R> h21 = H(2, s1), h20 = H(2, s);  // (3,1)
+            a = shift(alg_add(h11, b), l1);
+            a = alg_add(alg_add(h10, h50), a);
             f2.put(t, a);
             F = alg_add(F, a);
-            a = alg_add(get_field<R, true>(loop_field(W, f0 + 2, s)), shift(get_field<R, true>(loop_field(W, f0 + 2, s1)), l));
-            f3.put(t, a);                                                                      // (3,1)
+            const alg<R> h01 = H(0, s1), h00 = H(0, s);  // (1,1)
+            a = alg_add(h20, shift(h21, l1));
+            f3.put(t, a);
             F = alg_add(F, a);
-            G = alg_add(get_field<R, true>(loop_field(W, f0, s)), shift(get_field<R, true>(loop_field(W, f0, s1)), l));
-            fg.put(t, G);                                                                      // (1,1)
+            G = alg_add(h00, shift(h01, l1));
+            fg.put(t, G);
         }
         __syncthreads();
         if (in && us.out) {
