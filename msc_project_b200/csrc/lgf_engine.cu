@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -60,8 +61,8 @@ size_t footprint_bytes(const int shape[4], int precision, int meas_slots) {
 // and 48^4), FP32 128.  A lattice too small to fill the SMs evenly with 96-site
 // tiles takes 32-site ones: the SM with the most tiles sets the time, so the
 // smaller tiles are taken where they cut that SM's sites by over a tenth
-// (8^4: 33 -> 23 us per step, 12^4 60 -> 54; 16^4, at 448 against 480 sites,
-// 140 either way).
+// (12^4: 60 -> 54 us per step; 16^4, at 448 against 480 sites, 140 either way;
+// 8^4 takes the split form, which has its own tile).
 int stage_max_threads(int precision) { return precision == LGF_PREC_FP64 ? LGF_STAGE_MAXT_D : LGF_STAGE_MAXT_F; }
 
 TileShape default_shape(int precision, long long volume) {
@@ -239,10 +240,10 @@ public:
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_desc_, sizeof(LatDesc<R>) * max_members_));
         // a lattice takes staple tiles, or plaquette and update tiles
         const long long cap_sites = max_tiles_ * (threads_ / 4);
-        tiles_cap_ = std::max(max_tiles_, sizeof(R) == sizeof(float) ? cap_sites / PLAQ_SITES + cap_sites / UPDATE_SITES + 2 * max_members_ : 0LL);
+        tiles_cap_ = cap_sites / PLAQ_SITES + cap_sites / UPDATE_SITES + 2 * max_members_;  // the plaquette form's are the most
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_tiles_, sizeof(int2) * tiles_cap_));
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_counts_, sizeof(int) * 2));
-        LGF_CUDA_TRY(ctx_, cudaMalloc(&d_seg_, sizeof(int2) * 3 * slots_));
+        LGF_CUDA_TRY(ctx_, cudaMalloc(&d_seg_, sizeof(int2) * 4 * slots_));
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_sel_, sizeof(int) * sel_ints(max_members_)));
         LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_counts_, 0, sizeof(int) * 2, ctx_->stream));
         LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_sel_, 0, sizeof(int) * sel_ints(max_members_), ctx_->stream));
@@ -311,14 +312,14 @@ public:
             append_measure_tiles(mtiles, (int)i, b.g, ls.meas_budget, 4.0 * 18 * sizeof(R));
             seg_len_[i] = (int)mtiles.size() - seg_off_[i];
         }
-        // the stage's launches: a launch per run of whole members with the
-        // staple form, two (plaquettes, update) per run with the plaquette form
+        // the stage's launches, form by form (stage_form): one per run of whole
+        // members, two (plaquettes, update) with the plaquette form
         std::vector<int2> segs;
-        stage_nseg_ = plaq_nseg_ = 0;
-        for (int form = 0; form < 2; ++form) {
+        nseg_ = {0, 0, 0};
+        for (int form = 0; form < 3; ++form) {
             std::vector<int> which, len;
             for (size_t i = 0; i < members.size(); ++i) {
-                if (plaquette_stage<R>(members[i]->g) != (form == 1)) continue;
+                if (stage_form<R>(members[i]->g) != form) continue;
                 which.push_back((int)i);
                 len.push_back((members[i]->g.V + threads_ / 4 - 1) / (threads_ / 4));
             }
@@ -328,16 +329,17 @@ public:
             for (const int2& run : member_runs(len, slots_, 8LL * stage_grid_max_)) {
                 const size_t m0 = m;
                 while (m < which.size() && pos < (long long)run.x + run.y) pos += len[m++];
-                for (int part = 0; part <= form; ++part) {
+                for (int part = 0; part < (form == 1 ? 2 : 1); ++part) {
                     const int first = (int)tiles.size();
                     for (size_t k = m0; k < m; ++k) {
                         const Geom& g = members[which[k]]->g;
                         if (form == 1) append_site_tiles(tiles, which[k], g, part ? UPDATE_SITES : PLAQ_SITES);
+                        else if (form == 2) append_site_tiles(tiles, which[k], g, SPLIT_SITES);
                         else append_staple_tiles(tiles, which[k], g);
                     }
                     segs.push_back(make_int2(first, (int)tiles.size() - first));
                 }
-                ++(form ? plaq_nseg_ : stage_nseg_);
+                ++nseg_[form];
             }
         }
         if ((long long)tiles.size() > tiles_cap_)
@@ -364,8 +366,7 @@ public:
             LGF_CUDA_TRY(ctx_, cudaMalloc(&d_rtiles_, sizeof(int2) * rtiles_cap_));
         }
         ntiles_ = (int)tiles.size();
-        seg_tiles_.clear();
-        for (const int2& q : segs) seg_tiles_.push_back(q.y);
+        seg_tiles_ = segs;
         // one page-locked area carries the descriptors, both tile lists and the segments
         const size_t bd = align16(sizeof(LatDesc<R>) * members.size()), bt = align16(sizeof(int2) * tiles.size()),
                      bm = align16(sizeof(int4) * mtiles.size()), bs = sizeof(int2) * segs.size();
@@ -461,6 +462,8 @@ public:
             }
         }
         meas_small_ = nsmall > 0;
+        small_tiles_ = (int)ts;
+        slice_count_ = (int)tr;
         meas_nseg_ = nsmall < which.size() ? (int)segs.size() : 0;
         {
             std::lock_guard<std::mutex> lk(ctx_->list_mu);
@@ -476,13 +479,13 @@ public:
         return LGF_OK;
     }
 
-    int launch_step() override { return launch_stages(stage_nseg_, plaq_nseg_); }
+    int launch_step() override { return launch_stages(); }
 
     // a single kernel: k = 0..2 stage k+1, k = 3 the measurement kernel alone
     // (every launch segment of it)
     int launch_one(int k) override {
         if (k < 3) {
-            launch_stage(k + 1, stage_nseg_, plaq_nseg_);
+            launch_stage(k + 1);
         } else {
             launch_measure_kernels<false>(meas_nseg_, meas_small_, MeasSites{});
         }
@@ -527,7 +530,7 @@ public:
         LGF_CUDA_TRY(ctx_, cudaGraphLaunch(g, ctx_->stream));
         return LGF_OK;
     }
-    int launches_per_step() const override { return 3 * (stage_nseg_ + 2 * plaq_nseg_); }
+    int launches_per_step() const override { return 3 * (nseg_[0] + 2 * nseg_[1] + nseg_[2]); }
     int launches_per_measure() const override { return (meas_small_ ? 1 : 0) + (meas_nseg_ ? 4 * meas_nseg_ + 1 : 0) + 1; }
     int threads() const override { return threads_; }
     const TileShape& shape() const override { return shape_; }
@@ -572,30 +575,33 @@ private:
             append_stage_tiles(tiles, i, g, threads_ / 4, ls.stage_budget, 4.0 * (2 * 18 + 8) * sizeof(R));
     }
     // a stage launch's grid: persistent, or fewer blocks when its list is shorter
-    int stage_grid(int j, int most) const { return dynamic_ ? most : std::max(1, std::min(seg_tiles_[j], most)); }
-    int step_graph() const { return stage_nseg_ * (slots_ + 1) + plaq_nseg_; }
-    // stage S: n launches of the staple form, then np pairs of the plaquette form
-    template <int S> void launch_stage_of(int n, int np) {
+    int stage_grid(int j, int most) const { return dynamic_ ? most : std::max(1, std::min(seg_tiles_[j].y, most)); }
+    Work stage_work(int j) const { return dynamic_ ? Work{d_seg_ + j, 0, 0} : Work{nullptr, seg_tiles_[j].x, seg_tiles_[j].y}; }
+    int step_graph() const { return (nseg_[0] * (slots_ + 1) + nseg_[1]) * (slots_ + 1) + nseg_[2]; }
+    // stage S: the launches of the staple form, the plaquette form's pairs, the split form's
+    template <int S> void launch_stage_of() {
         int j = 0;
-        for (; j < n; ++j)
-            k_rk3_stage<R, S><<<stage_grid(j, stage_grid_max_), threads_, 0, ctx_->stream>>>(d_desc_, d_tiles_, d_seg_ + j);
+        for (int k = 0; k < nseg_[0]; ++k, ++j)
+            k_rk3_stage<R, S><<<stage_grid(j, stage_grid_max_), threads_, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
         if constexpr (sizeof(R) == sizeof(float))
-            for (; j < n + 2 * np; j += 2) {
-                k_rk3_plaquettes<R, S><<<stage_grid(j, plaq_grid_max_), 6 * PLAQ_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, d_seg_ + j);
-                k_rk3_update<R, S><<<stage_grid(j + 1, update_grid_max_), 4 * UPDATE_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, d_seg_ + j + 1);
+            for (int k = 0; k < nseg_[1]; ++k, j += 2) {
+                k_rk3_plaquettes<R, S><<<stage_grid(j, plaq_grid_max_), 6 * PLAQ_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
+                k_rk3_update<R, S><<<stage_grid(j + 1, update_grid_max_), 4 * UPDATE_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j + 1));
             }
+        for (int k = 0; k < nseg_[2]; ++k, ++j)
+            k_rk3_split<R, S><<<stage_grid(j, ctx_->sm_count), SPLIT_THREADS, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
     }
-    void launch_stage(int S, int n, int np) {
-        if (S == 1) launch_stage_of<1>(n, np);
-        if (S == 2) launch_stage_of<2>(n, np);
-        if (S == 3) launch_stage_of<3>(n, np);
+    void launch_stage(int S) {
+        if (S == 1) launch_stage_of<1>();
+        if (S == 2) launch_stage_of<2>();
+        if (S == 3) launch_stage_of<3>();
     }
-    int launch_stages(int n, int np) {
+    int launch_stages() {
         if (!dynamic_ && ntiles_ == 0) return LGF_OK;
         static const char* names[3] = {"lgf.rk3_stage1", "lgf.rk3_stage2", "lgf.rk3_stage3"};
         for (int S = 1; S <= 3; ++S) {
             NvtxRange r(names[S - 1]);
-            launch_stage(S, n, np);
+            launch_stage(S);
         }
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
@@ -607,7 +613,9 @@ private:
     }
     int launch_reduce() override {
         const int rg = dynamic_ ? ctx_->sm_count : std::max(1, (int)std::min<long long>(rtiles_cap_, 4 * ctx_->sm_count));
-        k_reduce<R><<<rg, RED_THREADS, 0, ctx_->stream>>>(d_desc_, d_rtiles_, d_counts_ + 1);
+        // (the segment table stands for "read it on the device")
+        const Work work = dynamic_ ? Work{d_seg_, 0, 0} : Work{nullptr, 0, slice_count_};
+        k_reduce<R><<<rg, RED_THREADS, 0, ctx_->stream>>>(d_desc_, d_rtiles_, d_counts_ + 1, work);
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
     }
@@ -616,7 +624,7 @@ private:
         const int2* segs = reinterpret_cast<const int2*>(d_sel_ + SEL_HEADER);
         if (small)
             k_measure<R, OUT><<<meas_grid(mtiles_cap_, small_grid_max_), dim3(MEAS_SITES, MEAS_WARPS), measure_smem_bytes<R>(), ctx_->stream>>>(
-                d_desc_, d_mtiles_, segs, out);
+                d_desc_, d_mtiles_, dynamic_ ? Work{segs, 0, 0} : Work{nullptr, 0, small_tiles_}, out);
         if (nseg == 0) return;
         const int2* runs = segs + SEL_SEGS;
         launch_round<0, OUT>(runs, runs + slots_, nseg, out);
@@ -640,7 +648,7 @@ private:
     int capture_one(bool step, int nseg, cudaGraphExec_t* out) {
         cudaGraph_t graph = nullptr;
         LGF_CUDA_TRY(ctx_, cudaStreamBeginCapture(ctx_->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = step ? launch_stages(stage_nseg_, plaq_nseg_) : launch_measurement(nseg, meas_small_);
+        int rc = step ? launch_stages() : launch_measurement(nseg, meas_small_);
         cudaError_t e = cudaStreamEndCapture(ctx_->stream, &graph);
         if (rc != LGF_OK) {
             if (graph) cudaGraphDestroy(graph);
@@ -687,12 +695,14 @@ private:
     int stage_grid_max_ = 1, small_grid_max_ = 1, loops_grid_max_ = 1, planes_grid_max_ = 1;
     int meas_groups_ = LOOP_MAX_GROUPS, unit_sites_ = PLANE_MAX_SITES;  // tiles per loops block, sites per plane unit
     int slots_;                                   // launch slots per kernel (member_runs)
-    int stage_nseg_ = 0, plaq_nseg_ = 0, meas_nseg_ = 1;  // launch segments in use (staple and plaquette form, measurement)
+    std::array<int, 3> nseg_{};                   // stage launch segments in use, by stage form
+    int meas_nseg_ = 1;                           // the measurement's
+    int small_tiles_ = 0, slice_count_ = 0;       // the measured members' small tiles and x0 slices
     bool meas_small_ = false;                      // some measured lattice takes the one-launch kernel
     int2* d_seg_ = nullptr;                        // the stage's launch segments
     long long tiles_cap_ = 0;                      // capacity of d_tiles_
     int plaq_grid_max_ = 1, update_grid_max_ = 1;
-    std::vector<int> seg_tiles_;                   // tiles of each stage launch
+    std::vector<int2> seg_tiles_;                  // tiles of each stage launch (first, count)
     std::map<int, cudaGraphExec_t> step_execs_;    // by launch counts (step_graph)
     std::vector<cudaGraphExec_t> meas_execs_;      // by segment count (and small lattices)
 };

@@ -47,34 +47,38 @@ namespace lgf {
 // Z = -1/2 [ (W - W^dag) - 1/3 Tr(W - W^dag) ],  W = U_mu(x) A,
 // A = sum_{nu != mu} U_nu(x+mu) (U_nu(x) U_mu(x+nu))^dag
 //                  + (U_mu(x-nu) U_nu(x-nu+mu))^dag U_nu(x-nu)
+// S += the two staples of link (s, mu) in the plane of nu; xpm = s + mu, xn = the nu coordinate of s
+template <typename R>
+__device__ __forceinline__ void add_staples(su3<R>& S, const cplx<R>* __restrict__ U, const Geom& g, int s, int mu, const Dir& dm,
+                                            int xpm, int nu, int xn) {
+    const int V = g.V;
+    const int xpn = fwd(g, s, nu, xn), xmn = bwd(g, s, nu, xn);
+    const int xmnpm = fwd(xmn, dm);  // the mu coordinate of x-nu is x_mu
+    {
+        su3<R> a2 = load_link(U, V, nu, s);
+        su3<R> a3 = load_link(U, V, mu, xpn);
+        su3<R> t = mul_nn_su3(a2, a3);
+        su3<R> a1 = load_link(U, V, nu, xpm);
+        acc_na(S, a1, t);
+    }
+    {
+        su3<R> b1 = load_link(U, V, mu, xmn);
+        su3<R> b2 = load_link(U, V, nu, xmnpm);
+        su3<R> t = mul_nn_su3(b1, b2);
+        su3<R> b3 = load_link(U, V, nu, xmn);
+        acc_an(S, t, b3);
+    }
+}
+
 template <typename R>
 __device__ __forceinline__ su3<R> staple_sum(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c, int mu) {
-    const int V = g.V;
     const Dir dm = dir_of(g, c, mu);
     su3<R> S;
     su3_zero(S);
     const int xpm = fwd(s, dm);
 #pragma unroll
-    for (int nu = 0; nu < 4; ++nu) {
-        if (nu == mu) continue;
-        const int xpn = fwd(g, s, nu, c.x[nu]);
-        const int xmn = bwd(g, s, nu, c.x[nu]);
-        const int xmnpm = fwd(xmn, dm);  // the mu coordinate of x-nu is x_mu
-        {
-            su3<R> a2 = load_link(U, V, nu, s);
-            su3<R> a3 = load_link(U, V, mu, xpn);
-            su3<R> t = mul_nn_su3(a2, a3);
-            su3<R> a1 = load_link(U, V, nu, xpm);
-            acc_na(S, a1, t);
-        }
-        {
-            su3<R> b1 = load_link(U, V, mu, xmn);
-            su3<R> b2 = load_link(U, V, nu, xmnpm);
-            su3<R> t = mul_nn_su3(b1, b2);
-            su3<R> b3 = load_link(U, V, nu, xmn);
-            acc_an(S, t, b3);
-        }
-    }
+    for (int nu = 0; nu < 4; ++nu)
+        if (nu != mu) add_staples(S, U, g, s, mu, dm, xpm, nu, c.x[nu]);
     return S;
 }
 
@@ -391,6 +395,17 @@ template <typename R> __device__ __forceinline__ alg<R> alg_add(const alg<R>& x,
     return z;
 }
 
+// The tiles of one launch: seg->x .. + seg->y of the list, read on the device so
+// that a captured graph follows the list; or, for a group that never changes
+// (seg null), the range and its only member by value, which takes two of the
+// four dependent loads (range, tile, descriptor, links) that open every kernel
+// out of its latency: 1 to 1.5 us of an 8^4 step's three launches.
+struct Work { const int2* seg; int first, count; };
+__device__ __forceinline__ int2 work_range(const Work& w) { return w.seg ? *w.seg : make_int2(w.first, w.count); }
+template <typename R> __device__ __forceinline__ const LatDesc<R>* work_member(const Work& w, const LatDesc<R>* descs, int member) {
+    return w.seg ? descs + member : descs;
+}
+
 // ------------------------------------------------------------------ stage
 // One RK3 stage (low-storage form of the reference's integrator):
 //   S=1:  A = Z0;                    U1 = exp(eps/4 Z0) U0
@@ -425,7 +440,7 @@ __device__ __forceinline__ void update_link(R* A, cplx<R>* Uout, double eps, int
     store_link(Uout, V, mu, s, exp_times(X, u));
 }
 
-// Staple form: FP64, and small FP32 lattices (plaquette_stage).
+// Staple form: FP64, and FP32 lattices below plaquette_stage's line.
 // Persistent: blocks stride over one segment of the tile list (seg = first
 // tile, count); tile = (lattice, first site).
 // A tile of T threads (T a multiple of 128) covers T/4 consecutive sites with
@@ -437,11 +452,11 @@ template <> struct StageMaxThreads<double> { static constexpr int value = LGF_ST
 
 template <typename R, int S>
 __global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_rk3_stage(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
-                                                   const int2* __restrict__ seg) {
-    const int2 r = *seg;  // this launch's tiles: tiles[r.x, r.x + r.y)
+                                                   Work work) {
+    const int2 r = work_range(work);  // this launch's tiles: tiles[r.x, r.x + r.y)
     for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
         const int2 tile = tiles[ti];
-        const LatDesc<R>* d = descs + tile.x;
+        const LatDesc<R>* d = work_member(work, descs, tile.x);
         const Geom g = d->g;
         const int mu = (threadIdx.x >> 5) & 3;
         const int s = tile.y + ((threadIdx.x >> 7) << 5) + (threadIdx.x & 31);
@@ -454,6 +469,59 @@ __global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_r
         su3<R> u;
         const alg<R> Z = flow_gradient<R>(Uin, g, s, c, mu, u);
         update_link<R, S>(A, Uout, eps, g.V, s, mu, Z, u);
+    }
+}
+
+// Split form: lattices of up to one 32-site tile per SM.  With one warp per
+// direction and tile an SM's schedulers hold a warp each, and a stage is the
+// latency of one thread's six staples; here three warps take two staples each
+// and the first adds their sums (in a fixed order) and updates the link.
+// 8^4 FP64 22.6 -> 20 us per step (19 with the range by value, Work), FP32
+// 18.5 -> 17.5 (16.5).  Above the line an SM with two tiles would run them in
+// turn, and the staple form runs them side by side.
+constexpr int SPLIT_SITES = 32, SPLIT_THREADS = 12 * SPLIT_SITES;
+constexpr long long SPLIT_MAX_SITES = 148 * SPLIT_SITES;
+template <typename R, int S>
+__global__ void __launch_bounds__(SPLIT_THREADS, 1) k_rk3_split(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
+                                                               Work work) {
+    __shared__ typename vec2_of<R>::type part_sum[2][9][4 * SPLIT_SITES];
+    const int2 r = work_range(work);
+    const int lane = threadIdx.x & 31, mu = (threadIdx.x >> 5) & 3, part = threadIdx.x >> 7, column = threadIdx.x & 127;
+    for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
+        const int2 tile = tiles[ti];
+        const LatDesc<R>* d = work_member(work, descs, tile.x);
+        const Geom g = d->g;
+        const int s = tile.y + lane;
+        const bool in = s < g.V;
+        const cplx<R>* Uin = stage_in<R, S>(d);
+        su3<R> sum;
+        su3_zero(sum);
+        if (in) {
+            const Coord c = site_coord(g, s);
+            const Dir dm = dir_of(g, c, mu);
+            const int nu = part + (part >= mu ? 1 : 0);
+            add_staples(sum, Uin, g, s, mu, dm, fwd(s, dm), nu, sel4(nu, c.x[0], c.x[1], c.x[2], c.x[3]));
+            if (part > 0) {
+#pragma unroll
+                for (int k = 0; k < 9; ++k) {
+                    typename vec2_of<R>::type v;
+                    v.x = sum.m[k].re;
+                    v.y = sum.m[k].im;
+                    part_sum[part - 1][k][column] = v;
+                }
+            }
+        }
+        __syncthreads();
+        if (in && part == 0) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const typename vec2_of<R>::type v = part_sum[0][k][column], w = part_sum[1][k][column];
+                sum.m[k] = cmk<R>((sum.m[k].re + v.x) + w.x, (sum.m[k].im + v.y) + w.y);
+            }
+            const su3<R> u = load_link(Uin, g.V, mu, s);
+            update_link<R, S>(d->A, stage_out<R, S>(d), d->eps, g.V, s, mu, ta_of_product(u, sum, R(-0.5)), u);
+        }
+        __syncthreads();
     }
 }
 
@@ -540,12 +608,12 @@ __device__ __forceinline__ alg<R> force_at(const cplx<R>* __restrict__ U, const 
 // 24 warps of 80 registers per SM (30 of 64 registers: 16^4 5% slower)
 template <typename R, int S>
 __global__ void __launch_bounds__(6 * PLAQ_SITES, 4) k_rk3_plaquettes(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
-                                                                     const int2* __restrict__ seg) {
-    const int2 r = *seg;  // this launch's tiles: tiles[r.x, r.x + r.y)
+                                                                     Work work) {
+    const int2 r = work_range(work);  // this launch's tiles: tiles[r.x, r.x + r.y)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
         const int2 tile = tiles[ti];
-        const LatDesc<R>* d = descs + tile.x;
+        const LatDesc<R>* d = work_member(work, descs, tile.x);
         const Geom g = d->g;
         const int s = tile.y + (w / 6) * 32 + lane;
         if (s < g.V) plaquette_at<R>(stage_in<R, S>(d), stage_free<R, S>(d), g, s, site_coord(g, s), w % 6);
@@ -556,12 +624,12 @@ __global__ void __launch_bounds__(6 * PLAQ_SITES, 4) k_rk3_plaquettes(const LatD
 // per step instead of 1012; 16 of 127: 1037)
 template <typename R, int S>
 __global__ void __launch_bounds__(4 * UPDATE_SITES, 5) k_rk3_update(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
-                                                                   const int2* __restrict__ seg) {
-    const int2 r = *seg;
+                                                                   Work work) {
+    const int2 r = work_range(work);
     const int mu = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
         const int2 tile = tiles[ti];
-        const LatDesc<R>* d = descs + tile.x;
+        const LatDesc<R>* d = work_member(work, descs, tile.x);
         const Geom g = d->g;
         const int s = tile.y + lane;
         if (s >= g.V) continue;
@@ -579,6 +647,10 @@ __global__ void __launch_bounds__(4 * UPDATE_SITES, 5) k_rk3_update(const LatDes
 constexpr int PLAQ_MIN_SITES = 8192;
 template <typename R> __host__ __device__ __forceinline__ bool plaquette_stage(const Geom& g) {
     return sizeof(R) == sizeof(float) && g.V >= PLAQ_MIN_SITES;
+}
+// 0: staple form, 1: plaquette form, 2: split form
+template <typename R> __host__ __device__ __forceinline__ int stage_form(const Geom& g) {
+    return g.V <= SPLIT_MAX_SITES ? 2 : (plaquette_stage<R>(g) ? 1 : 0);
 }
 
 template <typename R> __device__ __forceinline__ void store_alg_as_antiherm(double2* dst, const alg<R>& z) {
@@ -927,13 +999,13 @@ __device__ __forceinline__ void measure_tile(MeasSmem<R>* sm, const cplx<R>* __r
 template <typename R, bool OUT>
 __global__ void __launch_bounds__(MEAS_SITES * MEAS_WARPS, 1) k_measure(const LatDesc<R>* __restrict__ descs,
                                                                        const int4* __restrict__ mtiles,
-                                                                       const int2* __restrict__ seg, MeasSites out) {
+                                                                       Work work, MeasSites out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MeasSmem<R>* sm = reinterpret_cast<MeasSmem<R>*>(smem_raw);
-    const int2 r = *seg;  // this launch's tiles: mtiles[r.x, r.x + r.y)
+    const int2 r = work_range(work);  // this launch's tiles: mtiles[r.x, r.x + r.y)
     for (int ti = r.x + blockIdx.x; ti < r.x + r.y; ti += gridDim.x) {
         const int4 tile = mtiles[ti];
-        const LatDesc<R>* d = descs + tile.x;
+        const LatDesc<R>* d = work_member(work, descs, tile.x);
         const Geom g = d->g;
         measure_tile<R, OUT, false>(sm, d->U0, g, tile.y, tile.z, d->partial, d->nchunk, out);
         __syncthreads();
@@ -969,14 +1041,14 @@ __device__ __forceinline__ double2 block_sum(double e, double q, double* se, dou
 
 template <typename R>
 __global__ void __launch_bounds__(RED_THREADS) k_reduce(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ rtiles,
-                                                        const int* __restrict__ nrtiles) {
+                                                        const int* __restrict__ nrtiles, Work work) {
     __shared__ double se[RED_THREADS], sq[RED_THREADS];
     __shared__ bool last;
     const double inv4pi2 = 1.0 / (4.0 * 3.14159265358979323846 * 3.14159265358979323846);
-    const int n = *nrtiles;
+    const int n = work.seg ? *nrtiles : work.count;
     for (int ti = blockIdx.x; ti < n; ti += gridDim.x) {
         const int2 tile = rtiles[ti];
-        const LatDesc<R>* d = descs + tile.x;
+        const LatDesc<R>* d = work_member(work, descs, tile.x);
         const int t = tile.y, N0 = d->g.n[0], nchunk = d->nchunk;
         double e = 0.0, q = 0.0;
         for (int j = threadIdx.x; j < nchunk; j += RED_THREADS) {

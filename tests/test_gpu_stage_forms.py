@@ -1,5 +1,5 @@
-"""The FP32 stage's plaquette form (lattices of 8192 sites and more) and its
-staple form below, at tile edges: slices and volumes that are no multiple of
+"""The stage's forms -- split (lattices of up to 148 tiles of 32 sites), FP32
+plaquettes (8192 sites and more), staples -- at tile edges: slices and volumes that are no multiple of
 32 sites, extents of 4 (every neighbour wraps), volumes on both sides of the
 rule's line.
 
@@ -15,7 +15,7 @@ from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(4, 4, 4, 6), (8, 8, 8, 14), (8, 8, 8, 16), (4, 4, 4, 130), (10, 14, 10, 6), (6, 10, 14, 18), (4, 50, 6, 10)]
+SHAPES = [(4, 4, 4, 6), (4, 6, 8, 10), (8, 8, 8, 8), (4, 4, 4, 74), (4, 4, 4, 76), (8, 8, 8, 14), (8, 8, 8, 16), (4, 4, 4, 130), (10, 14, 10, 6), (6, 10, 14, 18), (4, 50, 6, 10)]
 
 
 @pytest.mark.parametrize("shape", SHAPES)
@@ -37,6 +37,18 @@ def test_fp32_force_matches_fp64(ctx, shape):
     assert np.max(np.abs(got - want)) < 1.5e-5
     # three exponentials of eps times such a force, three products: 9 * 2^-24 * ~8 roundings
     assert np.max(np.abs(step - step64)) < 5e-6
+
+
+@pytest.mark.parametrize("shape", [(4, 4, 4, 4), (4, 6, 8, 10), (8, 8, 8, 8), (4, 4, 4, 74), (4, 4, 4, 76)])
+def test_fp64_small_lattices_match_the_oracle(ctx, shape):
+    U = O.generate_G(shape, 23, 0.5)
+    want = U
+    for _ in range(2):
+        want = O.rk3_step(want, shape, 0.01)
+    with ctx.lattice(shape, FP64) as lat:
+        lat.upload(U)
+        lat.flow(0.01, 2, 0, measure_at_t0=False)
+        assert np.max(np.abs(lat.download() - np.asarray(want).reshape(-1))) < 1e-13  # six stages of ~30 roundings
 
 
 def test_fp32_results_do_not_depend_on_the_batch(ctx):
