@@ -190,8 +190,9 @@ template <bool FILE, typename R> __device__ __forceinline__ su3<R> load_link_fro
         return load_link(U, V, mu, s);
     }
 }
-// Links are read in R and multiplied in D; FILE: U is in file order instead of
-// the device layout.
+// Links are read in R and multiplied in D; FILE: U is the caller's own array in
+// file order instead of the device layout, and products are formed in full: the
+// result is that of the matrices as given, also where they are not quite SU(3).
 template <typename R, typename D = R, bool FILE = false> struct Plane {
     const cplx<R>* __restrict__ U;
     int V, mu, nu;
@@ -241,12 +242,12 @@ template <typename R, typename D = R, bool FILE = false> struct Plane {
             const su3<D> l = su3_cast<D>(load_link_from<FILE>(U, V, dir, p.s));
             p.s = (xc == d.n - 1) ? p.s - (d.n - 1) * d.stride : p.s + d.stride;
             xc = wrap_inc(xc, d.n);
-            P = mul_nn_su3(P, l);
+            P = FILE ? mul_nn(P, l) : mul_nn_su3(P, l);
         } else {
             p.s = (xc == 0) ? p.s + (d.n - 1) * d.stride : p.s - d.stride;
             xc = wrap_dec(xc, d.n);
             const su3<D> l = su3_cast<D>(load_link_from<FILE>(U, V, dir, p.s));
-            P = mul_na_su3(P, l);
+            P = FILE ? mul_na(P, l) : mul_na_su3(P, l);
         }
     }
 };
@@ -720,11 +721,11 @@ template <typename R> constexpr bool meas_smem_acc() { return LGF_MEAS_SMEM_ACC 
 // extension rebuilds the third (mul_nn_su3 / mul_na_su3 read rows 0 and 1 of
 // their left operand), so a parked path is exactly the one put there.
 constexpr int MEAS_STASH_ENTRIES = 6;
-template <typename R> struct PathStash {
+template <typename R, int ENTRIES = MEAS_STASH_ENTRIES> struct PathStash {
     typename vec2_of<R>::type* p;  // entry k at p[k * MEAS_ACC_STRIDE]
     __device__ __forceinline__ void put(const su3<R>& P) const {
 #pragma unroll
-        for (int k = 0; k < MEAS_STASH_ENTRIES; ++k) {
+        for (int k = 0; k < ENTRIES; ++k) {
             p[k * MEAS_ACC_STRIDE].x = P.m[k].re;
             p[k * MEAS_ACC_STRIDE].y = P.m[k].im;
         }
@@ -733,7 +734,7 @@ template <typename R> struct PathStash {
         su3<R> P;
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
-            if (k < MEAS_STASH_ENTRIES) {
+            if (k < ENTRIES) {
                 const typename vec2_of<R>::type v = p[k * MEAS_ACC_STRIDE];
                 P.m[k] = cmk<R>(v.x, v.y);
             } else {
@@ -746,17 +747,19 @@ template <typename R> struct PathStash {
 
 // Shared memory of one measurement block: the straight lines of length 2 and
 // 3 from each of its 32 sites in the 8 signed directions (every plane and
-// quadrant of the site reuses them), then the per-plane results.
-template <typename R> struct MeasSmem {
+// quadrant of the site reuses them), then the per-plane results.  With FILE
+// the paths keep all nine entries, and there is room for one parked path.
+template <typename R, bool FILE = false> struct MeasSmem {
+    static constexpr int ENTRIES = FILE ? 9 : MEAS_STASH_ENTRIES, PARKED = FILE ? 1 : 2;
     union {
-        R line[8][2][2 * MEAS_STASH_ENTRIES][MEAS_SITES];  // [2*dir + (sign<0)][length-2][real of entry][site]
+        R line[8][2][2 * ENTRIES][MEAS_SITES];  // [2*dir + (sign<0)][length-2][real of entry][site]
         struct {                       // after the lines are dead: the second quadrant half's sums
             alg<R> G[6][MEAS_SITES];
             alg<R> Fh[6][MEAS_SITES];
         } part;
     };
     R acc[meas_smem_acc<R>() ? 16 : 1][meas_smem_acc<R>() ? MEAS_ACC_STRIDE : 1];  // G, Fhat columns (LGF_MEAS_SMEM_ACC)
-    typename vec2_of<R>::type stash[2][MEAS_STASH_ENTRIES][MEAS_ACC_STRIDE];  // two paths per thread (PathStash)
+    typename vec2_of<R>::type stash[PARKED][ENTRIES][MEAS_ACC_STRIDE];  // parked paths per thread (PathStash)
     alg<R> F[6][MEAS_SITES];          // improved F per plane
     double E[6][MEAS_SITES];
 };
@@ -776,20 +779,20 @@ struct MeasSites {
 
 // A line is only ever extended (the left operand of a product that rebuilds
 // the third row), so like a parked path it keeps its first two rows.
-template <typename R>
-__device__ __forceinline__ void store_line(MeasSmem<R>* sm, int sdir, int len, int lane, const su3<R>& L) {
+template <typename R, bool FILE>
+__device__ __forceinline__ void store_line(MeasSmem<R, FILE>* sm, int sdir, int len, int lane, const su3<R>& L) {
 #pragma unroll
-    for (int k = 0; k < MEAS_STASH_ENTRIES; ++k) {
+    for (int k = 0; k < MeasSmem<R, FILE>::ENTRIES; ++k) {
         sm->line[sdir][len - 2][2 * k][lane] = L.m[k].re;
         sm->line[sdir][len - 2][2 * k + 1][lane] = L.m[k].im;
     }
 }
-template <typename R>
-__device__ __forceinline__ su3<R> load_line(const MeasSmem<R>* sm, int sdir, int len, int lane) {
+template <typename R, bool FILE>
+__device__ __forceinline__ su3<R> load_line(const MeasSmem<R, FILE>* sm, int sdir, int len, int lane) {
     su3<R> L;
 #pragma unroll
     for (int k = 0; k < 9; ++k)
-        L.m[k] = k < MEAS_STASH_ENTRIES
+        L.m[k] = k < MeasSmem<R, FILE>::ENTRIES
                      ? cmk<R>(sm->line[sdir][len - 2][2 * k][lane], sm->line[sdir][len - 2][2 * k + 1][lane])
                      : cmk<R>(R(0), R(0));  // never read: the next product rebuilds the row
     return L;
@@ -808,11 +811,13 @@ __device__ __forceinline__ su3<R> load_line(const MeasSmem<R>* sm, int sdir, int
 // 12 matrix products and 14 global link loads per quadrant; the paths that
 // are extended after other work are parked in the thread's shared-memory
 // column (PathStash: Pm(1,1), Pm(2,1), Pn(1,2)), and the leaves are added in
-// the order (1,1) | (2,1), (3,1), (1,2), (1,3), (2,2).
+// the order (1,1) | (2,1), (3,1), (1,2), (1,3), (2,2).  With FILE, Pm(2,1) is
+// formed again instead (one product and one load more).
 template <typename R, bool FILE, typename Acc>
 __device__ __forceinline__ void plane_fields_body(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c,
-                                                  int mu, int nu, const MeasSmem<R>* sm, int lane, int qa, int qb,
-                                                  Acc G, Acc Fhat, PathStash<R> sa, PathStash<R> sb) {
+                                                  int mu, int nu, const MeasSmem<R, FILE>* sm, int lane, int qa, int qb,
+                                                  Acc G, Acc Fhat, PathStash<R, MeasSmem<R, FILE>::ENTRIES> sa,
+                                                  PathStash<R, MeasSmem<R, FILE>::ENTRIES> sb) {
     Plane<R, R, FILE> P;
     P.U = U;
     P.V = g.V;
@@ -849,7 +854,7 @@ __device__ __forceinline__ void plane_fields_body(const cplx<R>* __restrict__ U,
         Pm = load_line(sm, sdm, 2, lane);
         P.ext(Pm, p21, false, sn);  // Pm(2,1), p21 at x + 2m + n
         leaf_acc(Pn, Pm, sg * k12, Fhat);
-        sb.put(Pm);
+        if (!FILE) sb.put(Pm);
         // (3,1)
         P.ext(Pn, pn, true, sm_);  // Pn(3,1)
         PlanePos p31 = x0;
@@ -876,7 +881,14 @@ __device__ __forceinline__ void plane_fields_body(const cplx<R>* __restrict__ U,
         // (2,2)
         Pn = sa.get();
         P.ext(Pn, p12, true, sm_);  // Pn(2,2)
-        Pm = sb.get();
+        if (FILE) {
+            p21 = x0;
+            P.advance(p21, true, sm_, 2);
+            Pm = load_line(sm, sdm, 2, lane);
+            P.ext(Pm, p21, false, sn);  // Pm(2,1)
+        } else {
+            Pm = sb.get();
+        }
         P.ext(Pm, p21, false, sn);  // Pm(2,2)
         leaf_acc(Pn, Pm, sg * k22, Fhat);
     }
@@ -884,10 +896,11 @@ __device__ __forceinline__ void plane_fields_body(const cplx<R>* __restrict__ U,
 
 template <typename R, bool FILE>
 __device__ __forceinline__ void plane_fields_smem(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c,
-                                                  int mu, int nu, MeasSmem<R>* sm, int lane, int qa, int qb,
+                                                  int mu, int nu, MeasSmem<R, FILE>* sm, int lane, int qa, int qb,
                                                   alg<R>& Greg, alg<R>& Fhreg) {
     const int column = threadIdx.y * MEAS_SITES + lane;
-    const PathStash<R> sa{&sm->stash[0][0][column]}, sb{&sm->stash[1][0][column]};
+    const PathStash<R, MeasSmem<R, FILE>::ENTRIES> sa{&sm->stash[0][0][column]},
+        sb{&sm->stash[MeasSmem<R, FILE>::PARKED - 1][0][column]};  // (unused with FILE)
     if constexpr (meas_smem_acc<R>()) {
         R* col = &sm->acc[0][column];
         const SmemAcc<R> G{col}, Fhat{col + 8 * MEAS_ACC_STRIDE};
@@ -916,7 +929,7 @@ __device__ __forceinline__ void plane_fields_smem(const cplx<R>* __restrict__ U,
 //                                             (TopologicalCharge.cpp:11-16)
 constexpr int MEAS_WARPS = 12;
 template <typename R, bool OUT, bool FILE>
-__device__ __forceinline__ void measure_tile(MeasSmem<R>* sm, const cplx<R>* __restrict__ U, const Geom& g, int slice, int chunk,
+__device__ __forceinline__ void measure_tile(MeasSmem<R, FILE>* sm, const cplx<R>* __restrict__ U, const Geom& g, int slice, int chunk,
                                              double2* __restrict__ partial, int nchunk, const MeasSites& out) {
     const int lane = threadIdx.x, w = threadIdx.y, p = w % 6, part = w / 6;
     const int off = meas_site_offset(g, meas_patched(g), chunk, lane);
@@ -1014,7 +1027,7 @@ __global__ void __launch_bounds__(MEAS_SITES * MEAS_WARPS, 1) k_measure(const La
 
 // Dynamic shared memory of k_measure<R> (above 48 KB: raised with the kernel's
 // attribute before the first launch).
-template <typename R> inline size_t measure_smem_bytes() { return sizeof(MeasSmem<R>); }
+template <typename R, bool FILE = false> inline size_t measure_smem_bytes() { return sizeof(MeasSmem<R, FILE>); }
 
 constexpr int RED_THREADS = 256;
 

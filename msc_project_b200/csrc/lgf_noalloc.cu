@@ -45,15 +45,19 @@ double2* g_noalloc_addr[NOALLOC_MAX_DEVICES] = {};
 // Grid (nchunk, N0), one 32-site tile per block: the one-launch measurement
 // (measure_tile) reading the caller's file-order links in place.  The fixed
 // scratch has no room for the loops' projections that lgf_measure.cuh shares
-// between sites.  Bound by link loads (load_link_from<true>): 14 per plane and
-// quadrant with shared paths instead of 40 for separate loops.  One B200, all
-// launches on 32x16^3: 2.81 ms with separate loops, 1.40 with shared paths and
-// a 16-byte load per lane, 1.20 with links read by lane pairs (1.24 by fours:
-// the selects cost more than the lines they save).
+// between sites.  Bound by link loads (load_link_from<true>): 15 per plane and
+// quadrant with shared paths instead of 40 for separate loops.  Products keep
+// all three rows of the caller's matrices (the loops' error against extended
+// precision is the separate loops', 1e-15 of a flowed charge profile; with the
+// third row rebuilt it was 8e-15, and links 1e-7 off SU(3) moved E and Q by as
+// much).  One B200, all launches on 32x16^3: 2.81 ms with separate loops, 1.33
+// so (two-row products 1.20; with those, a 16-byte load per lane instead of
+// lane pairs 1.40, links read by fours 1.24: the selects cost more than the
+// lines they save).
 __global__ void __launch_bounds__(MEAS_SITES * MEAS_WARPS, 1) k_noalloc_measure(const cplx<double>* __restrict__ L, Geom g,
                                                                                double2* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    measure_tile<double, false, true>(reinterpret_cast<MeasSmem<double>*>(smem_raw), L, g, blockIdx.y, blockIdx.x, partials,
+    measure_tile<double, false, true>(reinterpret_cast<MeasSmem<double, true>*>(smem_raw), L, g, blockIdx.y, blockIdx.x, partials,
                                       gridDim.x, MeasSites{});
 }
 
@@ -122,7 +126,7 @@ int noalloc_scratch(int dev, double2** out) {
             if (e != cudaSuccess) cudaGetLastError();  // this lookup's own error
             return LGF_ECUDA;
         }
-        e = cudaFuncSetAttribute(k_noalloc_measure, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)measure_smem_bytes<double>());
+        e = cudaFuncSetAttribute(k_noalloc_measure, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)measure_smem_bytes<double, true>());
         if (e != cudaSuccess) {
             cudaGetLastError();
             return LGF_ECUDA;
@@ -164,7 +168,7 @@ extern "C" int lgf_measure_noalloc(const double* links, const int shape[4], doub
     double2* partials = scratch;
     double2* slice_sums = scratch + NOALLOC_MAX_PARTIALS;
     cudaStream_t st = (cudaStream_t)stream;
-    k_noalloc_measure<<<dim3(nchunk, g.n[0]), dim3(MEAS_SITES, MEAS_WARPS), measure_smem_bytes<double>(), st>>>(
+    k_noalloc_measure<<<dim3(nchunk, g.n[0]), dim3(MEAS_SITES, MEAS_WARPS), measure_smem_bytes<double, true>(), st>>>(
         (const cplx<double>*)links, g, partials);
     k_noalloc_slices<<<g.n[0], RED_THREADS, 0, st>>>(partials, nchunk, g, slice_sums, out);
     k_noalloc_total<<<1, RED_THREADS, 0, st>>>(slice_sums, g, out);

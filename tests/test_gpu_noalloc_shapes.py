@@ -32,3 +32,19 @@ def test_noalloc_matches_measure(ctx, shape):
     assert rel_err(got[0], E) < 1e-12 and q_err(got[1], Q) < 1e-12
     assert rel_err(got[2:2 + shape[0]], es) < 1e-12
     assert np.max(np.abs(got[2 + shape[0]:] - qs)) < 1e-12
+
+
+def test_noalloc_reads_the_links_as_given(ctx):
+    """Links 1e-6 off SU(3): the result is that of the given matrices (full products), to rounding."""
+    import torch
+    shape = (4, 6, 4, 6)
+    rng = np.random.default_rng(17)
+    U = np.ascontiguousarray(O.generate_G(shape, 17, 0.5)).reshape(-1)
+    U = U + 1e-6 * rng.standard_normal(U.size)
+    dev = torch.from_numpy(U).to("cuda:0")
+    out = torch.empty(2 + 2 * shape[0], dtype=torch.float64, device="cuda:0")
+    ptr = lambda t: ctypes.cast(t.data_ptr(), ctypes.POINTER(ctypes.c_double))  # noqa: E731
+    assert ctx.lib.lgf_measure_noalloc(ptr(dev), (ctypes.c_int * 4)(*shape), ptr(out),
+                                       ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == C.LGF_OK
+    got = out.cpu().numpy()
+    assert rel_err(got[0], O.energy_density(U, shape)) < 1e-12 and q_err(got[1], O.topological_charge(U, shape)) < 1e-12
