@@ -250,12 +250,10 @@ public:
         int nb = 0;
         LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_stage<R, 1>, threads_, 0));
         stage_grid_max_ = std::max(1, nb) * ctx_->sm_count;
-        if constexpr (sizeof(R) == sizeof(float)) {
-            LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_plaquettes<R, 1>, 6 * PLAQ_SITES, 0));
-            plaq_grid_max_ = std::max(1, nb) * ctx_->sm_count;
-            LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_update<R, 1>, 4 * UPDATE_SITES, 0));
-            update_grid_max_ = std::max(1, nb) * ctx_->sm_count;
-        }
+        LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_plaquettes<R, 1>, 6 * PLAQ_SITES, 0));
+        plaq_grid_max_ = std::max(1, nb) * ctx_->sm_count;
+        LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_update<R, 1>, 4 * UPDATE_SITES, 0));
+        update_grid_max_ = std::max(1, nb) * ctx_->sm_count;
         // Measurement blocks: 4 tiles (loops) and 384 sites (planes) per block,
         // halved for one-warp-per-plane shapes, and smaller for lattices that
         // would not give every SM a block.
@@ -583,11 +581,10 @@ private:
         int j = 0;
         for (int k = 0; k < nseg_[0]; ++k, ++j)
             k_rk3_stage<R, S><<<stage_grid(j, stage_grid_max_), threads_, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
-        if constexpr (sizeof(R) == sizeof(float))
-            for (int k = 0; k < nseg_[1]; ++k, j += 2) {
-                k_rk3_plaquettes<R, S><<<stage_grid(j, plaq_grid_max_), 6 * PLAQ_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
-                k_rk3_update<R, S><<<stage_grid(j + 1, update_grid_max_), 4 * UPDATE_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j + 1));
-            }
+        for (int k = 0; k < nseg_[1]; ++k, j += 2) {
+            k_rk3_plaquettes<R, S><<<stage_grid(j, plaq_grid_max_), 6 * PLAQ_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
+            k_rk3_update<R, S><<<stage_grid(j + 1, update_grid_max_), 4 * UPDATE_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j + 1));
+        }
         for (int k = 0; k < nseg_[2]; ++k, ++j)
             k_rk3_split<R, S><<<stage_grid(j, ctx_->sm_count), SPLIT_THREADS, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
     }
@@ -1278,6 +1275,8 @@ int lgf_debug_gradient(lgf_lattice* lat, double* Z) {
     // (the plaquette form's fields go to the ring's second buffer, free between flows)
     const dim3 gp(blocks_for(b.g.V, 128), 6), gl(blocks_for(b.g.V, 128), 4);
     if (b.prec == LGF_PREC_FP64) {
+        if (plaquette_stage<double>(b.g))
+            k_debug_plaquettes<double><<<gp, 128, 0, ctx->stream>>>((const cplx<double>*)b.U[0], b.g, (double*)b.U[1]);
         k_debug_gradient<double><<<gl, 128, 0, ctx->stream>>>((const cplx<double>*)b.U[0], (const double*)b.U[1], b.g, d);
     } else {
         if (plaquette_stage<float>(b.g))

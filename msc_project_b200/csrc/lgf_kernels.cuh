@@ -441,7 +441,8 @@ __device__ __forceinline__ void update_link(R* A, cplx<R>* Uout, double eps, int
     store_link(Uout, V, mu, s, exp_times(X, u));
 }
 
-// Staple form: FP64, and FP32 lattices below plaquette_stage's line.
+// Staple form: large FP64 lattices, and middle-sized ones of either precision
+// (plaquette_stage, stage_form).
 // Persistent: blocks stride over one segment of the tile list (seg = first
 // tile, count); tile = (lattice, first site).
 // A tile of T threads (T a multiple of 128) covers T/4 consecutive sites with
@@ -526,7 +527,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) k_rk3_split(const LatDesc<R>
     }
 }
 
-// Plaquette form: FP32 lattices above the small ones.
+// Plaquette form: FP32 lattices above the small ones, FP64 ones that L2 holds.
 //
 // The force of link (x, mu) sums the six plaquettes that contain the link,
 // projected: Z = -i sum_nu F[W_+nu] + F[W_-nu] with W based at x and starting
@@ -543,11 +544,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) k_rk3_split(const LatDesc<R>
 // FP32, bound by instruction issue, gains: one B200, us per step (3 stages),
 // 24^3x48 803 -> 661, 32^4 1251 -> 1012, 48^4 6900 -> 5600, 16^4 89 -> 76,
 // 6x10x14x18 35 -> 31.
-// FP64, where both forms are bound by L2 latency and bandwidth (plaquettes
-// 153 us at 0.49 of the FP64 pipe, update 278 us at 0.45 with DRAM at 5 TB/s,
-// 24^3x48), does not: 1197 -> 1153, and 48^4 10160 -> 11700; keeping a chunk
-// of x0 slices' plaquettes in L2 with a launch per chunk was slower still
-// (1350 in chunks of 256 MB, 1570 of 64 MB).
+// FP64 gains where L2 holds what is read again, links and projections, 960
+// bytes per site: 16^4 138 -> 119, 32x16^3 272 -> 237, 12^4 53 -> 49.  Beyond
+// it is bound by that traffic (24^3x48: plaquettes 153 us at 0.49 of the FP64
+// pipe, update 278 us at 0.45 with DRAM at 5 TB/s): 24^3x48 1197 -> 1205, 48^4
+// 10160 -> 11250; keeping a chunk of x0 slices' plaquettes in L2 with a launch
+// per chunk was slower still (1350 in chunks of 256 MB, 1570 of 64 MB).
 constexpr int PLAQ_SITES = 32;    // sites of a plaquette tile: a warp per plane
 constexpr int UPDATE_SITES = 32;  // sites of an update tile: a warp per direction
 template <typename R> __device__ __forceinline__ R* plaq_field(R* K, int p, int s) {
@@ -606,9 +608,12 @@ __device__ __forceinline__ alg<R> force_at(const cplx<R>* __restrict__ U, const 
     return z;
 }
 
-// 24 warps of 80 registers per SM (30 of 64 registers: 16^4 5% slower)
+// FP32: 24 warps of 80 registers per SM (30 of 64 registers: 16^4 5% slower).
+// FP64: 12 of 158, which leave the compiler room to issue a plaquette's loads
+// together (18 of 96: 16^4 124 us per step instead of 119).
+template <typename R> __host__ __device__ constexpr int plaq_blocks() { return sizeof(R) == sizeof(float) ? 4 : 2; }
 template <typename R, int S>
-__global__ void __launch_bounds__(6 * PLAQ_SITES, 4) k_rk3_plaquettes(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
+__global__ void __launch_bounds__(6 * PLAQ_SITES, plaq_blocks<R>()) k_rk3_plaquettes(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
                                                                      Work work) {
     const int2 r = work_range(work);  // this launch's tiles: tiles[r.x, r.x + r.y)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -621,10 +626,12 @@ __global__ void __launch_bounds__(6 * PLAQ_SITES, 4) k_rk3_plaquettes(const LatD
     }
 }
 
-// 20 warps of 96 registers per SM (24 of 80 with each load beside its shift: 32^4 1030 us
-// per step instead of 1012; 16 of 127: 1037)
+// FP32: 20 warps of 96 registers per SM (24 of 80 with each load beside its
+// shift: 32^4 1030 us per step instead of 1012; 16 of 127: 1037).  FP64: 16 of
+// 128 (20 of 96 spill: 16^4 134 instead of 119; 12 of 168: 124).
+template <typename R> __host__ __device__ constexpr int update_blocks() { return sizeof(R) == sizeof(float) ? 5 : 4; }
 template <typename R, int S>
-__global__ void __launch_bounds__(4 * UPDATE_SITES, 5) k_rk3_update(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
+__global__ void __launch_bounds__(4 * UPDATE_SITES, update_blocks<R>()) k_rk3_update(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
                                                                    Work work) {
     const int2 r = work_range(work);
     const int mu = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -640,14 +647,16 @@ __global__ void __launch_bounds__(4 * UPDATE_SITES, 5) k_rk3_update(const LatDes
     }
 }
 
-// Whether a lattice's stages take the plaquette form.  Small FP32 lattices do
-// not: their two short launches cost more than the operations they save (8^4:
-// 22.6 against 18.5 us per step; from 15120 sites on, 31 against 35, they do).
-// The rule reads the lattice alone, so a lattice gives the same bits in every
-// group.
-constexpr int PLAQ_MIN_SITES = 8192;
+// Whether a lattice's stages take the plaquette form.  Small lattices do not:
+// the two short launches cost more than the operations they save (FP32 8^4:
+// 22.6 against 18.5 us per step, from 15120 sites on, 31 against 35, they do;
+// FP64 16384 sites: 43 against 41, 20736: 49 against 53).  Nor do FP64
+// lattices past L2 (196608 sites: 365 against 379; 276480, 331776, 442368:
+// equal within the runs' spread; 48^4 11% slower).  The rule reads the lattice
+// alone, so a lattice gives the same bits in every group.
+constexpr int PLAQ_MIN_SITES = 8192, PLAQ_MIN_SITES_FP64 = 18432, PLAQ_MAX_SITES_FP64 = 200000;
 template <typename R> __host__ __device__ __forceinline__ bool plaquette_stage(const Geom& g) {
-    return sizeof(R) == sizeof(float) && g.V >= PLAQ_MIN_SITES;
+    return sizeof(R) == sizeof(float) ? g.V >= PLAQ_MIN_SITES : g.V >= PLAQ_MIN_SITES_FP64 && g.V <= PLAQ_MAX_SITES_FP64;
 }
 // 0: staple form, 1: plaquette form, 2: split form
 template <typename R> __host__ __device__ __forceinline__ int stage_form(const Geom& g) {

@@ -1,6 +1,6 @@
-"""The stage's forms -- split (lattices of up to 148 tiles of 32 sites), FP32
-plaquettes (8192 sites and more), staples -- at tile edges: slices and volumes that are no multiple of
-32 sites, extents of 4 (every neighbour wraps), volumes on both sides of the
+"""The stage's forms -- split (lattices of up to 148 tiles of 32 sites), plaquettes
+(FP32 from 8192 sites on, FP64 from 18432 to 200000), staples -- at tile edges:
+slices and volumes that are no multiple of 32 sites, extents of 4 (every neighbour wraps), volumes on both sides of the
 rule's line.
 
 Tolerance: a force coordinate sums six projections of products of unit-size
@@ -39,8 +39,9 @@ def test_fp32_force_matches_fp64(ctx, shape):
     assert np.max(np.abs(step - step64)) < 5e-6
 
 
-@pytest.mark.parametrize("shape", [(4, 4, 4, 4), (4, 6, 8, 10), (8, 8, 8, 8), (4, 4, 4, 74), (4, 4, 4, 76)])
-def test_fp64_small_lattices_match_the_oracle(ctx, shape):
+@pytest.mark.parametrize("shape", [(4, 4, 4, 4), (4, 6, 8, 10), (8, 8, 8, 8), (4, 4, 4, 74), (4, 4, 4, 76), (12, 12, 8, 14),
+                                   (12, 12, 8, 16), (10, 14, 10, 14), (4, 4, 4, 290), (20, 20, 20, 24), (20, 20, 20, 26)])
+def test_fp64_steps_match_the_oracle(ctx, shape):
     U = O.generate_G(shape, 23, 0.5)
     want = U
     for _ in range(2):
@@ -51,15 +52,17 @@ def test_fp64_small_lattices_match_the_oracle(ctx, shape):
         assert np.max(np.abs(lat.download() - np.asarray(want).reshape(-1))) < 1e-13  # six stages of ~30 roundings
 
 
-def test_fp32_results_do_not_depend_on_the_batch(ctx):
+@pytest.mark.parametrize("prec, shapes", [
+    (FP32MIXED, [(6, 10, 14, 18), (4, 4, 4, 4), (8, 8, 8, 14), (8, 8, 8, 16), (16, 16, 8, 10)]),
+    (FP64, [(12, 12, 8, 14), (8, 8, 8, 8), (10, 14, 10, 14), (12, 12, 8, 16)])])
+def test_results_do_not_depend_on_the_batch(ctx, prec, shapes):
     """Small and large lattices in one batch take different forms and launches; each gives the bits it gives alone."""
-    shapes = [(6, 10, 14, 18), (4, 4, 4, 4), (8, 8, 8, 14), (8, 8, 8, 16), (16, 16, 8, 10)]
     links = [O.generate_G(s, 40 + i, 0.5) for i, s in enumerate(shapes)]
-    jobs = [Job(s, FP32MIXED, links=u, nsteps=4 + 2 * (i % 2), meas_every=2, reunit_every=3, want_links=True, slices=True)
+    jobs = [Job(s, prec, links=u, nsteps=4 + 2 * (i % 2), meas_every=2, reunit_every=3, want_links=True, slices=True)
             for i, (s, u) in enumerate(zip(shapes, links))]
     ctx.batch_run(jobs)
     for j, u in zip(jobs, links):
-        with ctx.lattice(j.shape, FP32MIXED) as lat:
+        with ctx.lattice(j.shape, prec) as lat:
             lat.upload(u)
             r = lat.flow(j.eps, j.nsteps, 2, reunit_every=3, slices=True)
             assert np.array_equal(r.E, j.result.E) and np.array_equal(r.Q, j.result.Q)
