@@ -540,6 +540,8 @@ def engine_arm(args):
                 forms["served_saturated_vs_batched_fp32mixed"] = (
                     sat[0]["site_steps_per_s"] / forms["batched"]["fp32mixed"]["site_steps_per_s"])
 
+    # counted once per stage and three times per measurement, a lower bound: the FP32-mixed stage is two launches
+    # and this lattice's measurement six
     launches_per_job = 3 * NSTEPS + 3 * nmeas + (NSTEPS // 10 if reunit else 0)
     line = {
         "metric": "site-RK3-steps/s", "value": value, "unit": "site-RK3-steps/s", "n_gpus": world,
@@ -554,7 +556,7 @@ def engine_arm(args):
                 "d2h_bytes_per_step": nmeas * 3 * 8},
         "flow_only": {"value": flow_only, "unit": "site-RK3-steps/s",
                       "note": "the same 300 steps without E/Q measurements (device time)"},
-        "roofline": {"bound": pipe_name, "kernel": "k_rk3_stage (mean of the 3 stages)",
+        "roofline": {"bound": pipe_name, "kernel": ("k_rk3_stage" if prec == FP64 else "k_rk3_plaquettes + k_rk3_update") + " (mean of the 3 stages)",
                      "achieved": stage_tflops, "peak": fma_peak, "unit": "TFLOP/s", "frac": stage_tflops / fma_peak,
                      "peak_kind": f"nominal: {N_SM} SM x {fma_lanes} {pipe_name.upper()} FMA lanes x 2 flops x the run's "
                                   f"median SM clock (no measured {pipe_name.upper()} peak exists for this pool)",

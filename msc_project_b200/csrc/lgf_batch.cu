@@ -4,7 +4,7 @@
 // set of one RK3 stage (input and output link buffers plus the su(3)
 // accumulator) fits in the 126 MB L2 (budget 96 MB).  A wave is one group:
 // every RK3 stage of all its jobs is a single persistent launch over the
-// wave's shared tile list, one RK3 step (three stage launches) is captured
+// wave's shared tile list, one RK3 step (its stage launches) is captured
 // once as a CUDA graph and replayed, and jobs that finish early leave the
 // work list (the graph reads the list and its length from device memory, so
 // it is not re-captured).  Waves run one after another, so a wave's links stay

@@ -226,6 +226,9 @@ public:
     ~Group() override {
         cudaStreamSynchronize(ctx_->stream);  // the lists are in use until then
         drop_graphs();
+        for (auto st : side_) if (st) cudaStreamDestroy(st);
+        for (auto e : join_) if (e) cudaEventDestroy(e);
+        if (fork_) cudaEventDestroy(fork_);
         cudaFree(d_desc_);
         cudaFree(d_tiles_);
         cudaFree(d_mtiles_);
@@ -247,8 +250,13 @@ public:
         LGF_CUDA_TRY(ctx_, cudaMalloc(&d_sel_, sizeof(int) * sel_ints(max_members_)));
         LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_counts_, 0, sizeof(int) * 2, ctx_->stream));
         LGF_CUDA_TRY(ctx_, cudaMemsetAsync(d_sel_, 0, sizeof(int) * sel_ints(max_members_), ctx_->stream));
+        if (dynamic_ && max_members_ > 1) {
+            LGF_CUDA_TRY(ctx_, cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
+            for (auto& e : join_) LGF_CUDA_TRY(ctx_, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            for (int k = 1; k >= 0; --k) LGF_CUDA_TRY(ctx_, cudaStreamCreateWithFlags(&side_[k], cudaStreamNonBlocking));
+        }
         int nb = 0;
-        LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_stage<R, 1>, threads_, 0));
+        LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_stage<R, 1, false>, threads_, 0));
         stage_grid_max_ = std::max(1, nb) * ctx_->sm_count;
         LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_plaquettes<R, 1>, 6 * PLAQ_SITES, 0));
         plaq_grid_max_ = std::max(1, nb) * ctx_->sm_count;
@@ -313,11 +321,17 @@ public:
         // the stage's launches, form by form (stage_form): one per run of whole
         // members, two (plaquettes, update) with the plaquette form
         std::vector<int2> segs;
-        nseg_ = {0, 0, 0};
-        for (int form = 0; form < 3; ++form) {
+        // (form 3: the split form's lattices where they have more tiles than there are SMs)
+        nseg_ = {0, 0, 0, 0};
+        long long split_tiles = 0;
+        for (auto* b : members)
+            if (stage_form<R>(b->g) == 2) split_tiles += (b->g.V + SPLIT_SITES - 1) / SPLIT_SITES;
+        for (int form = 0; form < FORMS; ++form) {
             std::vector<int> which, len;
             for (size_t i = 0; i < members.size(); ++i) {
-                if (stage_form<R>(members[i]->g) != form) continue;
+                int f = stage_form<R>(members[i]->g);
+                if (f == 2 && split_tiles > ctx_->sm_count) f = 3;
+                if (f != form) continue;
                 which.push_back((int)i);
                 len.push_back((members[i]->g.V + threads_ / 4 - 1) / (threads_ / 4));
             }
@@ -528,7 +542,7 @@ public:
         LGF_CUDA_TRY(ctx_, cudaGraphLaunch(g, ctx_->stream));
         return LGF_OK;
     }
-    int launches_per_step() const override { return 3 * (nseg_[0] + 2 * nseg_[1] + nseg_[2]); }
+    int launches_per_step() const override { return 3 * (nseg_[0] + 2 * nseg_[1] + nseg_[2] + nseg_[3]); }
     int launches_per_measure() const override { return (meas_small_ ? 1 : 0) + (meas_nseg_ ? 4 * meas_nseg_ + 1 : 0) + 1; }
     int threads() const override { return threads_; }
     const TileShape& shape() const override { return shape_; }
@@ -575,31 +589,62 @@ private:
     // a stage launch's grid: persistent, or fewer blocks when its list is shorter
     int stage_grid(int j, int most) const { return dynamic_ ? most : std::max(1, std::min(seg_tiles_[j].y, most)); }
     Work stage_work(int j) const { return dynamic_ ? Work{d_seg_ + j, 0, 0} : Work{nullptr, seg_tiles_[j].x, seg_tiles_[j].y}; }
-    int step_graph() const { return (nseg_[0] * (slots_ + 1) + nseg_[1]) * (slots_ + 1) + nseg_[2]; }
-    // stage S: the launches of the staple form, the plaquette form's pairs, the split form's
-    template <int S> void launch_stage_of() {
+    int step_graph() const {
+        int key = 0;
+        for (const int n : nseg_) key = key * (slots_ + 1) + n;
+        return key;
+    }
+    // stage S of one form's lattices: the staple form, the plaquette form's
+    // pairs, the split form's (either kernel)
+    template <int S> void launch_form_of(int form, cudaStream_t st) {
         int j = 0;
-        for (int k = 0; k < nseg_[0]; ++k, ++j)
-            k_rk3_stage<R, S><<<stage_grid(j, stage_grid_max_), threads_, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
-        for (int k = 0; k < nseg_[1]; ++k, j += 2) {
-            k_rk3_plaquettes<R, S><<<stage_grid(j, plaq_grid_max_), 6 * PLAQ_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
-            k_rk3_update<R, S><<<stage_grid(j + 1, update_grid_max_), 4 * UPDATE_SITES, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j + 1));
+        for (int f = 0; f < form; ++f) j += f == 1 ? 2 * nseg_[f] : nseg_[f];
+        for (int k = 0; k < nseg_[form]; ++k) {
+            if (form == 0) {
+                k_rk3_stage<R, S, false><<<stage_grid(j, stage_grid_max_), threads_, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
+            } else if (form == 1) {
+                k_rk3_plaquettes<R, S><<<stage_grid(j, plaq_grid_max_), 6 * PLAQ_SITES, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
+                ++j;
+                k_rk3_update<R, S><<<stage_grid(j, update_grid_max_), 4 * UPDATE_SITES, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
+            } else if (form == 2) {
+                k_rk3_split<R, S><<<stage_grid(j, ctx_->sm_count), SPLIT_THREADS, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
+            } else {
+                k_rk3_stage<R, S, true><<<stage_grid(j, stage_grid_max_), threads_, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
+            }
+            ++j;
         }
-        for (int k = 0; k < nseg_[2]; ++k, ++j)
-            k_rk3_split<R, S><<<stage_grid(j, ctx_->sm_count), SPLIT_THREADS, 0, ctx_->stream>>>(d_desc_, d_tiles_, stage_work(j));
+    }
+    void launch_form(int S, int form, cudaStream_t st) {
+        if (S == 1) launch_form_of<1>(form, st);
+        if (S == 2) launch_form_of<2>(form, st);
+        if (S == 3) launch_form_of<3>(form, st);
     }
     void launch_stage(int S) {
-        if (S == 1) launch_stage_of<1>();
-        if (S == 2) launch_stage_of<2>();
-        if (S == 3) launch_stage_of<3>();
+        for (int form = 0; form < FORMS; ++form) launch_form(S, form, ctx_->stream);
     }
+    // One RK3 step.  Lattices do not read one another, so the forms of a mixed
+    // group run beside each other, joined at the step's end, and small
+    // lattices' launches fill each other's tails.
     int launch_stages() {
         if (!dynamic_ && ntiles_ == 0) return LGF_OK;
         static const char* names[3] = {"lgf.rk3_stage1", "lgf.rk3_stage2", "lgf.rk3_stage3"};
+        int forms[FORMS], n = 0;
+        for (int form = 0; form < FORMS; ++form)
+            if (nseg_[form]) forms[n++] = form;
+        const bool beside = n > 1 && side_[0];
+        if (beside) {
+            LGF_CUDA_TRY(ctx_, cudaEventRecord(fork_, ctx_->stream));
+            for (int k = 1; k < n; ++k) LGF_CUDA_TRY(ctx_, cudaStreamWaitEvent(side_[k - 1], fork_, 0));
+        }
         for (int S = 1; S <= 3; ++S) {
             NvtxRange r(names[S - 1]);
-            launch_stage(S);
+            for (int k = 0; k < n; ++k) launch_form(S, forms[k], beside && k > 0 ? side_[k - 1] : ctx_->stream);
         }
+        if (beside)
+            for (int k = 1; k < n; ++k) {
+                LGF_CUDA_TRY(ctx_, cudaEventRecord(join_[k - 1], side_[k - 1]));
+                LGF_CUDA_TRY(ctx_, cudaStreamWaitEvent(ctx_->stream, join_[k - 1], 0));
+            }
         LGF_CUDA_TRY(ctx_, cudaGetLastError());
         return LGF_OK;
     }
@@ -692,7 +737,10 @@ private:
     int stage_grid_max_ = 1, small_grid_max_ = 1, loops_grid_max_ = 1, planes_grid_max_ = 1;
     int meas_groups_ = LOOP_MAX_GROUPS, unit_sites_ = PLANE_MAX_SITES;  // tiles per loops block, sites per plane unit
     int slots_;                                   // launch slots per kernel (member_runs)
-    std::array<int, 3> nseg_{};                   // stage launch segments in use, by stage form
+    static constexpr int FORMS = 4;               // staple, plaquette, split, split on the staple kernel
+    cudaStream_t side_[2] = {};                   // a mixed group's other forms (at most three forms at a time)
+    cudaEvent_t fork_ = nullptr, join_[2] = {};
+    std::array<int, FORMS> nseg_{};                   // stage launch segments in use, by stage form
     int meas_nseg_ = 1;                           // the measurement's
     int small_tiles_ = 0, slice_count_ = 0;       // the measured members' small tiles and x0 slices
     bool meas_small_ = false;                      // some measured lattice takes the one-launch kernel

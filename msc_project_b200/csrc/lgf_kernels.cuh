@@ -1,7 +1,8 @@
 // sm_100a kernels of the Wilson-flow engine.
 //
-//   k_rk3_stage<R,S>   one fused Luscher RK3 stage for every link (FP64; FP32:
-//                      k_rk3_plaquettes + k_rk3_update): staple,
+//   k_rk3_stage<R,S,PARTS>  one fused Luscher RK3 stage for every link (by size,
+//                      stage_form: also k_rk3_split, or k_rk3_plaquettes +
+//                      k_rk3_update): staple,
 //                      projected force Z, su(3) accumulator update,
 //                      Cayley-Hamilton exponential, link update (ping-pong).
 //                      Replaces Wilson::calculate_FlowGradient
@@ -70,12 +71,29 @@ __device__ __forceinline__ void add_staples(su3<R>& S, const cplx<R>* __restrict
     }
 }
 
-template <typename R>
+// PARTS: a sum per nu, added in order (the split form's grouping)
+template <typename R, bool PARTS = false>
 __device__ __forceinline__ su3<R> staple_sum(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c, int mu) {
     const Dir dm = dir_of(g, c, mu);
     su3<R> S;
     su3_zero(S);
     const int xpm = fwd(s, dm);
+    if (PARTS) {
+#pragma unroll
+        for (int part = 0; part < 3; ++part) {
+            const int nu = part + (part >= mu ? 1 : 0);
+            const int xn = sel4(nu, c.x[0], c.x[1], c.x[2], c.x[3]);
+            if (part == 0) {
+                add_staples(S, U, g, s, mu, dm, xpm, nu, xn);
+            } else {
+                su3<R> P;
+                su3_zero(P);
+                add_staples(P, U, g, s, mu, dm, xpm, nu, xn);
+                su3_addto(S, P);
+            }
+        }
+        return S;
+    }
 #pragma unroll
     for (int nu = 0; nu < 4; ++nu)
         if (nu != mu) add_staples(S, U, g, s, mu, dm, xpm, nu, c.x[nu]);
@@ -114,10 +132,10 @@ template <typename R> __device__ __forceinline__ alg<R> ta_of_product(const su3<
     return z;
 }
 
-template <typename R>
+template <typename R, bool PARTS = false>
 __device__ __forceinline__ alg<R> flow_gradient(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c,
                                                 int mu, su3<R>& u_out) {
-    const su3<R> S = staple_sum<R>(U, g, s, c, mu);
+    const su3<R> S = staple_sum<R, PARTS>(U, g, s, c, mu);
     u_out = load_link(U, g.V, mu, s);
     return ta_of_product(u_out, S, R(-0.5));
 }
@@ -452,7 +470,7 @@ __device__ __forceinline__ void update_link(R* A, cplx<R>* Uout, double eps, int
 template <typename R> struct StageMaxThreads { static constexpr int value = LGF_STAGE_MAXT_F; };
 template <> struct StageMaxThreads<double> { static constexpr int value = LGF_STAGE_MAXT_D; };
 
-template <typename R, int S>
+template <typename R, int S, bool PARTS>
 __global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_rk3_stage(const LatDesc<R>* __restrict__ descs, const int2* __restrict__ tiles,
                                                    Work work) {
     const int2 r = work_range(work);  // this launch's tiles: tiles[r.x, r.x + r.y)
@@ -469,7 +487,7 @@ __global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_r
         const double eps = d->eps;
         const Coord c = site_coord(g, s);
         su3<R> u;
-        const alg<R> Z = flow_gradient<R>(Uin, g, s, c, mu, u);
+        const alg<R> Z = flow_gradient<R, PARTS>(Uin, g, s, c, mu, u);
         update_link<R, S>(A, Uout, eps, g.V, s, mu, Z, u);
     }
 }
@@ -481,6 +499,11 @@ __global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_r
 // 8^4 FP64 22.6 -> 20 us per step (19 with the range by value, Work), FP32
 // 18.5 -> 17.5 (16.5).  Above the line an SM with two tiles would run them in
 // turn, and the staple form runs them side by side.
+// Where a group's small lattices have more tiles than that, the staple form
+// with the same grouping of the sum (PARTS) takes them, so that the bits are
+// those the lattice gives alone: 64 x 8^4 batched, 200 steps, FP32 84 -> 78 ms
+// on the device, FP64 118 -> 123 (the second sum spills 40 bytes; the split
+// kernel itself, a tile per SM at a time, took 1.5 times as long).
 constexpr int SPLIT_SITES = 32, SPLIT_THREADS = 12 * SPLIT_SITES;
 constexpr long long SPLIT_MAX_SITES = 148 * SPLIT_SITES;
 template <typename R, int S>

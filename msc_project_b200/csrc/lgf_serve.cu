@@ -541,12 +541,11 @@ void lgf_server::run() {
     if (snap_thread.joinable()) snap_thread.join();
 }
 
-// Kernel shape (block size, measurement warps per plane) of the shared
-// launches of one precision: the defaults.  A shape tuned on one volume
-// class is not carried over to every job of a mix: a one-warp-per-plane
-// measurement tuned (by under 2%) on 24^3x48 slowed a served mix of four
-// volumes by 12%.  Each job's work order is still its own class's tuned
-// order (the groups' per-volume lists).
+// Kernel shape (stage and measurement block sizes) of the shared launches of
+// one precision: the defaults.  A shape tuned on one volume class is not
+// carried over to every job of a mix: one tuned (by under 2%) on 24^3x48
+// slowed a served mix of four volumes by 12%.  Each job's work order is still
+// its own class's tuned order (the groups' per-volume lists).
 static TileShape serve_shape(const lgf_ctx*, int prec) { return default_shape(prec, 1LL << 40); }
 
 extern "C" {

@@ -54,7 +54,10 @@ def test_fp64_steps_match_the_oracle(ctx, shape):
 
 @pytest.mark.parametrize("prec, shapes", [
     (FP32MIXED, [(6, 10, 14, 18), (4, 4, 4, 4), (8, 8, 8, 14), (8, 8, 8, 16), (16, 16, 8, 10)]),
-    (FP64, [(12, 12, 8, 14), (8, 8, 8, 8), (10, 14, 10, 14), (12, 12, 8, 16)])])
+    (FP64, [(12, 12, 8, 14), (8, 8, 8, 8), (10, 14, 10, 14), (12, 12, 8, 16)]),
+    # more small tiles than SMs: the batch takes the staple form with the split form's sums
+    (FP32MIXED, [(8, 8, 8, 8), (4, 6, 8, 10), (6, 10, 14, 18), (4, 4, 4, 74)]),
+    (FP64, [(8, 8, 8, 8), (4, 6, 8, 10), (12, 12, 8, 14), (4, 4, 4, 74)])])
 def test_results_do_not_depend_on_the_batch(ctx, prec, shapes):
     """Small and large lattices in one batch take different forms and launches; each gives the bits it gives alone."""
     links = [O.generate_G(s, 40 + i, 0.5) for i, s in enumerate(shapes)]
