@@ -61,8 +61,8 @@ size_t footprint_bytes(const int shape[4], int precision, int meas_slots) {
 // and 48^4), FP32 128.  A lattice too small to fill the SMs evenly with 96-site
 // tiles takes 32-site ones: the SM with the most tiles sets the time, so the
 // smaller tiles are taken where they cut that SM's sites by over a tenth
-// (12^4: 60 -> 54 us per step; 16^4, at 448 against 480 sites, 140 either way;
-// 8^4 takes the split form, which has its own tile).
+// (12^4 in the staple form: 60 -> 54 us per step; 16^4, at 448 against 480
+// sites, 140 either way).  The other stage forms have tiles of their own.
 int stage_max_threads(int precision) { return precision == LGF_PREC_FP64 ? LGF_STAGE_MAXT_D : LGF_STAGE_MAXT_F; }
 
 TileShape default_shape(int precision, long long volume) {
