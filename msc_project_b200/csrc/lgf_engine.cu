@@ -269,14 +269,17 @@ public:
         while (meas_groups_ > 1 && cap_sites < (long long)MEAS_SITES * meas_groups_ * ctx_->sm_count) meas_groups_ /= 2;
         unit_sites_ = shape_.meas_split == 2 ? PLANE_MAX_SITES : PLANE_MAX_SITES / 2;
         while (unit_sites_ > 96 && 3 * cap_sites < (long long)unit_sites_ * ctx_->sm_count) unit_sites_ /= 2;
-        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_measure<R, true>, MEAS_SITES * MEAS_WARPS, measure_smem_bytes<R>(), &nb)));
-        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_measure<R, false>, MEAS_SITES * MEAS_WARPS, measure_smem_bytes<R>(), &small_grid_max_)));
-        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_loops<R, 0>, 96 * meas_groups_, loops_smem_bytes(meas_groups_), &loops_grid_max_)));
-        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_loops<R, 1>, 96 * meas_groups_, loops_smem_bytes(meas_groups_), &nb)));
-        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 0, false>, unit_sites_, planes_smem_bytes<R>(unit_sites_), &planes_grid_max_)));
-        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 1, false>, unit_sites_, planes_smem_bytes<R>(unit_sites_), &nb)));
-        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 0, true>, unit_sites_, planes_smem_bytes<R>(unit_sites_), &nb)));
-        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 1, true>, unit_sites_, planes_smem_bytes<R>(unit_sites_), &nb)));
+        const size_t one = measure_smem_bytes<R>(), loops = loops_smem_bytes(meas_groups_), loops_most = loops_smem_bytes(LOOP_MAX_GROUPS);
+        const size_t planes = planes_smem_bytes<R>(unit_sites_), planes_most = planes_smem_bytes<R>(PLANE_MAX_SITES);
+        const int lt = 96 * meas_groups_;
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_measure<R, true>, MEAS_SITES * MEAS_WARPS, one, one, &nb)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_measure<R, false>, MEAS_SITES * MEAS_WARPS, one, one, &small_grid_max_)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_loops<R, 0>, lt, loops, loops_most, &loops_grid_max_)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_loops<R, 1>, lt, loops, loops_most, &nb)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 0, false>, unit_sites_, planes, planes_most, &planes_grid_max_)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 1, false>, unit_sites_, planes, planes_most, &nb)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 0, true>, unit_sites_, planes, planes_most, &nb)));
+        LGF_CUDA_TRY(ctx_, (meas_occupancy(k_meas_planes<R, 1, true>, unit_sites_, planes, planes_most, &nb)));
         if (dynamic_) {
             // members change after capture: size the measurement lists for the
             // largest resident set the tile capacity allows (x0 extents <= 256)
@@ -552,9 +555,12 @@ private:
     int meas_grid(long long work, int grid_max) const {
         return dynamic_ ? grid_max : (int)std::max(1LL, std::min(work, (long long)grid_max));
     }
-    // raise the kernel's shared-memory limit and find its persistent grid
-    template <typename K> cudaError_t meas_occupancy(K kernel, int threads, size_t smem, int* grid) const {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // Set the kernel's shared-memory limit and find its persistent grid for this
+    // group's blocks.  The limit belongs to the kernel on the device, for every
+    // group and context of the process, and the last one set holds: it is the
+    // most that any group's blocks take, never this group's own.
+    template <typename K> cudaError_t meas_occupancy(K kernel, int threads, size_t smem, size_t most, int* grid) const {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         int nb = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem);
         *grid = std::max(1, nb) * ctx_->sm_count;
