@@ -1316,14 +1316,17 @@ __global__ void k_debug_plaquettes(const cplx<R>* __restrict__ U, Geom g, R* __r
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < g.V) plaquette_at<R>(U, K, g, s, site_coord(g, s), blockIdx.y);
 }
-// flow gradient Z(x, mu) for every link, file order [s][mu][9] (double2), in the lattice's stage form
+// flow gradient Z(x, mu) for every link, file order [s][mu][9] (double2), summed as the lattice's stage form sums it
 template <typename R>
 __global__ void k_debug_gradient(const cplx<R>* __restrict__ U, const R* __restrict__ K, Geom g, double2* __restrict__ out) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x, mu = blockIdx.y;
     if (s >= g.V) return;
     const Coord c = site_coord(g, s);
+    const int form = stage_form<R>(g);
     su3<R> u;
-    const alg<R> Z = plaquette_stage<R>(g) ? force_at<R>(U, K, g, s, c, mu) : flow_gradient<R>(U, g, s, c, mu, u);
+    const alg<R> Z = form == 1   ? force_at<R>(U, K, g, s, c, mu)
+                     : form == 2 ? flow_gradient<R, true>(U, g, s, c, mu, u)
+                                 : flow_gradient<R, false>(U, g, s, c, mu, u);
     store_alg_as_antiherm(out + ((size_t)s * 4 + mu) * 9, Z);
 }
 
