@@ -256,7 +256,7 @@ public:
             for (int k = 1; k >= 0; --k) LGF_CUDA_TRY(ctx_, cudaStreamCreateWithFlags(&side_[k], cudaStreamNonBlocking));
         }
         int nb = 0;
-        LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_stage<R, 1, false>, threads_, 0));
+        LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_stage<R, 1, true>, threads_, 0));
         stage_grid_max_ = std::max(1, nb) * ctx_->sm_count;
         LGF_CUDA_TRY(ctx_, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rk3_plaquettes<R, 1>, 6 * PLAQ_SITES, 0));
         plaq_grid_max_ = std::max(1, nb) * ctx_->sm_count;
@@ -324,16 +324,16 @@ public:
         // the stage's launches, form by form (stage_form): one per run of whole
         // members, two (plaquettes, update) with the plaquette form
         std::vector<int2> segs;
-        // (form 3: the split form's lattices where they have more tiles than there are SMs)
+        // (split lattices with more tiles than there are SMs take the staple kernel, FORM_PARTS)
         nseg_ = {0, 0, 0, 0};
         long long split_tiles = 0;
         for (auto* b : members)
-            if (stage_form<R>(b->g) == 2) split_tiles += (b->g.V + SPLIT_SITES - 1) / SPLIT_SITES;
+            if (stage_form<R>(b->g) == FORM_SPLIT) split_tiles += (b->g.V + SPLIT_SITES - 1) / SPLIT_SITES;
         for (int form = 0; form < FORMS; ++form) {
             std::vector<int> which, len;
             for (size_t i = 0; i < members.size(); ++i) {
                 int f = stage_form<R>(members[i]->g);
-                if (f == 2 && split_tiles > ctx_->sm_count) f = 3;
+                if (f == FORM_SPLIT && split_tiles > ctx_->sm_count) f = FORM_PARTS;
                 if (f != form) continue;
                 which.push_back((int)i);
                 len.push_back((members[i]->g.V + threads_ / 4 - 1) / (threads_ / 4));
@@ -344,12 +344,12 @@ public:
             for (const int2& run : member_runs(len, slots_, 8LL * stage_grid_max_)) {
                 const size_t m0 = m;
                 while (m < which.size() && pos < (long long)run.x + run.y) pos += len[m++];
-                for (int part = 0; part < (form == 1 ? 2 : 1); ++part) {
+                for (int part = 0; part < (form == FORM_PLAQUETTE ? 2 : 1); ++part) {
                     const int first = (int)tiles.size();
                     for (size_t k = m0; k < m; ++k) {
                         const Geom& g = members[which[k]]->g;
-                        if (form == 1) append_site_tiles(tiles, which[k], g, part ? UPDATE_SITES : PLAQ_SITES);
-                        else if (form == 2) append_site_tiles(tiles, which[k], g, SPLIT_SITES);
+                        if (form == FORM_PLAQUETTE) append_site_tiles(tiles, which[k], g, part ? UPDATE_SITES : PLAQ_SITES);
+                        else if (form == FORM_SPLIT) append_site_tiles(tiles, which[k], g, SPLIT_SITES);
                         else append_staple_tiles(tiles, which[k], g);
                     }
                     segs.push_back(make_int2(first, (int)tiles.size() - first));
@@ -545,7 +545,7 @@ public:
         LGF_CUDA_TRY(ctx_, cudaGraphLaunch(g, ctx_->stream));
         return LGF_OK;
     }
-    int launches_per_step() const override { return 3 * (nseg_[0] + 2 * nseg_[1] + nseg_[2] + nseg_[3]); }
+    int launches_per_step() const override { return 3 * (nseg_[FORM_STAPLE] + 2 * nseg_[FORM_PLAQUETTE] + nseg_[FORM_SPLIT] + nseg_[FORM_PARTS]); }
     int launches_per_measure() const override { return (meas_small_ ? 1 : 0) + (meas_nseg_ ? 4 * meas_nseg_ + 1 : 0) + 1; }
     int threads() const override { return threads_; }
     const TileShape& shape() const override { return shape_; }
@@ -604,18 +604,18 @@ private:
     // pairs, the split form's (either kernel)
     template <int S> void launch_form_of(int form, cudaStream_t st) {
         int j = 0;
-        for (int f = 0; f < form; ++f) j += f == 1 ? 2 * nseg_[f] : nseg_[f];
+        for (int f = 0; f < form; ++f) j += f == FORM_PLAQUETTE ? 2 * nseg_[f] : nseg_[f];
         for (int k = 0; k < nseg_[form]; ++k) {
-            if (form == 0) {
-                k_rk3_stage<R, S, false><<<stage_grid(j, stage_grid_max_), threads_, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
-            } else if (form == 1) {
+            if (form == FORM_PLAQUETTE) {
                 k_rk3_plaquettes<R, S><<<stage_grid(j, plaq_grid_max_), 6 * PLAQ_SITES, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
                 ++j;
                 k_rk3_update<R, S><<<stage_grid(j, update_grid_max_), 4 * UPDATE_SITES, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
-            } else if (form == 2) {
+            } else if (form == FORM_SPLIT) {
                 k_rk3_split<R, S><<<stage_grid(j, ctx_->sm_count), SPLIT_THREADS, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
-            } else {
+            } else if (form == FORM_PARTS || sizeof(R) == sizeof(float)) {  // (FP32 has no other staple form)
                 k_rk3_stage<R, S, true><<<stage_grid(j, stage_grid_max_), threads_, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
+            } else if constexpr (sizeof(R) == sizeof(double)) {
+                k_rk3_stage<R, S, false><<<stage_grid(j, stage_grid_max_), threads_, 0, st>>>(d_desc_, d_tiles_, stage_work(j));
             }
             ++j;
         }
@@ -743,7 +743,6 @@ private:
     int stage_grid_max_ = 1, small_grid_max_ = 1, loops_grid_max_ = 1, planes_grid_max_ = 1;
     int meas_groups_ = LOOP_MAX_GROUPS, unit_sites_ = PLANE_MAX_SITES;  // tiles per loops block, sites per plane unit
     int slots_;                                   // launch slots per kernel (member_runs)
-    static constexpr int FORMS = 4;               // staple, plaquette, split, split on the staple kernel
     cudaStream_t side_[2] = {};                   // a mixed group's other forms (at most three forms at a time)
     cudaEvent_t fork_ = nullptr, join_[2] = {};
     std::array<int, FORMS> nseg_{};                   // stage launch segments in use, by stage form

@@ -71,7 +71,8 @@ __device__ __forceinline__ void add_staples(su3<R>& S, const cplx<R>* __restrict
     }
 }
 
-// PARTS: a sum per nu, added in order (the split form's grouping)
+// PARTS: a sum per nu, added in order (the split form's grouping; in FP32 also
+// 2 us per step faster than one sum up to 14208 sites)
 template <typename R, bool PARTS = false>
 __device__ __forceinline__ su3<R> staple_sum(const cplx<R>* __restrict__ U, const Geom& g, int s, const Coord& c, int mu) {
     const Dir dm = dir_of(g, c, mu);
@@ -460,7 +461,7 @@ __device__ __forceinline__ void update_link(R* A, cplx<R>* Uout, double eps, int
 }
 
 // Staple form: large FP64 lattices, and middle-sized ones of either precision
-// (plaquette_stage, stage_form).
+// (stage_form); PARTS as in staple_sum.
 // Persistent: blocks stride over one segment of the tile list (seg = first
 // tile, count); tile = (lattice, first site).
 // A tile of T threads (T a multiple of 128) covers T/4 consecutive sites with
@@ -671,19 +672,30 @@ __global__ void __launch_bounds__(4 * UPDATE_SITES, update_blocks<R>()) k_rk3_up
 }
 
 // Whether a lattice's stages take the plaquette form.  Small lattices do not:
-// the two short launches cost more than the operations they save (FP32 8^4:
-// 22.6 against 18.5 us per step, from 15120 sites on, 31 against 35, they do;
-// FP64 16384 sites: 43 against 41, 20736: 49 against 53).  Nor do FP64
-// lattices past L2 (196608 sites: 365 against 379; 276480, 331776, 442368:
-// equal within the runs' spread; 48^4 11% slower).  The rule reads the lattice
-// alone, so a lattice gives the same bits in every group.
-constexpr int PLAQ_MIN_SITES = 8192, PLAQ_MIN_SITES_FP64 = 18432, PLAQ_MAX_SITES_FP64 = 200000;
+// the two short launches cost more than the operations they save.  FP32, us per
+// step in the staple form with a sum per direction (PARTS), with one sum for
+// all, and in the plaquette form:
+//    4800  18.4  20.5  22.6      8192  18.6  21    24        9600  22.5  24.6  26.6
+//   12000  22.6  24.7  26.6     13824  23.2  24.6  27       14400  31.8  34.8  29.3
+//   15120        34.8  30.7     20736        37    34.8
+// so the line is one wave of the staple form: three 32-site tiles per SM.
+// FP64: 16384 sites 41 (staple, PARTS 41) against 43, 20736: 53 against 49.  Nor
+// do FP64 lattices past L2 (196608 sites: 365 against 379; 276480, 331776,
+// 442368: equal within the runs' spread; 48^4 11% slower).  The rule reads the
+// lattice alone, so a lattice gives the same bits in every group.
+constexpr int STAPLE_MAX_SITES_FP32 = 3 * 148 * 32;
+constexpr int PLAQ_MIN_SITES_FP64 = 18432, PLAQ_MAX_SITES_FP64 = 200000;
 template <typename R> __host__ __device__ __forceinline__ bool plaquette_stage(const Geom& g) {
-    return sizeof(R) == sizeof(float) ? g.V >= PLAQ_MIN_SITES : g.V >= PLAQ_MIN_SITES_FP64 && g.V <= PLAQ_MAX_SITES_FP64;
+    return sizeof(R) == sizeof(float) ? g.V > STAPLE_MAX_SITES_FP32 : g.V >= PLAQ_MIN_SITES_FP64 && g.V <= PLAQ_MAX_SITES_FP64;
 }
-// 0: staple form, 1: plaquette form, 2: split form
+// The forms: staple with one sum for all directions (FP64: above the split
+// form 26.6 us per step against 28.7 to 30.7 with PARTS), plaquette, split, and
+// staple with a sum per direction (FP32, and split lattices in large groups).
+constexpr int FORM_STAPLE = 0, FORM_PLAQUETTE = 1, FORM_SPLIT = 2, FORM_PARTS = 3, FORMS = 4;
 template <typename R> __host__ __device__ __forceinline__ int stage_form(const Geom& g) {
-    return g.V <= SPLIT_MAX_SITES ? 2 : (plaquette_stage<R>(g) ? 1 : 0);
+    if (g.V <= SPLIT_MAX_SITES) return FORM_SPLIT;
+    if (plaquette_stage<R>(g)) return FORM_PLAQUETTE;
+    return sizeof(R) == sizeof(float) ? FORM_PARTS : FORM_STAPLE;
 }
 
 template <typename R> __device__ __forceinline__ void store_alg_as_antiherm(double2* dst, const alg<R>& z) {
@@ -1324,9 +1336,9 @@ __global__ void k_debug_gradient(const cplx<R>* __restrict__ U, const R* __restr
     const Coord c = site_coord(g, s);
     const int form = stage_form<R>(g);
     su3<R> u;
-    const alg<R> Z = form == 1   ? force_at<R>(U, K, g, s, c, mu)
-                     : form == 2 ? flow_gradient<R, true>(U, g, s, c, mu, u)
-                                 : flow_gradient<R, false>(U, g, s, c, mu, u);
+    const alg<R> Z = form == FORM_PLAQUETTE ? force_at<R>(U, K, g, s, c, mu)
+                     : form == FORM_STAPLE  ? flow_gradient<R, false>(U, g, s, c, mu, u)
+                                            : flow_gradient<R, true>(U, g, s, c, mu, u);
     store_alg_as_antiherm(out + ((size_t)s * 4 + mu) * 9, Z);
 }
 
