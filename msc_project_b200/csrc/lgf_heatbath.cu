@@ -10,12 +10,12 @@
 // overrelaxation reflects the subgroup (:78-104).
 //
 // B200 mapping: one launch per (parity, direction) class updates all its links
-// in place in parallel, on a copy of the links in parity order -- the staple of
-// a link reads only other directions and opposite-parity links of its own
-// direction, so the class has no internal dependencies.  Measured per class
-// launch, FP64, against site order (same bits): 32x16^3 heatbath 40 -> 30 us,
-// overrelaxation 33 -> 22; 24^3x48 197 -> 145 and 169 -> 109; FP32 100 -> 100
-// and 68 -> 60 on 24^3x48; the copy there and back costs about three launches.
+// in place in parallel, for more than a sweep or two on a copy of the links in
+// parity order -- the staple of a link reads only other directions and
+// opposite-parity links of its own direction, so the class has no internal
+// dependencies.  Measured per class launch, FP64, against site order (same
+// bits): 32x16^3 heatbath 40 -> 30 us, overrelaxation 33 -> 22; 24^3x48 197 ->
+// 145 and 169 -> 109; FP32 105 -> 100 and 68 -> 60 on 24^3x48.
 //  Random numbers come from a counter hash of (seed, class epoch,
 // subgroup, site, draw), so results do not depend on the launch shape.  The
 // rejection loop is bounded (HB_MAX_ATTEMPTS); a subgroup whose draws all
@@ -40,7 +40,7 @@ __device__ __forceinline__ double hb_draw(unsigned long long seed, unsigned long
     return unit_open(seed, base + (unsigned long long)k);
 }
 
-// Sweeps run on a copy of the links in parity order: the V/2 even sites, then
+// Longer runs of sweeps work on a copy of the links in parity order: the V/2 even sites, then
 // the odd ones, each in site order, in the same 32-site blocks.  A class
 // updates and reads whole runs of one parity there, where in site order every
 // second site of a run is of the other parity and half of each 32-byte sector
@@ -129,17 +129,20 @@ __device__ __forceinline__ su3<R> staple_sum_parity(const cplx<R>* U, const Geom
     return S;
 }
 
-// One (parity, direction) class.  MINB: resident blocks per SM that the
-// registers are capped for (heatbath_blocks).
-template <typename R, int MINB>
+// One (parity, direction) class of links in parity order, or (PARITY false) in
+// site order; the same bits either way.  MINB: resident blocks per SM that the
+// registers are capped for (heatbath_kernel).
+template <typename R, int MINB, bool PARITY>
 __global__ void __launch_bounds__(128, MINB) k_checkerboard(cplx<R>* U, Geom g, int mu, int parity, double beta,
                                                             unsigned long long seed, unsigned long long epoch, int overrelax,
                                                             unsigned int* __restrict__ failures) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (g.V >> 1)) return;
     const ParitySite x = parity_site(g, parity, t);
-    const int s = site_index(g, x), at = parity_index(g, x);  // the random numbers are keyed by the site
-    const su3<R> A = staple_sum_parity<R>(U, g, x, mu);
+    const int s = site_index(g, x), at = PARITY ? parity_index(g, x) : s;  // the random numbers are keyed by the site
+    su3<R> A;
+    if constexpr (PARITY) A = staple_sum_parity<R>(U, g, x, mu);
+    else A = staple_sum<R>(U, g, s, site_coord(g, s), mu);
     su3<R> u = load_link(U, g.V, mu, at);
 #pragma unroll 1
     for (int sg = 0; sg < 3; ++sg) {
@@ -324,14 +327,22 @@ __global__ void __launch_bounds__(256) k_plaquette(const cplx<R>* __restrict__ U
     if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 
-// The class kernel for nb blocks.  FP64 at 3 blocks per SM (168 registers) runs
-// a full wave of blocks in 1/1.3 of the time of 4 (128 registers, some spills),
-// so 4 are taken where they save enough waves (32x16^3: one wave instead of
-// two, 22 against 24 us; 24^3x48: 6 of 3 beat 5 of 4).  FP32 takes 5 (96).
-template <typename R> auto heatbath_kernel(int nb, int sms) {
+// The class kernel for nb blocks: of the register caps (blocks per SM) the one
+// whose waves cost least, a full wave of m blocks per SM taken as cost[m].
+// FP64: 3 blocks (168 registers) 1, 4 (128, some spills) 1.3: 32x16^3 runs one
+// wave of 4 instead of two of 3, 22 against 24 us; 24^3x48 6 of 3, not 5 of 4.
+// FP32: 4 blocks (128) 4 (4.2 in parity order), 5 (96) 5.05, 6 (80, some spills)
+// 6.2: many waves cost about the same with each cap, and 192000 sites fit one wave of 6 (overrelaxation of
+// 4 sweeps in parity order 591 us, 674 in two waves of 5).
+template <typename R, bool PARITY> auto heatbath_kernel(int nb, int sms) {
     auto waves = [&](int per_sm) { return (nb + per_sm * sms - 1) / (per_sm * sms); };
-    if constexpr (sizeof(R) == sizeof(double)) return 10 * waves(3) > 13 * waves(4) ? k_checkerboard<R, 4> : k_checkerboard<R, 3>;
-    else return k_checkerboard<R, 5>;
+    if constexpr (sizeof(R) == sizeof(double)) {
+        return 10 * waves(3) > 13 * waves(4) ? k_checkerboard<R, 4, PARITY> : k_checkerboard<R, 3, PARITY>;
+    } else {
+        const int c4 = (PARITY ? 420 : 400) * waves(4), c5 = 505 * waves(5), c6 = 620 * waves(6);
+        if (c6 < c4 && c6 < c5) return k_checkerboard<R, 6, PARITY>;
+        return c5 < c4 ? k_checkerboard<R, 5, PARITY> : k_checkerboard<R, 4, PARITY>;
+    }
 }
 
 // n_iter x (heatbath sweep unless or_only, then or_per_hb overrelaxation sweeps)
@@ -342,12 +353,24 @@ int heatbath_impl(lgf_ctx* ctx, lgf_lattice* lat, double beta, int n_iter, int o
     unsigned int* dfail = reinterpret_cast<unsigned int*>(b.slot);  // (a flow resets its slot before it counts)
     LGF_CUDA_TRY(ctx, cudaMemsetAsync(dfail, 0, sizeof(unsigned int), ctx->stream));
     const int V = b.g.V, th = 128, nb = (V / 2 + th - 1) / th;
-    cplx<R>*U = (cplx<R>*)b.U[0], *P = (cplx<R>*)b.U[1];
+    // The copy to parity order and back costs about as much as it saves in one
+    // FP64 sweep, or in FP32, where a heatbath class gains little, in two
+    // overrelaxation sweeps; while L2 holds both copies and they are more than a
+    // few blocks per SM, in less.  Parity against site order, us, each with its
+    // best register cap: FP64 one heatbath sweep 24^3x48 1680 against 1470, one
+    // overrelaxation sweep 1280 against 1190 (160000 to 331776 sites 3 to 5% the
+    // other way), one of each 2460 against 2580; FP32 one of each 24^3x48 1455
+    // against 1405, 16^4 267 against 250, but 32x16^3 344 against 360 and
+    // 221184 sites 489 against 505; one and two overrelaxation sweeps more on
+    // 24^3x48 1890 against 1900, four 2030 against 2140.
+    const long long heat = or_only ? 0 : n_iter, over = (long long)n_iter * or_per_hb, sweeps = heat + over;
+    const bool parity = sizeof(R) == sizeof(double) || (V > 80000 && V < 250000) ? sweeps >= 2 : sweeps >= 4 || heat + 2 * over >= 5;
+    cplx<R>*U = (cplx<R>*)b.U[0], *P = parity ? (cplx<R>*)b.U[1] : U;
     const dim3 order((V + th - 1) / th, 4);
     cudaError_t e = cudaSuccess;
     const bool any = n_iter > 0 && (!or_only || or_per_hb > 0);
-    if (any) k_parity_order<R, true><<<order, th, 0, ctx->stream>>>(U, P, b.g);
-    auto sweep_class = heatbath_kernel<R>(nb, ctx->sm_count);
+    if (any && parity) k_parity_order<R, true><<<order, th, 0, ctx->stream>>>(U, P, b.g);
+    auto sweep_class = parity ? heatbath_kernel<R, true>(nb, ctx->sm_count) : heatbath_kernel<R, false>(nb, ctx->sm_count);
     for (int it = 0; it < n_iter && e == cudaSuccess; ++it) {
         for (int sweep = or_only ? 1 : 0; sweep <= or_per_hb && e == cudaSuccess; ++sweep) {
             const int over = sweep > 0;
@@ -359,7 +382,7 @@ int heatbath_impl(lgf_ctx* ctx, lgf_lattice* lat, double beta, int n_iter, int o
             e = cudaGetLastError();
         }
     }
-    if (any && e == cudaSuccess) {
+    if (any && parity && e == cudaSuccess) {
         k_parity_order<R, false><<<order, th, 0, ctx->stream>>>(P, U, b.g);
         e = cudaGetLastError();
     }
