@@ -988,6 +988,8 @@ int lgf_ctx_create(int device, lgf_ctx** out) {
         delete ctx;
         return LGF_ECUDA;
     }
+    // (without it every group pays for the chunk: no failure)
+    if (cudaMalloc(&ctx->small, 256) != cudaSuccess) cudaGetLastError();
     *out = ctx;
     return LGF_OK;
 }
@@ -997,6 +999,7 @@ int lgf_ctx_destroy(lgf_ctx* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     release_pinned_chunks(ctx);
+    cudaFree(ctx->small);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return LGF_OK;
