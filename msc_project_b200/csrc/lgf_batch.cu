@@ -45,13 +45,13 @@ int validate_job(lgf_ctx* ctx, const lgf_job& j) {
     return LGF_OK;
 }
 
-// tile shape for a wave whose largest lattice has this shape: tuned once per
-// precision and volume class (a small lattice prefers more, smaller blocks)
-TileShape shape_for(lgf_ctx* ctx, int prec, const int shape[4]) {
+// tile shape for waves whose largest lattice has this shape: tuned once per
+// precision and volume class (stage: its stage block size too)
+TileShape shape_for(lgf_ctx* ctx, int prec, const int shape[4], bool stage) {
     const long long V = 1LL * shape[0] * shape[1] * shape[2] * shape[3];
     if (has_tuned(ctx, prec, V)) return tuned_shape(ctx, prec, V);
     TileShape best = default_shape(prec, V);
-    if (tune_shape(ctx, prec, shape, &best) != LGF_OK) {
+    if (tune_shape(ctx, prec, shape, stage, &best) != LGF_OK) {
         ctx->err.clear();
         return default_shape(prec, V);
     }
@@ -252,6 +252,7 @@ int lgf_batch_run(lgf_ctx* ctx, lgf_job* jobs, int njobs, lgf_batch_stats* stats
     // group the jobs by precision and pick each group's block size (autotuned
     // once per context, before the timed region)
     std::vector<JobRun*> groups[2];
+    std::vector<std::vector<JobRun*>> waves_of[2];
     TileShape shapes[2];
     for (int prec = 0; prec < 2; ++prec) {
         int big[4] = {4, 4, 4, 4};
@@ -264,7 +265,23 @@ int lgf_batch_run(lgf_ctx* ctx, lgf_job* jobs, int njobs, lgf_batch_stats* stats
                     std::memcpy(big, r->job->shape, sizeof big);
                 }
             }
-        if (!groups[prec].empty()) shapes[prec] = shape_for(ctx, prec, big);
+        if (groups[prec].empty()) continue;
+        waves_of[prec] = l2_waves(groups[prec], prec);
+        // the block size that most of the staple kernel's sites are best served
+        // by; timed on the largest lattice only where a launch is about that large
+        long long votes[4] = {0, 0, 0, 0}, most = 0;
+        for (const auto& wave : waves_of[prec]) {
+            std::vector<const Geom*> g;
+            for (const auto* r : wave) g.push_back(&r->buf.g);
+            const StapleSites n = staple_sites(prec, g, ctx->sm_count);
+            for (const long long sites : {n.one_sum, n.parts}) {
+                votes[default_shape(prec, sites).threads / 128] += sites;
+                most = std::max(most, sites);
+            }
+        }
+        shapes[prec] = shape_for(ctx, prec, big, 2 * most <= 3 * bigV);
+        const int best = (int)(std::max_element(votes, votes + 4) - votes);
+        if (!has_tuned_stage(ctx, prec, bigV) && votes[best] > 0) shapes[prec].threads = 128 * best;
     }
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -277,7 +294,7 @@ int lgf_batch_run(lgf_ctx* ctx, lgf_job* jobs, int njobs, lgf_batch_stats* stats
         // one group for every wave of this precision, sized for the largest:
         // a wave replaces the previous one's members without a new group, a
         // new capture or a device synchronisation in between
-        const auto waves = l2_waves(groups[prec], prec);
+        const auto& waves = waves_of[prec];
         long long max_tiles = 1;
         int max_members = 1;
         for (const auto& wave : waves) {

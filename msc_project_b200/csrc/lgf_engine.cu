@@ -62,15 +62,36 @@ size_t footprint_bytes(const int shape[4], int precision, int meas_slots) {
 // tiles takes 32-site ones: the SM with the most tiles sets the time, so the
 // smaller tiles are taken where they cut that SM's sites by over a tenth
 // (12^4 in the staple form: 60 -> 54 us per step; 16^4, at 448 against 480
-// sites, 140 either way).  The other stage forms have tiles of their own.
+// sites, 140 either way); and 64-site ones up to one per SM (8192 sites 28.7 ->
+// 26.6 us, 2 x 8^4 batched 39 -> 31).  The other stage forms have tiles of their
+// own, so in a batch the sites are those that run the staple kernel together:
+// 64 x 8^4, 200 steps, 113 ms with 384 threads, 121 with the 128 that one 8^4
+// would take; 16 x 8^4 30.1 and 31.0; 7 x 8^4 17.8 and 14.7.
 int stage_max_threads(int precision) { return precision == LGF_PREC_FP64 ? LGF_STAGE_MAXT_D : LGF_STAGE_MAXT_F; }
 
 TileShape default_shape(int precision, long long volume) {
     const long long sms = 148;
     auto most_sites = [&](long long tile) { return ((volume + tile - 1) / tile + sms - 1) / sms * tile; };
     TileShape t;
-    t.threads = precision == LGF_PREC_FP64 && 10 * most_sites(32) > 9 * most_sites(96) ? 384 : 128;
+    t.threads = 128;
+    if (precision == LGF_PREC_FP64) {
+        if (volume > 32 * sms && volume <= 64 * sms) t.threads = 256;
+        else if (10 * most_sites(32) > 9 * most_sites(96)) t.threads = 384;
+    }
     return t;
+}
+
+template <typename R> static StapleSites staple_sites_of(const std::vector<const Geom*>& members, int sms) {
+    long long sites[FORMS] = {0, 0, 0, 0}, split_tiles = 0;
+    for (const Geom* g : members) {
+        const int form = stage_form<R>(*g);
+        sites[form] += g->V;
+        if (form == FORM_SPLIT) split_tiles += (g->V + SPLIT_SITES - 1) / SPLIT_SITES;
+    }
+    return {sites[FORM_STAPLE], sites[FORM_PARTS] + (split_tiles > sms ? sites[FORM_SPLIT] : 0)};
+}
+StapleSites staple_sites(int precision, const std::vector<const Geom*>& members, int sms) {
+    return precision == LGF_PREC_FP64 ? staple_sites_of<double>(members, sms) : staple_sites_of<float>(members, sms);
 }
 
 static const lgf_ctx::Tuned* find_tuned(const lgf_ctx* ctx, int precision, long long volume) {
@@ -83,18 +104,28 @@ static const lgf_ctx::Tuned* find_tuned(const lgf_ctx* ctx, int precision, long 
 
 TileShape tuned_shape(const lgf_ctx* ctx, int precision, long long volume) {
     const lgf_ctx::Tuned* t = find_tuned(ctx, precision, volume);
-    return t ? t->shape : default_shape(precision, volume);
+    TileShape s = default_shape(precision, volume);
+    if (!t) return s;
+    if (t->stage) return t->shape;
+    s.meas_budget = t->shape.meas_budget;
+    s.meas_split = t->shape.meas_split;
+    return s;
 }
 
 bool has_tuned(const lgf_ctx* ctx, int precision, long long volume) { return find_tuned(ctx, precision, volume) != nullptr; }
+bool has_tuned_stage(const lgf_ctx* ctx, int precision, long long volume) {
+    const lgf_ctx::Tuned* t = find_tuned(ctx, precision, volume);
+    return t && t->stage;
+}
 
-void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape& shape) {
+void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape& shape, bool stage) {
     for (auto& t : ctx->tuned)
         if (t.prec == precision && t.volume == volume) {
             t.shape = shape;
+            t.stage = stage;
             return;
         }
-    ctx->tuned.push_back({precision, volume, shape});
+    ctx->tuned.push_back({precision, volume, shape, stage});
 }
 
 void buf_free(LatticeBuf& b) {
@@ -717,8 +748,7 @@ private:
     // costs a 48^4 member 40% in the measurement.
     TileShape list_shape(long long V) const {
         if (!per_volume_) return shape_;
-        const int prec = std::is_same<R, double>::value ? LGF_PREC_FP64 : LGF_PREC_FP32MIXED;
-        return has_tuned(ctx_, prec, V) ? tuned_shape(ctx_, prec, V) : default_shape(prec, V);
+        return tuned_shape(ctx_, std::is_same<R, double>::value ? LGF_PREC_FP64 : LGF_PREC_FP32MIXED, V);
     }
 
     lgf_ctx* ctx_;

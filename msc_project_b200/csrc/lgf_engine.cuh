@@ -106,8 +106,10 @@ struct lgf_ctx {
     // 8^4 lattice's first measurement.
     void* small = nullptr;
     // autotuned tile shapes: (precision, lattice volume, shape); a result
-    // applies to volumes within a factor of two of the tuned one
-    struct Tuned { int prec; long long volume; lgf::TileShape shape; };
+    // applies to volumes within a factor of two of the tuned one.  stage: the
+    // stage's block size and order were chosen too (by the caller, or timed on a
+    // lattice that runs the staple kernel); else they follow default_shape
+    struct Tuned { int prec; long long volume; lgf::TileShape shape; bool stage; };
     std::vector<Tuned> tuned;
     // two pinned host chunks for uploads/downloads from pageable memory
     // (allocated on first use; a server's worker shares them, hence the lock)
@@ -135,14 +137,18 @@ int set_error(lgf_ctx* ctx, int code, const char* fmt, ...);
 bool valid_shape(const int shape[4]);
 size_t footprint_bytes(const int shape[4], int precision, int meas_slots);
 int stage_max_threads(int precision);  // the stage kernel's launch bound for this precision
-// until tuned; volume: sites of the lattice (of a mix: of its launches)
+// until tuned; volume: sites of the lattice (of a mix: of a staple launch)
 TileShape default_shape(int precision, long long volume);
+// sites of the two launches of the staple kernel when these lattices flow together
+struct StapleSites { long long one_sum, parts; };
+StapleSites staple_sites(int precision, const std::vector<const Geom*>& members, int sms);
 // the tuned shape for a lattice of this precision and volume, else the default
 TileShape tuned_shape(const lgf_ctx* ctx, int precision, long long volume);
 bool has_tuned(const lgf_ctx* ctx, int precision, long long volume);
-void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape& shape);
-// times the candidate shapes on a lattice of this shape; the fastest is recorded and returned
-int tune_shape(lgf_ctx* ctx, int precision, const int shape[4], TileShape* best);
+bool has_tuned_stage(const lgf_ctx* ctx, int precision, long long volume);
+void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape& shape, bool stage);
+// times the candidate shapes on a lattice of this shape (the stage's if asked); the fastest is recorded and returned
+int tune_shape(lgf_ctx* ctx, int precision, const int shape[4], bool stage, TileShape* best);
 
 // Device resources of one lattice (precision-erased).
 struct LatticeBuf {

@@ -6,10 +6,11 @@
 // with CUDA events on the context's stream (each over at least ~20 ms of
 // launches; a candidate must beat the current shape by 2%), one parameter at
 // a time:
-//   stage:       block size {128, 256, 384},
+//   stage:       (lattices of the staple form) block size {128, 256, 384},
 //                then the tile order {x1 columns per CTA, row blocks through
 //                x0}, then (row blocks) the block budget {2, 8, 32 MB};
-//   measurement: blocks of {12, 6} warps, then the block budget {2, 8, 64 MB}.
+//   measurement: (lattices above the one-launch form) blocks of {12, 6} warps,
+//                then the block budget {2, 8, 64 MB}.
 // The winner is recorded in the context and used by every later group whose
 // largest lattice falls in the same volume class (within a factor of two).
 // No candidate changes a result: only block shapes and tile order differ.
@@ -63,13 +64,23 @@ int time_shape(lgf_ctx* ctx, int prec, LatticeBuf& b, const TileShape& t, int k,
 
 }  // namespace
 
-int tune_shape(lgf_ctx* ctx, int prec, const int shape[4], TileShape* best) {
+int tune_shape(lgf_ctx* ctx, int prec, const int shape[4], bool with_stage, TileShape* best) {
+    // Only what the lattice's kernels read: the plaquette and the split form
+    // have tiles of their own, and so has the measurement of small lattices.
+    // (Timed there, candidates differ by noise, and the pick would decide for
+    // other lattices of the volume class or the batch.)
+    const Geom g = make_geom(shape);
+    const int form = prec == LGF_PREC_FP64 ? stage_form<double>(g) : stage_form<float>(g);
+    const bool stage = with_stage && (form == FORM_STAPLE || form == FORM_PARTS), measure = !small_measure(g);
+    TileShape cur = default_shape(prec, g.V);
     LatticeBuf b;
-    int rc = buf_alloc(ctx, b, shape, prec, 1);
-    if (rc != LGF_OK) return rc;
-    rc = launch_generate(ctx, b, 12345, 0.5);
+    int rc = LGF_OK;
+    if (stage || measure) {
+        rc = buf_alloc(ctx, b, shape, prec, 1);
+        if (rc != LGF_OK) return rc;
+        rc = launch_generate(ctx, b, 12345, 0.5);
+    }
     b.eps = 0.01;
-    TileShape cur = default_shape(prec, b.g.V);
     float cur_ms = 0.f;
     const double MB = double(1 << 20);
     // A candidate replaces the current shape only when it is more than 2%
@@ -79,11 +90,11 @@ int tune_shape(lgf_ctx* ctx, int prec, const int shape[4], TileShape* best) {
     const float KEEP = 0.98f, TARGET_MS = 20.f;
     // ---- RK3 stage: one step (three stage launches) per repetition
     float probe = 0.f;
-    if (rc == LGF_OK) rc = time_shape(ctx, prec, b, cur, -1, 1, &probe);
+    if (rc == LGF_OK && stage) rc = time_shape(ctx, prec, b, cur, -1, 1, &probe);
     const int reps = std::max(3, std::min(200, (int)(TARGET_MS / std::max(probe, 1e-3f))));
-    if (rc == LGF_OK) rc = time_shape(ctx, prec, b, cur, -1, reps, &cur_ms);
+    if (rc == LGF_OK && stage) rc = time_shape(ctx, prec, b, cur, -1, reps, &cur_ms);
     auto try_stage = [&](TileShape t) {
-        if (rc != LGF_OK || t == cur) return;
+        if (rc != LGF_OK || !stage || t == cur) return;
         float ms = 0.f;
         rc = time_shape(ctx, prec, b, t, -1, reps, &ms);
         if (rc == LGF_OK && ms < KEEP * cur_ms) {
@@ -111,13 +122,13 @@ int tune_shape(lgf_ctx* ctx, int prec, const int shape[4], TileShape* best) {
     // ---- measurement kernels alone, starting from whole-slice blocks (the
     // fewest DRAM bytes for the loops' links); smaller blocks replace them
     // only when 2% faster
-    cur.meas_budget = 64.0 * MB;
+    if (measure) cur.meas_budget = 64.0 * MB;
     float meas_ms = 0.f;
-    if (rc == LGF_OK) rc = time_shape(ctx, prec, b, cur, 3, 1, &probe);
+    if (rc == LGF_OK && measure) rc = time_shape(ctx, prec, b, cur, 3, 1, &probe);
     const int mreps = std::max(3, std::min(200, (int)(TARGET_MS / std::max(probe, 1e-3f))));
-    if (rc == LGF_OK) rc = time_shape(ctx, prec, b, cur, 3, mreps, &meas_ms);
+    if (rc == LGF_OK && measure) rc = time_shape(ctx, prec, b, cur, 3, mreps, &meas_ms);
     auto try_meas = [&](TileShape t) {
-        if (rc != LGF_OK || t == cur) return;
+        if (rc != LGF_OK || !measure || t == cur) return;
         float ms = 0.f;
         rc = time_shape(ctx, prec, b, t, 3, mreps, &ms);
         if (rc == LGF_OK && ms < KEEP * meas_ms) {
@@ -138,7 +149,7 @@ int tune_shape(lgf_ctx* ctx, int prec, const int shape[4], TileShape* best) {
     cudaStreamSynchronize(ctx->stream);
     buf_free(b);
     if (rc != LGF_OK) return rc;
-    record_tuned(ctx, prec, 1LL * shape[0] * shape[1] * shape[2] * shape[3], cur);
+    record_tuned(ctx, prec, g.V, cur, stage);
     if (best) *best = cur;
     return LGF_OK;
 }
@@ -170,7 +181,7 @@ int lgf_autotune_tiles(lgf_ctx* ctx, int precision, const int shape[4], lgf_tile
     if (!valid_shape(shape)) return set_error(ctx, LGF_EINVAL, "autotune shape must be even and >= 4");
     cudaSetDevice(ctx->device);
     TileShape t;
-    int rc = tune_shape(ctx, precision, shape, &t);
+    int rc = tune_shape(ctx, precision, shape, true, &t);
     if (rc == LGF_OK && best) to_abi(t, best);
     return rc;
 }
@@ -189,7 +200,7 @@ int lgf_set_tiles(lgf_ctx* ctx, int precision, const int shape[4], const lgf_til
         (t.stage_order != 0 && t.stage_order != 1) ||
         tiles->stage_budget_kb < 1 || tiles->meas_budget_kb < 1 || (t.meas_split != 1 && t.meas_split != 2))
         return set_error(ctx, LGF_EINVAL, "invalid tile shape");
-    record_tuned(ctx, precision, 1LL * shape[0] * shape[1] * shape[2] * shape[3], t);
+    record_tuned(ctx, precision, 1LL * shape[0] * shape[1] * shape[2] * shape[3], t, true);
     return LGF_OK;
 }
 
