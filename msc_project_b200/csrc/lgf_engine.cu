@@ -558,6 +558,11 @@ public:
     // graph launch; a graph per count of launch segments, captured on first use
     int replay_step() override {
         NvtxRange r("lgf.rk3_step");
+        // a server's mixes may run through any combination of the forms' counts
+        if (step_execs_.size() >= MAX_STEP_GRAPHS && !step_execs_.count(step_graph())) {
+            LGF_CUDA_TRY(ctx_, cudaStreamSynchronize(ctx_->stream));  // none is running when it goes
+            drop_step_graphs();
+        }
         cudaGraphExec_t& g = step_execs_[step_graph()];
         if (!g) {
             int rc = capture_one(true, 0, &g);
@@ -609,9 +614,12 @@ private:
         for (auto g : meas_execs_) if (g) return true;
         return false;
     }
-    void drop_graphs() {
+    void drop_step_graphs() {
         for (auto& g : step_execs_) if (g.second) cudaGraphExecDestroy(g.second);
         step_execs_.clear();
+    }
+    void drop_graphs() {
+        drop_step_graphs();
         for (auto& g : meas_execs_) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     }
 
@@ -783,6 +791,7 @@ private:
     long long tiles_cap_ = 0;                      // capacity of d_tiles_
     int plaq_grid_max_ = 1, update_grid_max_ = 1;
     std::vector<int2> seg_tiles_;                  // tiles of each stage launch (first, count)
+    static constexpr size_t MAX_STEP_GRAPHS = 64;  // as many as the counts of one form (up to 32 slots) twice over
     std::map<int, cudaGraphExec_t> step_execs_;    // by launch counts (step_graph)
     std::vector<cudaGraphExec_t> meas_execs_;      // by segment count (and small lattices)
 };
