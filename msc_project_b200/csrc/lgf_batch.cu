@@ -58,36 +58,51 @@ TileShape shape_for(lgf_ctx* ctx, int prec, const int shape[4], bool stage) {
     return best;
 }
 
-// Every job's results: one run of copies into a page-locked area and one wait
-// for all of them, then the final links that are asked for.
+// Every job's results: runs of copies into a page-locked area of a bounded size
+// (the context keeps it) with one wait each, a larger job's on its own through
+// the pinned chunks, then the final links that are asked for.
+constexpr size_t RESULT_AREA_BYTES = 16u << 20;
+
 int fetch_results(lgf_ctx* ctx, std::vector<std::unique_ptr<JobRun>>& runs) {
     auto per = [](const JobRun& r) { return 2 + 2 * (size_t)r.buf.g.n[0]; };
-    size_t total = 0;
-    for (const auto& r : runs) total += per(*r) * r->nmeas * sizeof(double);
-    if (total > 0) {
+    auto bytes = [&](const JobRun& r) { return per(r) * r.nmeas * sizeof(double); };
+    auto deliver = [&](const JobRun& r, const double* v) {
+        const lgf_meas* out = r.job->meas;
+        const int N0 = r.buf.g.n[0];
+        for (int m = 0; out && m < r.nmeas; ++m, v += per(r)) {
+            out->t[m] = r.tvals[m];
+            out->E[m] = v[0];
+            out->Q[m] = v[1];
+            if (out->E_slice) std::memcpy(out->E_slice + (size_t)m * N0, v + 2, N0 * sizeof(double));
+            if (out->Q_slice) std::memcpy(out->Q_slice + (size_t)m * N0, v + 2 + N0, N0 * sizeof(double));
+        }
+    };
+    for (size_t i = 0, j; i < runs.size(); i = j) {
+        size_t total = bytes(*runs[i]);
+        for (j = i + 1; j < runs.size() && total + bytes(*runs[j]) <= RESULT_AREA_BYTES; ++j) total += bytes(*runs[j]);
+        if (total == 0) continue;
+        if (total > RESULT_AREA_BYTES) {  // one job
+            std::vector<double> h(total / sizeof(double));
+            const int rc = copy_out(ctx, h.data(), runs[i]->buf.meas, total);
+            if (rc != LGF_OK) return rc;
+            deliver(*runs[i], h.data());
+            continue;
+        }
         std::lock_guard<std::mutex> lk(ctx->list_mu);
         char* h = nullptr;
         LGF_CUDA_TRY(ctx, ctx->list_stage.acquire(total, &h));
         size_t off = 0;
-        for (const auto& r : runs) {
-            const size_t n = per(*r) * r->nmeas * sizeof(double);
-            if (n) LGF_CUDA_TRY(ctx, cudaMemcpyAsync(h + off, r->buf.meas, n, cudaMemcpyDeviceToHost, ctx->stream));
+        for (size_t k = i; k < j; ++k) {
+            const size_t n = bytes(*runs[k]);
+            if (n) LGF_CUDA_TRY(ctx, cudaMemcpyAsync(h + off, runs[k]->buf.meas, n, cudaMemcpyDeviceToHost, ctx->stream));
             off += n;
         }
         LGF_CUDA_TRY(ctx, ctx->list_stage.release(ctx->stream));
         LGF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-        const double* v = (const double*)h;
-        for (const auto& r : runs) {
-            const lgf_meas* out = r->job->meas;
-            const int N0 = r->buf.g.n[0];
-            for (int m = 0; m < r->nmeas; ++m, v += per(*r)) {
-                if (!out) continue;
-                out->t[m] = r->tvals[m];
-                out->E[m] = v[0];
-                out->Q[m] = v[1];
-                if (out->E_slice) std::memcpy(out->E_slice + (size_t)m * N0, v + 2, N0 * sizeof(double));
-                if (out->Q_slice) std::memcpy(out->Q_slice + (size_t)m * N0, v + 2 + N0, N0 * sizeof(double));
-            }
+        off = 0;
+        for (size_t k = i; k < j; ++k) {
+            deliver(*runs[k], (const double*)(h + off));
+            off += bytes(*runs[k]);
         }
     }
     for (const auto& r : runs) {
