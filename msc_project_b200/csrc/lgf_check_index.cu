@@ -12,7 +12,7 @@
 //     bijections into the padded buffers with 16-byte aligned vector loads;
 //   - the stage and measurement tile lists cover every tile exactly once for
 //     row-block and column orders and a range of budgets and block sizes, and
-//     the measurement's strips or patches cover every site of a slice once;
+//     the measurement's chunks cover every site of a slice once;
 //   - the units of the measurement's plane kernel cover every site of every
 //     plane once as an output, with the three rows before it in the unit;
 //   - the launch segments of a group (member_runs) split a list of members
@@ -23,10 +23,6 @@
 #include <set>
 #include <vector>
 
-// both measurement geometries are checked: strips by default builds, patches here
-#ifndef LGF_MEAS_PATCH
-#define LGF_MEAS_PATCH 1
-#endif
 #include "lgf_measure.cuh"
 #include "lgf_tiles.h"
 
@@ -179,9 +175,9 @@ static void check_tiles(const Geom& g) {
         std::vector<char> hit(g.Vs, 0);
         for (int c = 0; c < nchunk; ++c)
             for (int l = 0; l < MEAS_SITES; ++l) {
-                const int off = meas_site_offset(g, meas_patched(g), c, l);
+                const int off = meas_site_offset(c, l);
                 if (off < g.Vs) CHECK(!hit[off]++);
-                else CHECK(!meas_patched(g));  // only a strip's last chunk runs past the slice
+                else CHECK(c == nchunk - 1);  // only the last chunk runs past the slice
             }
         for (int o = 0; o < g.Vs; ++o) CHECK(hit[o] == 1);
     }

@@ -101,9 +101,9 @@ __device__ __forceinline__ su3<R> staple_sum(const cplx<R>* __restrict__ U, cons
     return S;
 }
 
-// ta_part(A B, s) computing only what the projection reads: the imaginary
-// parts of the diagonal and the three off-diagonal pairs (90 real
-// operations instead of 108 for the full product)
+// s times the traceless anti-Hermitian part of A B, W - W^dag - 1/3 Tr(W - W^dag),
+// computing only what it reads of the product: the imaginary parts of the
+// diagonal and the three off-diagonal pairs (90 real operations instead of 108)
 template <typename R> __device__ __forceinline__ alg<R> ta_of_product(const su3<R>& A, const su3<R>& B, R s) {
     R d[3];
 #pragma unroll
@@ -725,33 +725,11 @@ template <typename R> __device__ __forceinline__ void store_alg_as_herm(double2*
 
 constexpr int MEAS_SITES = 32;  // sites per measurement block (x) ; planes in y
 
-// Measurement tile geometry.  A tile's 32 sites are 32 consecutive sites of
-// the slice (a strip), or, built with -DLGF_MEAS_PATCH=1, a patch of 4 x2 rows
-// by 8 x3 positions at fixed (x0, x1) when N2 % 4 == 0 and N3 % 8 == 0.  The
-// patch keeps the +-3 stencil of the six planes compact (a strip along x3
-// touches ~5500 distinct sites per tile, a 4 x 8 patch ~3600) and each warp
-// load still covers four whole 128-byte lines, but measured on one B200 it
-// is 2-8% slower in FP64 (16^4 to 48^4), 4-6% faster in FP32 up to 32^4 and
-// 13% slower on 48^4, so strips are the default.  Chunk c of a slice is patch
-// (x1, b2, b3) = (c / (nb2 nb3), (c / nb3) % nb2, c % nb3); a slice has
-// Vs / 32 chunks either way.  The geometry is a fixed function of the
+// Offset within its x0 slice of lane l's site in measurement chunk c: a tile is
+// 32 consecutive sites of the slice.  The geometry is a fixed function of the
 // lattice shape, so the grouping of the partial sums (and every result bit)
 // does not depend on tile shapes or batch partners.
-#ifndef LGF_MEAS_PATCH
-#define LGF_MEAS_PATCH 0
-#endif
-constexpr int MEAS_PATCH_ROWS = 4, MEAS_PATCH_COLS = 8;
-__host__ __device__ __forceinline__ bool meas_patched(const Geom& g) {
-    return LGF_MEAS_PATCH && g.n[2] % MEAS_PATCH_ROWS == 0 && g.n[3] % MEAS_PATCH_COLS == 0;
-}
-// offset within its x0 slice of lane l's site in measurement chunk c
-__host__ __device__ __forceinline__ int meas_site_offset(const Geom& g, bool patched, int c, int l) {
-    if (!patched) return c * MEAS_SITES + l;
-    const int nb3 = g.n[3] / MEAS_PATCH_COLS, nb2 = g.n[2] / MEAS_PATCH_ROWS;
-    const int x1 = c / (nb2 * nb3), r = c - x1 * (nb2 * nb3), b2 = r / nb3, b3 = r - b2 * nb3;
-    return (x1 * g.n[2] + b2 * MEAS_PATCH_ROWS + l / MEAS_PATCH_COLS) * g.n[3] + b3 * MEAS_PATCH_COLS +
-           l % MEAS_PATCH_COLS;
-}
+__host__ __device__ __forceinline__ int meas_site_offset(int c, int l) { return c * MEAS_SITES + l; }
 #ifndef LGF_MEAS_SMEM_ACC
 #define LGF_MEAS_SMEM_ACC 1
 #endif
@@ -976,7 +954,7 @@ template <typename R, bool OUT, bool FILE>
 __device__ __forceinline__ void measure_tile(MeasSmem<R, FILE>* sm, const cplx<R>* __restrict__ U, const Geom& g, int slice, int chunk,
                                              double2* __restrict__ partial, int nchunk, const MeasSites& out) {
     const int lane = threadIdx.x, w = threadIdx.y, p = w % 6, part = w / 6;
-    const int off = meas_site_offset(g, meas_patched(g), chunk, lane);
+    const int off = meas_site_offset(chunk, lane);
     const bool valid = off < g.Vs;
     const int s = slice * g.Vs + (valid ? off : 0);
     const Coord c = site_coord(g, s);

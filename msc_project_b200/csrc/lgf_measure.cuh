@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(96 * LOOP_MAX_GROUPS, 1) k_meas_loops(const La
         const int4 tile = mtiles[ti];
         const LatDesc<R>* d = descs + tile.x;
         const Geom g = d->g;
-        const int off = meas_site_offset(g, meas_patched(g), tile.z, lane);
+        const int off = meas_site_offset(tile.z, lane);
         if (off >= g.Vs) continue;
         const int s = tile.y * g.Vs + off;
         const Coord c = site_coord(g, s);
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(SITES_THREADS) k_meas_sites(const LatDesc<R>* 
         const int4 tile = mtiles[ti];
         const LatDesc<R>* d = descs + tile.x;
         const Geom g = d->g;
-        const int off = meas_site_offset(g, meas_patched(g), tile.z, lane);
+        const int off = meas_site_offset(tile.z, lane);
         double e = 0.0, q = 0.0;
         if (off < g.Vs) {
             const int s = tile.y * g.Vs + off;

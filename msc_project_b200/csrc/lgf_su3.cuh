@@ -209,23 +209,6 @@ template <typename R> __device__ __forceinline__ void su3_addto(su3<R>& a, const
 // Re X02, Im X02, Re X12, Im X12), X22 = -i(v0+v1), X_ji = -conj(X_ij).
 template <typename R> struct alg { R v[8]; };
 
-// Traceless anti-Hermitian part  (W - W^dag) - 1/3 Tr(W - W^dag), scaled by s,
-// as 8 coordinates.  Only the entries needed are read.
-template <typename R> __device__ __forceinline__ alg<R> ta_part(const su3<R>& W, R s) {
-    alg<R> z;
-    R d0 = R(2) * W.m[0].im, d1 = R(2) * W.m[4].im, d2 = R(2) * W.m[8].im;
-    R tr = (d0 + d1 + d2) * R(1.0 / 3.0);
-    z.v[0] = s * (d0 - tr);
-    z.v[1] = s * (d1 - tr);
-    z.v[2] = s * (W.m[1].re - W.m[3].re);
-    z.v[3] = s * (W.m[1].im + W.m[3].im);
-    z.v[4] = s * (W.m[2].re - W.m[6].re);
-    z.v[5] = s * (W.m[2].im + W.m[6].im);
-    z.v[6] = s * (W.m[5].re - W.m[7].re);
-    z.v[7] = s * (W.m[5].im + W.m[7].im);
-    return z;
-}
-
 // Hermitian traceless Q = -i X from the 8 coordinates of X (double).
 struct herm_d {
     double a0, a1, a2;            // real diagonal
