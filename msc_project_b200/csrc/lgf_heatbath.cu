@@ -332,14 +332,16 @@ __global__ void __launch_bounds__(256) k_plaquette(const cplx<R>* __restrict__ U
 // FP64: 3 blocks (168 registers) 1, 4 (128, some spills) 1.3: 32x16^3 runs one
 // wave of 4 instead of two of 3, 22 against 24 us; 24^3x48 6 of 3, not 5 of 4.
 // FP32: 4 blocks (128) 4 (4.2 in parity order), 5 (96) 5.05, 6 (80, some spills)
-// 6.2: many waves cost about the same with each cap, and 192000 sites fit one wave of 6 (overrelaxation of
-// 4 sweeps in parity order 591 us, 674 in two waves of 5).
+// 6.2 (6.9): many waves cost about the same with each cap, and 192000 sites fit
+// one wave of 6 (overrelaxation of 4 sweeps in parity order 591 us, 674 in two
+// waves of 5).  In parity order three waves of 6 lose to four of 5: 24^3x48, 4
+// overrelaxation sweeps, 2205 against 2140 us.
 template <typename R, bool PARITY> auto heatbath_kernel(int nb, int sms) {
     auto waves = [&](int per_sm) { return (nb + per_sm * sms - 1) / (per_sm * sms); };
     if constexpr (sizeof(R) == sizeof(double)) {
         return 10 * waves(3) > 13 * waves(4) ? k_checkerboard<R, 4, PARITY> : k_checkerboard<R, 3, PARITY>;
     } else {
-        const int c4 = (PARITY ? 420 : 400) * waves(4), c5 = 505 * waves(5), c6 = 620 * waves(6);
+        const int c4 = (PARITY ? 420 : 400) * waves(4), c5 = 505 * waves(5), c6 = (PARITY ? 690 : 620) * waves(6);
         if (c6 < c4 && c6 < c5) return k_checkerboard<R, 6, PARITY>;
         return c5 < c4 ? k_checkerboard<R, 5, PARITY> : k_checkerboard<R, 4, PARITY>;
     }
