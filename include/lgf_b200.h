@@ -213,7 +213,7 @@ typedef struct lgf_tile_shape {
     int stage_threads;    /* RK3 stage block size: 128, 256 or 384 (4 link directions x threads/4 sites) */
     int stage_order;      /* 0: blocks of x1 rows swept through x0; 1: x1 columns walked per block */
     int stage_budget_kb;  /* order 0: stage working set per row block and x0 slice */
-    int meas_budget_kb;   /* measurement: link bytes per row block and x0 slice (7 slices live) */
+    int meas_budget_kb;   /* measurement: link bytes per row block and x0 slice (loops read x0 .. x0+3) */
     int meas_split;       /* measurement blocks of 6 warps (1) or 12 warps (2) */
 } lgf_tile_shape;
 

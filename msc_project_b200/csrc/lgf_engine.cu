@@ -753,7 +753,7 @@ private:
     // in a group of uneven volumes (per_volume_: batches, serving) each
     // member is ordered as tuned for its own volume class, else by the
     // defaults -- an order tuned on 24^3x48 (whole-slice measurement blocks)
-    // costs a 48^4 member 40% in the measurement.
+    // costs a 48^4 member 2 to 4% in the measurement.
     TileShape list_shape(long long V) const {
         if (!per_volume_) return shape_;
         return tuned_shape(ctx_, std::is_same<R, double>::value ? LGF_PREC_FP64 : LGF_PREC_FP32MIXED, V);

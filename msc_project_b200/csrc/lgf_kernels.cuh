@@ -275,8 +275,9 @@ template <typename R, typename D = R, bool FILE = false> struct Plane {
 // (double, LGF_MEAS_SMEM_ACC) its own column of shared memory.  The FP64
 // kernel holds two path matrices, the incoming link and these sums at its
 // peak; at 168 registers that spilled ~0.6 KB per thread, and with the sums in
-// shared memory (48 KB per block) it spills ~50 B and runs 12-13% faster on
-// 16^4 to 48^4.  Same operations, same order, either way (bit-identical).
+// shared memory (48 KB per block) it spills ~50 B and ran 12-13% faster when
+// this kernel measured 16^4 to 48^4.  Same operations, same order, either way
+// (bit-identical).
 template <typename R> struct RegAcc {
     alg<R>& a;
     __device__ __forceinline__ R get(int k) const { return a.v[k]; }
@@ -503,7 +504,7 @@ __global__ void __launch_bounds__(StageMaxThreads<R>::value, LGF_STAGE_MINB) k_r
 // Where a group's small lattices have more tiles than that, the staple form
 // with the same grouping of the sum (PARTS) takes them, so that the bits are
 // those the lattice gives alone: 64 x 8^4 batched, 200 steps, FP32 84 -> 78 ms
-// on the device, FP64 118 -> 123 (the second sum spills 40 bytes; the split
+// on the device, FP64 117 -> 113 with the launch's best block size (the split
 // kernel itself, a tile per SM at a time, took 1.5 times as long).
 constexpr int SPLIT_SITES = 32, SPLIT_THREADS = 12 * SPLIT_SITES;
 constexpr long long SPLIT_MAX_SITES = 148 * SPLIT_SITES;

@@ -77,8 +77,10 @@ typedef double LoopReal;
 
 // Lattices of up to one 32-site tile per SM are measured by the one-launch
 // kernel k_measure instead (lgf_kernels.cuh): with too few threads to fill the
-// SMs its 33 us (FP64, 8^4) beat the five launches' 46 us; 12^4, with 4.4
-// tiles per SM, takes 135 against 109 us.  The rule reads the lattice alone,
+// SMs its 33 us (FP64, 8^4) beat the five launches' 46 us.  Above, the SMs with
+// two tiles run them in turn: FP64 4800 to 8192 sites 61 against 47 us, 10000
+// 86 against 63, 12^4 138 against 105; FP32, whose loops are multiplied in
+// double here, 41 to 42 against 43 to 45, 10000 57 against 54, 12^4 88 against 84.  The rule reads the lattice alone,
 // so a lattice gives the same bits in every group.
 constexpr int SMALL_MEAS_TILES = 148;
 __host__ __device__ __forceinline__ bool small_measure(const Geom& g) {

@@ -13,18 +13,18 @@ namespace lgf {
 // ------------------------------------------------------------ work order
 // The persistent kernels take tiles in list order, so the list order sets the
 // L2 reuse distance of the stencil.  In plain site order the x0 +- 1 (and, in
-// the measurement, up to +- 3) neighbours of a site are reused one slice of
+// the measurement, up to + 3) neighbours of a site are reused one slice of
 // work later; once a slice of work exceeds the L2 budget they come from HBM
 // again.  Large lattices are therefore ordered in blocks of x1 (and x2) rows,
 // each block swept through every x0 slice before the next block starts.  Only
 // the order changes: the set of tiles is the same, and no result depends on
 // it (no reduction runs in tile order).
-// Block budgets, measured on 16^4 .. 48^4 (FP64, 100 steps): 8 MB / 2 MB gave
-// +5% on 24^3x48 and +7% on 32^4 over the plain site order; 24/8, 12/4, 4/1
-// and smaller were between the two.
+// Block budgets, measured on 16^4 .. 48^4 (FP64, 100 steps, a measurement that
+// read x0 +- 3): 8 MB / 2 MB gave +5% on 24^3x48 and +7% on 32^4 over the plain
+// site order; 24/8, 12/4, 4/1 and smaller were between the two.
 // (The budgets are fields of TileShape: stage bytes, default 8 MB, and
-// measurement link bytes, default 2 MB, per block and slice; x0 +- 3 keeps
-// 7 slices of a measurement block live.)
+// measurement link bytes, default 2 MB, per block and slice; the loops read
+// x0 .. x0 + 3, so four slices of a measurement block are live.)
 
 // A block: x1 in [a1, b1), x2 in [a2, b2), all x3.  One block per slice when
 // a slice of work fits the budget; else blocks of whole x1 rows, at least
