@@ -106,19 +106,19 @@ TileShape tuned_shape(const lgf_ctx* ctx, int precision, long long volume) {
     const lgf_ctx::Tuned* t = find_tuned(ctx, precision, volume);
     TileShape s = default_shape(precision, volume);
     if (!t) return s;
-    if (t->stage) return t->shape;
+    if (t->stage != StageChoice::none) return t->shape;
     s.meas_budget = t->shape.meas_budget;
     s.meas_split = t->shape.meas_split;
     return s;
 }
 
 bool has_tuned(const lgf_ctx* ctx, int precision, long long volume) { return find_tuned(ctx, precision, volume) != nullptr; }
-bool has_tuned_stage(const lgf_ctx* ctx, int precision, long long volume) {
+StageChoice tuned_stage(const lgf_ctx* ctx, int precision, long long volume) {
     const lgf_ctx::Tuned* t = find_tuned(ctx, precision, volume);
-    return t && t->stage;
+    return t ? t->stage : StageChoice::none;
 }
 
-void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape& shape, bool stage) {
+void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape& shape, StageChoice stage) {
     for (auto& t : ctx->tuned)
         if (t.prec == precision && t.volume == volume) {
             t.shape = shape;

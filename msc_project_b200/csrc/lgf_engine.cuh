@@ -46,6 +46,9 @@ struct TileShape {
     }
     bool operator!=(const TileShape& o) const { return !(*this == o); }
 };
+// where a recorded shape's stage part comes from: default_shape, a timing of
+// one lattice that runs the staple kernel, or the caller
+enum class StageChoice { none, timed, set };
 }  // namespace lgf
 
 namespace lgf {
@@ -106,10 +109,9 @@ struct lgf_ctx {
     // 8^4 lattice's first measurement.
     void* small = nullptr;
     // autotuned tile shapes: (precision, lattice volume, shape); a result
-    // applies to volumes within a factor of two of the tuned one.  stage: the
-    // stage's block size and order were chosen too (by the caller, or timed on a
-    // lattice that runs the staple kernel); else they follow default_shape
-    struct Tuned { int prec; long long volume; lgf::TileShape shape; bool stage; };
+    // applies to volumes within a factor of two of the tuned one; its stage part
+    // where it was chosen too, else default_shape's
+    struct Tuned { int prec; long long volume; lgf::TileShape shape; lgf::StageChoice stage; };
     std::vector<Tuned> tuned;
     // two pinned host chunks for uploads/downloads from pageable memory
     // (allocated on first use; a server's worker shares them, hence the lock)
@@ -145,8 +147,8 @@ StapleSites staple_sites(int precision, const std::vector<const Geom*>& members,
 // the tuned shape for a lattice of this precision and volume, else the default
 TileShape tuned_shape(const lgf_ctx* ctx, int precision, long long volume);
 bool has_tuned(const lgf_ctx* ctx, int precision, long long volume);
-bool has_tuned_stage(const lgf_ctx* ctx, int precision, long long volume);
-void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape& shape, bool stage);
+StageChoice tuned_stage(const lgf_ctx* ctx, int precision, long long volume);
+void record_tuned(lgf_ctx* ctx, int precision, long long volume, const TileShape& shape, StageChoice stage);
 // times the candidate shapes on a lattice of this shape (the stage's if asked); the fastest is recorded and returned
 int tune_shape(lgf_ctx* ctx, int precision, const int shape[4], bool stage, TileShape* best);
 

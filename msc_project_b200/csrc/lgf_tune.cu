@@ -149,7 +149,7 @@ int tune_shape(lgf_ctx* ctx, int prec, const int shape[4], bool with_stage, Tile
     cudaStreamSynchronize(ctx->stream);
     buf_free(b);
     if (rc != LGF_OK) return rc;
-    record_tuned(ctx, prec, g.V, cur, stage);
+    record_tuned(ctx, prec, g.V, cur, stage ? StageChoice::timed : StageChoice::none);
     if (best) *best = cur;
     return LGF_OK;
 }
@@ -200,7 +200,7 @@ int lgf_set_tiles(lgf_ctx* ctx, int precision, const int shape[4], const lgf_til
         (t.stage_order != 0 && t.stage_order != 1) ||
         tiles->stage_budget_kb < 1 || tiles->meas_budget_kb < 1 || (t.meas_split != 1 && t.meas_split != 2))
         return set_error(ctx, LGF_EINVAL, "invalid tile shape");
-    record_tuned(ctx, precision, 1LL * shape[0] * shape[1] * shape[2] * shape[3], t, true);
+    record_tuned(ctx, precision, 1LL * shape[0] * shape[1] * shape[2] * shape[3], t, StageChoice::set);
     return LGF_OK;
 }
 

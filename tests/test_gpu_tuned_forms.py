@@ -40,3 +40,15 @@ def test_a_batch_sizes_its_blocks_by_the_staple_lattices(spec, threads):
                 lat.generate(j.seed, 0.5)
                 r = lat.flow(0.01, 3, 3)
                 assert np.array_equal(r.Q, j.result.Q) and np.array_equal(lat.download(), j.links_out)
+
+
+def test_one_lattice_timed_does_not_size_a_larger_batch():
+    """A first batch of one lattice times its volume class; later batches of many take the size of their own launches."""
+    shape = (6, 10, 10, 8)
+    with Context(0) as c:
+        c.batch_run(jobs([(shape, 1)], FP64))
+        for n, threads in ((2, 384), (3, 128), (8, 384)):
+            js = jobs([(shape, n)], FP64)
+            assert c.batch_run(js).block_threads == threads
+        c.set_tiles(FP64, shape, stage_threads=256)  # the caller's choice holds
+        assert c.batch_run(jobs([(shape, 2)], FP64)).block_threads == 256
