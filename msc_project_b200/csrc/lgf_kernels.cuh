@@ -679,7 +679,10 @@ __global__ void __launch_bounds__(4 * UPDATE_SITES, update_blocks<R>()) k_rk3_up
 //    4800  18.4  20.5  22.6      8192  18.6  21    24        9600  22.5  24.6  26.6
 //   12000  22.6  24.7  26.6     13824  23.2  24.6  27       14400  31.8  34.8  29.3
 //   15120        34.8  30.7     20736        37    34.8
-// so the line is one wave of the staple form: three 32-site tiles per SM.
+// so the line is one wave of the staple form: three 32-site tiles per SM.  In
+// batches of eight and more such lattices the plaquette form would be 0 to 3%
+// faster (16 x 13440 sites, 100 steps, 34.5 against 35.7 ms; 39.8 with one sum),
+// in smaller ones slower (2 of them 6.3 against 5.5).
 // FP64: 16384 sites 41 (staple, PARTS 41) against 43, 20736: 53 against 49.  Nor
 // do FP64 lattices past L2 (196608 sites: 365 against 379; 276480, 331776,
 // 442368: equal within the runs' spread; 48^4 11% slower).  The rule reads the
